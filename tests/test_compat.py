@@ -150,7 +150,7 @@ def test_indexed_linear_stand_in(subscripts, dtype):
         assert (h_.cpu().double() - w_).abs().max() <= tol * max(1.0, float(w_.abs().max()))
 
 
-@pytest.mark.skipif(not os.path.isdir(REFERENCE), reason="reference checkout not present")
+@pytest.mark.skipif(not os.path.isdir(os.path.join(REFERENCE, "cuequivariance")), reason="reference checkout not present")
 def test_unmodified_reference_frontend_dispatches_to_the_stand_in():
     """Runs in a subprocess so that the reference import does not leak into other tests."""
     import subprocess
