@@ -217,7 +217,7 @@ def kernel_source_digest() -> str:
     import hashlib
 
     h = hashlib.sha1()
-    for name in ("cw_kernels.cu", "cw_macros.cuh", "gen_cw_groups.py"):
+    for name in ("cw_kernels.cu", "cw_kernels.cuh", "cw_entry.h", "cw_macros.cuh", "gen_cw_groups.py"):
         with open(os.path.join(ROOT, "cuequivariance_b200", "csrc", name), "rb") as f:
             h.update(f.read())
     return h.hexdigest()

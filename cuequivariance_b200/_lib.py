@@ -50,13 +50,14 @@ class CwArgs(C.Structure):
         ("gout", C.c_void_p), ("gw", C.c_void_p), ("gx1", C.c_void_p), ("gx2", C.c_void_p),
         ("senders", C.c_void_p), ("order", C.c_void_p), ("rowptr", C.c_void_p),
         ("tab_start", C.c_void_p), ("tab_j", C.c_void_p), ("tab_c", C.c_void_p),
-        ("bwd_coef", C.POINTER(C.c_float)),
+        ("bwd_coef", C.c_void_p),
         ("w_stride", C.c_int64), ("x1_stride", C.c_int64), ("x2_stride", C.c_int64), ("out_stride", C.c_int64),
         ("num_receivers", C.c_int64),
         ("extent", C.c_int32), ("x1_offset", C.c_int32), ("num_paths", C.c_int32), ("num_terms", C.c_int32),
         ("w_offset", C.c_int32 * 8), ("out_offset", C.c_int32 * 8),
         ("x1_mul_ir", C.c_int32), ("out_mul_ir", C.c_int32), ("channels_per_lane", C.c_int32), ("staging", C.c_int32),
         ("status", C.c_void_p), ("recv_mod", C.c_int32), ("variant", C.c_int32),
+        ("path_mask", C.c_int32), ("x2_width", C.c_int32), ("dtype", C.c_int32), ("reserved", C.c_int32),
     ]
 
 
@@ -69,7 +70,7 @@ class CwNoAllocArgs(C.Structure):
         ("num_edges", C.c_int64), ("num_receivers", C.c_int64),
         ("extent", C.c_int32), ("x1_offset", C.c_int32), ("num_paths", C.c_int32), ("num_terms", C.c_int32),
         ("w_offset", C.c_int32 * 8), ("out_offset", C.c_int32 * 8),
-        ("mul_ir", C.c_int32), ("reserved", C.c_int32),
+        ("mul_ir", C.c_int32), ("path_mask", C.c_int32),
     ]
 
 

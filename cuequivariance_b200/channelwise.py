@@ -53,23 +53,6 @@ def value_pattern(l1: int, l2: int, l3: int):
     return values, pairs
 
 
-SPLIT_GROUPS = False  # measured on B200: one launch per irrep beats two lighter launches
-
-
-def split_group(l1: int, paths: Sequence[Tuple[int, int]]) -> List[List[Tuple[int, int]]]:
-    """How the paths that read irrep ``l1`` are divided into kernel launches.  A launch keeps
-    one accumulator per output component of its paths in registers, so large groups are cut
-    in two parts of similar arithmetic weight (the two heaviest couplings form one part);
-    this keeps four channels per thread within the register budget."""
-    paths = list(paths)
-    if not SPLIT_GROUPS or (len(paths) <= 4 and sum(2 * l3 + 1 for _, l3 in paths) <= 16):
-        return [paths]
-    weight = {p: len(pair_pattern(l1, p[0], p[1], "k")) for p in paths}
-    heavy = sorted(paths, key=lambda p: -weight[p])[:2]
-    light = [p for p in paths if p not in heavy]
-    return [light, [p for p in paths if p in heavy]]
-
-
 def group_signature(l1: int, paths: Sequence[Tuple[int, int]]) -> str:
     return f"{l1}:" + ",".join(f"{a}.{b}" for a, b in paths)
 
@@ -157,9 +140,26 @@ def _library_groups() -> dict:
     return {L.cueq_b200_cw_group_signature(g).decode(): g for g in range(L.cueq_b200_cw_num_groups())}
 
 
+def _parse_signature(sig: str):
+    l1, paths = sig.split(":")
+    return int(l1), [tuple(int(v) for v in p.split(".")) for p in paths.split(",")]
+
+
+def covering_group(l1: int, paths) -> Optional[Tuple[int, list]]:
+    """(library group id, its path list) of the group of degree ``l1`` that contains ``paths``: the group itself or
+    a larger one, whose kernels then skip the paths that are not in the launch's path mask."""
+    best = None
+    for sig, gid in _library_groups().items():
+        gl1, gpaths = _parse_signature(sig)
+        if gl1 == l1 and set(paths) <= set(gpaths) and (best is None or len(gpaths) < len(best[1])):
+            best = (gid, gpaths)
+    return best
+
+
 class ChannelwisePlan:
     """What the kernels need for one channelwise polynomial: per group the library kernel
-    id, segment offsets and the M-tables (forward: k-major pairs, backward: i-major)."""
+    id, segment offsets and the M-tables (forward: k-major pairs, backward: i-major).  Offsets and tables are in
+    the numbering of the library's group; paths it has and the polynomial has not get no terms."""
 
     def __init__(self, groups, extent, row_sizes, x1_blocks, out_blocks):
         self.groups = groups
@@ -169,20 +169,21 @@ class ChannelwisePlan:
         self.out_blocks = out_blocks
         self._dev: dict = {}
 
-    def tables_on(self, device):
+    def tables_on(self, device, dtype=None):
         import torch
 
-        t = self._dev.get(device)
+        dtype = dtype or torch.float32
+        t = self._dev.get((device, dtype))
         if t is None:
             t = []
             for g in self.groups:
                 t.append({
                     k: (torch.tensor(g[k][0], dtype=torch.int32, device=device),
                         torch.tensor(g[k][1], dtype=torch.int32, device=device),
-                        torch.tensor(g[k][2], dtype=torch.float32, device=device))
+                        torch.tensor(g[k][2], dtype=dtype, device=device))
                     for k in ("fwd_tab", "bwd_tab")
                 })
-            self._dev[device] = t
+            self._dev[(device, dtype)] = t
         return t
 
 
@@ -198,7 +199,7 @@ def match_channelwise(polynomial) -> Optional[ChannelwisePlan]:
     if not x1_op.segments or not x2_op.segments:
         return None
     extent = x1_op.segments[0][1]
-    if extent % 4 or any(s[1] != extent for s in x1_op.segments) or any(s[1] != 1 for s in x2_op.segments):
+    if extent % 2 or any(s[1] != extent for s in x1_op.segments) or any(s[1] != 1 for s in x2_op.segments):
         return None
     if any(s[0] % 2 == 0 for s in x1_op.segments + x2_op.segments):
         return None
@@ -231,49 +232,46 @@ def match_channelwise(polynomial) -> Optional[ChannelwisePlan]:
         if not np.allclose(c, alpha * ref, rtol=1e-12, atol=1e-14):
             return None
         by_i1.setdefault(s1, []).append((l1, l2, l3, sw, so, c))
-    lib = _library_groups()
     groups = []
-    launches = []
     for s1, plist in sorted(by_i1.items()):
         l1 = plist[0][0]
-        all_paths = [(l2, l3) for _, l2, l3, _, _, _ in plist]
-        if len(set(all_paths)) != len(all_paths):
+        have = {(l2, l3): (sw, so, c) for _, l2, l3, sw, so, c in plist}
+        if len(have) != len(plist):
             return None
-        parts = split_group(l1, all_paths)
-        if any(group_signature(l1, part) not in lib for part in parts):
-            parts = [all_paths]
-        for part in parts:
-            launches.append((s1, [p for p in plist if (p[1], p[2]) in part]))
-    for s1, plist in launches:
-        l1 = plist[0][0]
-        sig = group_signature(l1, [(l2, l3) for _, l2, l3, _, _, _ in plist])
-        if sig not in lib:
+        found = covering_group(l1, have)
+        if found is None:
             return None
-        g = {"id": lib[sig], "x1_off": x1_off[s1], "w_off": [w_off[p[3]] for p in plist],
-             "out_off": [out_off[p[4]] for p in plist], "npath": len(plist), "out_segs": [p[4] for p in plist],
-             "x1_width": x1_op.segments[s1][0] * x1_op.segments[s1][1], "l1": l1}
+        gid, gpaths = found
+        mask = sum(1 << q for q, p in enumerate(gpaths) if p in have)
+        w_offs = [w_off[have[p][0]] if p in have else 0 for p in gpaths]
+        out_offs = [out_off[have[p][1]] if p in have else 0 for p in gpaths]
+        g = {"id": gid, "x1_off": x1_off[s1], "w_off": w_offs, "out_off": out_offs, "npath": len(gpaths), "mask": mask,
+             "out_segs": [so for _, _, _, _, so, _ in plist], "x1_width": x1_op.segments[s1][0] * x1_op.segments[s1][1], "l1": l1}
         # backward: one table entry per non-zero (i, k) pair, i-major
         start, tj, tc = [0], [], []
-        for l1_, l2, l3, _, _, c in plist:
-            for i, k, terms in pair_pattern(l1_, l2, l3, "i"):
+        for l2, l3 in gpaths:
+            c = have[(l2, l3)][2] if (l2, l3) in have else None
+            for i, k, terms in pair_pattern(l1, l2, l3, "i"):
                 for j, _ref in terms:
-                    tj.append(x2_off[l2] + j)
-                    tc.append(float(c[i, j, k]))
+                    # every entry keeps its terms (the kernels number the coefficients); absent paths multiply by zero
+                    tj.append(x2_off[l2] + j if c is not None else 0)
+                    tc.append(float(c[i, j, k]) if c is not None else 0.0)
                 start.append(len(tj))
         g["bwd_tab"] = (start, tj, tc)
         # forward: one entry per distinct value (see value_pattern); the descriptor's coefficient of a value is
         # read off the first pair that carries it
         start, tj, tc = [0], [], []
-        for l1_, l2, l3, _, _, c in plist:
-            values, pairs = value_pattern(l1_, l2, l3)
+        for l2, l3 in gpaths:
+            c = have[(l2, l3)][2] if (l2, l3) in have else None
+            values, pairs = value_pattern(l1, l2, l3)
             first = {}
             for i, k, s, sign in pairs:
                 first.setdefault(s, (i, k, sign))
             for s, terms in enumerate(values):
                 i, k, sign = first[s]
                 for j, _ref in terms:
-                    tj.append(x2_off[l2] + j)
-                    tc.append(sign * float(c[i, j, k]))
+                    tj.append(x2_off[l2] + j if c is not None else 0)
+                    tc.append(sign * float(c[i, j, k]) if c is not None else 0.0)
                 start.append(len(tj))
         g["fwd_tab"] = (start, tj, tc)
         g["nterm"] = len(g["bwd_tab"][1])
@@ -294,6 +292,19 @@ def _is_mul_ir(layout, blocks) -> Optional[bool]:
     return True if tuple(layout) == tuple(blocks) else None
 
 
+def _common_layout(x1_layout, x1_blocks, out_layout, out_blocks) -> Optional[bool]:
+    """mul_ir (True) or ir_mul (False) when both operands are held that way, else None.  Rows of scalars only are
+    the same in both layouts and follow the other operand."""
+    a, b = _is_mul_ir(x1_layout, x1_blocks), _is_mul_ir(out_layout, out_blocks)
+    if a is None or b is None:
+        return None
+    if a != b and not a and all(d == 1 for _, d in x1_blocks):
+        return b
+    if a != b and not b and all(d == 1 for _, d in out_blocks):
+        return a
+    return a if a == b else None
+
+
 class _ChannelwiseBase:
     def __init__(self, plan: ChannelwisePlan):
         self.plan = plan
@@ -304,14 +315,16 @@ class _ChannelwiseBase:
         from . import _lib
 
         plan = self.plan
-        if program.math_dtype != torch.float32 or any(x.dtype != torch.float32 for x in xs):
+        if program.math_dtype not in (torch.float32, torch.float64) or any(x.dtype != program.math_dtype for x in xs):
+            return None
+        if plan.extent % 4 and program.math_dtype == torch.float32:
             return None
         w_s, x1_s, x2_s = cfg.inputs[0], cfg.inputs[1], cfg.inputs[2]
         if w_s.mode != _lib.BATCHED or x2_s.mode != _lib.BATCHED or x1_s.mode == _lib.SHARED:
             return None
         if cfg.layout(0) is not None or cfg.layout(2) is not None:
             return None
-        x1_mul_ir = _is_mul_ir(cfg.layout(1), plan.x1_blocks)
+        x1_mul_ir = _common_layout(cfg.layout(1), plan.x1_blocks, cfg.layout(3), plan.out_blocks)
         if x1_mul_ir is None or any(x.data_ptr() % 16 for x in xs):
             return None
         senders = _CSR.int32(x1_s.index) if x1_s.mode == _lib.INDEXED else None
@@ -346,8 +359,11 @@ class _ChannelwiseBase:
         from . import _lib
 
         plan = self.plan
+        import torch
+
+        f64 = tensors["w"].dtype == torch.float64
         cache = g.setdefault("_arg_templates", {})
-        tmpl = cache.get(which)
+        tmpl = cache.get((which, f64))
         if tmpl is None:
             t = _lib.CwArgs()
             t.w_stride, t.x1_stride, t.x2_stride, t.out_stride = plan.row_sizes
@@ -359,11 +375,12 @@ class _ChannelwiseBase:
                 t.w_offset[q] = g["w_off"][q]
                 t.out_offset[q] = g["out_off"][q]
             keep = None
+            t.path_mask, t.x2_width, t.dtype = g["mask"], plan.row_sizes[2], _lib.F64 if f64 else _lib.F32
             if which == "bwd_tab":
-                keep = (C.c_float * g["nterm"])(*g["bwd_tab"][2])
-                t.bwd_coef = C.cast(keep, C.POINTER(C.c_float))
+                keep = ((C.c_double if f64 else C.c_float) * g["nterm"])(*g["bwd_tab"][2])
+                t.bwd_coef = C.cast(keep, C.c_void_p)
             tmpl = (bytes(t), keep)
-            cache[which] = tmpl
+            cache[(which, f64)] = tmpl
         a = _lib.CwArgs.from_buffer_copy(tmpl[0])
         for k, t in tensors.items():
             if t is not None and t.numel():
@@ -389,7 +406,7 @@ class _ChannelwiseBase:
         # the scalar-x1 group is the one where four channels per lane fit the register budget and pay off
         # (config 3: forward 0.58 -> 0.46 ms, backward 1.15 -> 1.00 ms; every other group is slower with four)
         a.channels_per_lane = CHANNELS_PER_LANE or (4 if g.get("l1") == 0 and plan.extent % 128 == 0 else 0)
-        a.staging = STAGING if which == "fwd_tab" else 0
+        a.staging = STAGING if which == "fwd_tab" and not f64 else 0
         a.variant = BWD_VARIANT if which == "bwd_tab" else 0
         if a.staging:
             a.status = _lib.status_word(tensors["w"].device).data_ptr()
@@ -406,7 +423,7 @@ class _ChannelwiseBase:
         from . import _lib, profiling
 
         order, rowptr, nrecv = csr
-        g, t = self.plan.groups[gi], self.plan.tables_on(w.device)[gi]
+        g, t = self.plan.groups[gi], self.plan.tables_on(w.device, w.dtype)[gi]
         stream = C.c_void_p(torch.cuda.current_stream(w.device).cuda_stream)
         with torch.cuda.device(w.device):
             a, _ = self._args(g, t, "fwd_tab", common, order, rowptr, nrecv, mul_ir, dict(w=w, x1=x1_block, x2=x2, out=out), x1_is_block=True)
@@ -421,7 +438,7 @@ class _ChannelwiseBase:
         from . import _lib, profiling
 
         order, rowptr, nrecv = csr
-        g, t = self.plan.groups[gi], self.plan.tables_on(w.device)[gi]
+        g, t = self.plan.groups[gi], self.plan.tables_on(w.device, w.dtype)[gi]
         stream = C.c_void_p(torch.cuda.current_stream(w.device).cuda_stream)
         with torch.cuda.device(w.device):
             a, keep = self._args(g, t, "bwd_tab", common, order, rowptr, nrecv, mul_ir,
@@ -439,8 +456,8 @@ class _ChannelwiseBase:
 
         plan = self.plan
         order, rowptr, nrecv = csr
-        out = torch.empty((nrecv, plan.row_sizes[3]), dtype=torch.float32, device=w.device)
-        tabs = plan.tables_on(w.device)
+        out = torch.empty((nrecv, plan.row_sizes[3]), dtype=w.dtype, device=w.device)
+        tabs = plan.tables_on(w.device, w.dtype)
         stream = C.c_void_p(torch.cuda.current_stream(w.device).cuda_stream)
         with torch.cuda.device(w.device):
             for g, t in zip(plan.groups, tabs):
@@ -467,7 +484,7 @@ class _ChannelwiseBase:
         gw = torch.empty_like(w) if needs[0] else None
         gx1 = torch.zeros_like(x1) if needs[1] else None
         gx2 = torch.zeros_like(x2) if needs[2] else None
-        tabs = plan.tables_on(dev)
+        tabs = plan.tables_on(dev, w.dtype)
         stream = C.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
         with torch.cuda.device(dev):
             for g, t in zip(plan.groups, tabs):
@@ -488,11 +505,10 @@ class ChannelwiseForward(_ChannelwiseBase):
         common = self._common(program, cfg, xs, 3)
         if common is None:
             return None
-        out_mul_ir = _is_mul_ir(cfg.layout(3), self.plan.out_blocks)
         csr = self._csr(cfg.outputs[0], cfg.batch, xs[0].device)
-        if out_mul_ir is None or csr is None or out_mul_ir != common["x1_mul_ir"]:
+        if csr is None:
             return None
-        return [self._launch_forward(common, csr, out_mul_ir, *xs)]
+        return [self._launch_forward(common, csr, common["x1_mul_ir"], *xs)]
 
     def derive(self, requires_gradient, has_cotangent):
         if not has_cotangent[0]:
@@ -512,16 +528,15 @@ class ChannelwiseBackward(_ChannelwiseBase):
         common = self._common(program, cfg, xs, n_in)
         if common is None:
             return None
-        out_mul_ir = _is_mul_ir(cfg.layout(3), self.plan.out_blocks)
         csr = self._csr(cfg.inputs[3], cfg.batch, xs[0].device)
-        if out_mul_ir is None or csr is None or out_mul_ir != common["x1_mul_ir"]:
+        if csr is None:
             return None
         for k, i in grad_specs:  # gradient layouts and addressing must mirror their inputs
             if cfg.layout(n_in + k) != cfg.layout(i) or cfg.outputs[k].mode != cfg.inputs[i].mode:
                 return None
             if cfg.outputs[k].index is not cfg.inputs[i].index:
                 return None
-        return common, csr, out_mul_ir
+        return common, csr, common["x1_mul_ir"]
 
     def try_run(self, program, cfg, xs):
         wanted = [i for i, n in enumerate(self.needs) if n]
@@ -611,11 +626,7 @@ class ChannelwiseSecondOrder(ChannelwiseBackward):
 
 
 def attach_specialisation(program) -> None:
-    """Routes a matching program to the channelwise kernels (float32 math only)."""
-    import torch
-
-    if program.math_dtype != torch.float32:
-        return
+    """Routes a matching program to the channelwise kernels."""
     plan = match_channelwise(program.original)
     if plan is not None:
         program._special = ChannelwiseForward(plan)

@@ -1,0 +1,4 @@
+// Channelwise kernels of the paths that read an irrep of degree 1, float64.
+#include "cw_kernels.cuh"
+
+CW_DEFINE_GROUP_F64(kGroupL1F64, CW_GROUP_L1)

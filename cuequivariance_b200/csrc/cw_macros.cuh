@@ -3,31 +3,31 @@
 // one value per channel.
 #pragma once
 
-template <int C>
-__device__ __forceinline__ void cw_mul(float (&d)[C], float s, const float (&a)[C]) {
+template <int C, class T>
+__device__ __forceinline__ void cw_mul(T (&d)[C], T s, const T (&a)[C]) {
 #pragma unroll
   for (int c = 0; c < C; ++c) d[c] = s * a[c];
 }
-template <int C>
-__device__ __forceinline__ void cw_fma(float (&d)[C], float s, const float (&a)[C]) {
+template <int C, class T>
+__device__ __forceinline__ void cw_fma(T (&d)[C], T s, const T (&a)[C]) {
 #pragma unroll
-  for (int c = 0; c < C; ++c) d[c] = fmaf(s, a[c], d[c]);
+  for (int c = 0; c < C; ++c) d[c] = fma(s, a[c], d[c]);
 }
-template <int C>
-__device__ __forceinline__ void cw_mulv(float (&d)[C], const float (&a)[C], const float (&b)[C]) {
+template <int C, class T>
+__device__ __forceinline__ void cw_mulv(T (&d)[C], const T (&a)[C], const T (&b)[C]) {
 #pragma unroll
   for (int c = 0; c < C; ++c) d[c] = a[c] * b[c];
 }
-template <int C>
-__device__ __forceinline__ void cw_fmav(float (&d)[C], const float (&a)[C], const float (&b)[C]) {
+template <int C, class T>
+__device__ __forceinline__ void cw_fmav(T (&d)[C], const T (&a)[C], const T (&b)[C]) {
 #pragma unroll
-  for (int c = 0; c < C; ++c) d[c] = fmaf(a[c], b[c], d[c]);
+  for (int c = 0; c < C; ++c) d[c] = fma(a[c], b[c], d[c]);
 }
-template <int C>
-__device__ __forceinline__ float cw_dot(const float (&a)[C], const float (&b)[C]) {
-  float v = a[0] * b[0];
+template <int C, class T>
+__device__ __forceinline__ T cw_dot(const T (&a)[C], const T (&b)[C]) {
+  T v = a[0] * b[0];
 #pragma unroll
-  for (int c = 1; c < C; ++c) v = fmaf(a[c], b[c], v);
+  for (int c = 1; c < C; ++c) v = fma(a[c], b[c], v);
   return v;
 }
 #define CW_MUL4(d, s, a) cw_mul(d, s, a)
@@ -49,5 +49,15 @@ __device__ __forceinline__ void cw_load_m(const float* __restrict__ M, float (&m
     if (a + 1 >= Q0 && a + 1 < Q0 + N) m[a + 1 - Q0] = v.y;
     if (a + 2 >= Q0 && a + 2 < Q0 + N) m[a + 2 - Q0] = v.z;
     if (a + 3 >= Q0 && a + 3 < Q0 + N) m[a + 3 - Q0] = v.w;
+  }
+}
+template <int Q0, int N>
+__device__ __forceinline__ void cw_load_m(const double* __restrict__ M, double (&m)[N]) {
+  constexpr int A0 = Q0 & ~1, A1 = (Q0 + N + 1) & ~1;
+#pragma unroll
+  for (int a = A0; a < A1; a += 2) {
+    const double2 v = *reinterpret_cast<const double2*>(M + a);
+    if (a + 0 >= Q0 && a + 0 < Q0 + N) m[a + 0 - Q0] = v.x;
+    if (a + 1 >= Q0 && a + 1 < Q0 + N) m[a + 1 - Q0] = v.y;
   }
 }

@@ -27,7 +27,7 @@ sys.path.insert(0, os.path.dirname(os.path.dirname(HERE)))
 
 import numpy as np  # noqa: E402
 
-from cuequivariance_b200.channelwise import group_signature as _signature, pair_pattern, split_group, value_pattern  # noqa: E402
+from cuequivariance_b200.channelwise import group_signature as _signature, pair_pattern, value_pattern  # noqa: E402
 
 # Groups to build: (l1, [(l2, l3), ...]).  The list below is the family used by MACE-style
 # models: second operand 0e+1o+..+L2 (spherical harmonics), outputs filtered to natural
@@ -89,14 +89,14 @@ def emit_group(l1: int, paths) -> str:
 
     # ---- forward ------------------------------------------------------------------------
     A("  // acc[out_offset(p) + k][c] += W[p][c] * sum_i (+-)V[slot(i,k)] * X[i][c];  V = the distinct values of M")
-    A("  template <int P, int C>")
-    A("  __device__ __forceinline__ static void fwd_path(const float (&X)[D1][C], const float (&W)[C], const float* __restrict__ M,")
-    A("                                                  float (&acc)[SUMD3][C]) {")
+    A("  template <int P, int C, class T>")
+    A("  __device__ __forceinline__ static void fwd_path(const T (&X)[D1][C], const T (&W)[C], const T* __restrict__ M,")
+    A("                                                  T (&acc)[SUMD3][C]) {")
     for p, (pat, d3) in enumerate(zip(pats, d3s)):
         A(f"    if constexpr (P == {p}) {{")
         # load the distinct values of this path as float4 where aligned
         values, vpairs = vals[p]
-        A(f"      float m[{len(values)}];")
+        A(f"      T m[{len(values)}];")
         A(f"      cw_load_m<{val_off[p]}, {len(values)}>(M, m);")
         by_i2: dict[int, list] = {}
         for (i, k, s, sign) in vpairs:
@@ -105,7 +105,7 @@ def emit_group(l1: int, paths) -> str:
             # fewer input than output components: scale the inputs by the weight once (d1 multiplies)
             # and add every product straight into its accumulator, instead of summing unweighted
             # products in temporaries and scaling d3 of them at the end
-            A(f"      float xw[{d1}][C];")
+            A(f"      T xw[{d1}][C];")
             for i in sorted(by_i2):
                 A(f"      CW_MULV4(xw[{i}], W, X[{i}]);")
             for i in sorted(by_i2):
@@ -114,7 +114,7 @@ def emit_group(l1: int, paths) -> str:
         else:
             # i-major emission: consecutive multiply-adds go to different accumulators t[k], so that
             # the chains over i of the d3 outputs interleave instead of running one after the other
-            A(f"      float t[{d3}][C];")
+            A(f"      T t[{d3}][C];")
             seen_k = set()
             for i in sorted(by_i2):
                 for q, k in by_i2[i]:
@@ -133,10 +133,10 @@ def emit_group(l1: int, paths) -> str:
     A("  // per path, pairs ordered by i: S[i] = sum_k M[q] G[k];  gX[i] += W*S[i];  gw = sum_i S[i] X[i];")
     A("  //           r[j] += c * dot4(W*X[i], G[k]) over the non-zero (i, j, k)")
     A("  // NEED_R = false leaves the x2-gradient partials (and the products that only feed them) out")
-    A("  template <int P, int C, bool NEED_R, class Coef>")
-    A("  __device__ __forceinline__ static void bwd_path(const float (&X)[D1][C], const float (&W)[C], const float* __restrict__ M,")
-    A("                                                  const float (&G)[MAXD3][C], const Coef& coef,")
-    A("                                                  float (&gX)[D1][C], float (&gw)[C], float (&r)[16]) {")
+    A("  template <int P, int C, bool NEED_R, class Coef, class T>")
+    A("  __device__ __forceinline__ static void bwd_path(const T (&X)[D1][C], const T (&W)[C], const T* __restrict__ M,")
+    A("                                                  const T (&G)[MAXD3][C], const Coef& coef,")
+    A("                                                  T (&gX)[D1][C], T (&gw)[C], T (&r)[16]) {")
     term_cursor = 0
     for p, (pat, d3, d2) in enumerate(zip(pats_i, d3s, d2s)):
         l2 = paths[p][0]
@@ -144,7 +144,7 @@ def emit_group(l1: int, paths) -> str:
         A(f"    if constexpr (P == {p}) {{")
         q0 = pair_off[p]
         A("#pragma unroll")
-        A("      for (int c = 0; c < C; ++c) gw[c] = 0.f;")
+        A("      for (int c = 0; c < C; ++c) gw[c] = T(0);")
         by_i: dict[int, list] = {}
         for q, (i, k, terms) in enumerate(pat):
             by_i.setdefault(i, []).append((q, k, terms))
@@ -153,7 +153,7 @@ def emit_group(l1: int, paths) -> str:
         scale_g = d3 < d1
         if scale_g:
             ks = sorted({k for lst in by_i.values() for _, k, _ in lst})
-            A(f"      float gs[{d3}][C];")
+            A(f"      T gs[{d3}][C];")
             for k in ks:
                 A(f"      CW_MULV4(gs[{k}], W, G[{k}]);")
         t = term_cursor
@@ -163,12 +163,12 @@ def emit_group(l1: int, paths) -> str:
                 continue
             qa = lst[0][0]
             A("      {")
-            A(f"        float m[{len(lst)}];")
+            A(f"        T m[{len(lst)}];")
             A(f"        cw_load_m<{q0 + qa}, {len(lst)}>(M, m);")
             if scale_g:
-                A("        float s[C];")
+                A("        T s[C];")
             else:
-                A("        float s[C], xw[C];")
+                A("        T s[C], xw[C];")
                 A(f"        CW_MULV4(xw, W, X[{i}]);")
             for n, (q, k, terms) in enumerate(lst):
                 if n == 0:
@@ -176,11 +176,11 @@ def emit_group(l1: int, paths) -> str:
                 else:
                     A(f"        CW_FMA4(s, m[{q - qa}], G[{k}]);")
                 if scale_g:
-                    A(f"        if constexpr (NEED_R) {{ const float v = CW_DOT4(X[{i}], gs[{k}]);")
+                    A(f"        if constexpr (NEED_R) {{ const T v = CW_DOT4(X[{i}], gs[{k}]);")
                 else:
-                    A(f"        if constexpr (NEED_R) {{ const float v = CW_DOT4(xw, G[{k}]);")
+                    A(f"        if constexpr (NEED_R) {{ const T v = CW_DOT4(xw, G[{k}]);")
                 for j, _c in terms:
-                    A(f"          r[{j_base + j}] = fmaf(coef.c[{t}], v, r[{j_base + j}]);")
+                    A(f"          r[{j_base + j}] = fma(coef.c[{t}], v, r[{j_base + j}]);")
                     t += 1
                 A("        }")
             A(f"        CW_FMAV4(gX[{i}], W, s);")
@@ -201,11 +201,10 @@ def all_groups():
             paths = group_paths(l1, L2, L3)
             if not paths:
                 continue
-            for part in split_group(l1, paths):
-                key = (l1, tuple(part))
-                if key not in seen:
-                    seen.add(key)
-                    out.append((l1, part))
+            key = (l1, tuple(paths))
+            if key not in seen:
+                seen.add(key)
+                out.append((l1, paths))
     return out
 
 
@@ -222,8 +221,8 @@ def main():
         parts.append(emit_group(l1, paths))
         parts.append("")
     names = [group_name(l1, p) for l1, p in groups]
-    parts.append("#define CW_FOR_EACH_GROUP(X) \\")
-    parts.append(" \\\n".join(f"  X({n})" for n in names))
+    for (l1, _), n in zip(groups, names):
+        parts.append(f"#define CW_GROUP_L{l1} {n}")
     parts.append("")
     os.makedirs(os.path.join(HERE, "generated"), exist_ok=True)
     path = os.path.join(HERE, "generated", "cw_groups.cuh")

@@ -174,7 +174,7 @@ int cueq_b200_sh_backward(const cueq_sh_args* args, void* stream);
  * Replace the uniform_1d op for the polynomial uv,iu,jv,kuv+ijk of
  * cue.descriptors.channelwise_tensor_product (cuequivariance/group_theory/descriptors/irreps_tp.py:232-321)
  * as called by ChannelWiseTensorProduct.forward (cuequivariance_torch/operations/tp_channel_wise.py:186-258),
- * float32, with the gather of x1 by sender, the scatter-add to receivers and the mul_ir<->ir_mul
+ * float32 or float64, with the gather of x1 by sender, the scatter-add to receivers and the mul_ir<->ir_mul
  * transpositions (tp_channel_wise.py:221-222,258) fused.  One call handles one *group*: the paths
  * that read the same irrep of x1.  Built-in groups are enumerated with cueq_b200_cw_num_groups /
  * cueq_b200_cw_group_signature ("l1:l2.l3,l2.l3,..." in descriptor path order).
@@ -187,7 +187,7 @@ int cueq_b200_sh_backward(const cueq_sh_args* args, void* stream);
  * (i,k) pair, path by path, i-major.  Forward call: one entry per DISTINCT value among a path's pairs
  * (pairs that carry the same combination of x2 up to sign share an entry; order of first appearance in
  * k-major order, first coefficient positive - cuequivariance_b200/channelwise.py:value_pattern).  bwd_coef (host memory,
- * num_terms floats) lists the coefficients in the backward term order. */
+ * num_terms values of the dtype) lists the coefficients in the backward term order. */
 typedef struct {
   const void* w;        /* [E, w_stride]    per-edge weights                                  */
   const void* x1;       /* [N1, x1_stride]  node features                                     */
@@ -202,8 +202,8 @@ typedef struct {
   const int32_t* rowptr;
   const int32_t* tab_start;
   const int32_t* tab_j;
-  const float* tab_c;
-  const float* bwd_coef;
+  const void* tab_c;    /* float or double, by dtype                                            */
+  const void* bwd_coef;
   int64_t w_stride, x1_stride, x2_stride, out_stride; /* row strides in elements               */
   int64_t num_receivers;
   int32_t extent;       /* channels per segment (multiple of 4)                                 */
@@ -225,6 +225,11 @@ typedef struct {
                            3 = as 2, with the x1 gradient of an edge leaving as one bulk reduction
                            (cp.reduce.async.bulk) per warp instead of vector reductions per lane (mul_ir
                            rows, 128 | extent; falls back to 2 where the rows are not 16-byte aligned)        */
+  int32_t path_mask;    /* bit q: path q of the group is part of the polynomial (0: all are); tables and offsets
+                           keep the full group's numbering, entries of absent paths have no terms           */
+  int32_t x2_width;     /* components of an x2 row: 1, 4, 9 or 16 (0: 16)                               */
+  int32_t dtype;        /* CUEQ_F32, or CUEQ_F64: two channels per thread, staging / variant ignored    */
+  int32_t reserved;
 } cueq_cw_args;
 
 int cueq_b200_cw_num_groups(void);
@@ -480,7 +485,7 @@ typedef struct {
   int32_t w_offset[8];
   int32_t out_offset[8];
   int32_t mul_ir;                /* layout of x1 and out, as in cueq_cw_args                         */
-  int32_t reserved;
+  int32_t path_mask;            /* as in cueq_cw_args; x2 rows have 16 components                     */
 } cueq_cw_noalloc_args;
 
 int cueq_b200_cw_forward_noalloc(int group, const cueq_cw_noalloc_args* args, void* stream);
