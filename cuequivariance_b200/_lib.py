@@ -40,7 +40,7 @@ class Buffer(C.Structure):
         ("dtype", C.c_int32),
         ("index", C.c_void_p),
         ("index_is_64", C.c_int32),
-        ("reserved", C.c_int32),
+        ("layout", C.c_int32),
     ]
 
 

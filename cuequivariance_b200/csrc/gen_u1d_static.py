@@ -2,10 +2,18 @@
 polynomial (see ``cuequivariance_b200/static_poly.py``).
 
 Each body evaluates one (row, channel) pair: operand segments are loaded into registers at
-first use, products of two segments of the same buffer are shared between paths, the terms of
-one (output segment, first-operand segment) pair are summed before the multiplication by the
-first operand (typically the weight), and each output segment is handed to a caller-supplied
-sink exactly once.
+first use, products of two segments of the same buffer are shared between paths, and each output
+segment is handed to a caller-supplied sink exactly once.
+
+The sum of an output segment is factored as in Horner's rule for several variables: the factor
+that most of its terms share is taken out, its cofactor and the remainder are treated the same
+way, down to sums of ``coefficient * segment`` or ``coefficient * shared product``, one multiply-add
+per term.  Factors are taken from the buffers that occur once in a term first (cotangent and weight,
+the one with fewer segments first) and from the repeated buffer last, which leaves its products as
+the innermost terms.  These bodies are bound by the FP32 issue rate, so the count of instructions is
+the time; for 0e+1o+2e+3o -> 0e+1o of degree 3, against one product and one multiply-add per term
+and a factored first operand only: forward 1089 -> 747, weight gradient 1155 -> 747, feature gradient
+2664 -> 1786 instructions.
 
     python cuequivariance_b200/csrc/gen_u1d_static.py
 """
@@ -63,56 +71,61 @@ def emit(name: str, poly) -> str:
 
     # accumulate per output segment over ALL operations bound to it
     by_out = {}
+    repeated = set()
     for ope, stp in merged.operations:
         k_out = [k for k, b in enumerate(ope.buffers) if b >= n_in][0]
         j = ope.buffers[k_out] - n_in
         ins = [k for k in range(len(ope.buffers)) if k != k_out]
+        repeated |= {b for b in ope.buffers if ope.buffers.count(b) > 1}
         for p in stp.paths:
             by_out.setdefault((j, p.indices[k_out]), []).append(
-                ([(ope.buffers[k], p.indices[k]) for k in ins], float(p.coefficients)))
+                (sorted((ope.buffers[k], p.indices[k]) for k in ins), float(p.coefficients)))
+    order = sorted(range(n_in), key=lambda b: (b in repeated, merged.inputs[b].num_segments))
     tmp = 0
-    for (j, so), terms in sorted(by_out.items()):
-        # group by the first factor (buffer, segment) of each term
-        groups = {}
-        consts = 0.0
-        for factors, c in terms:
-            if not factors:
-                consts += c
-                continue
-            groups.setdefault(factors[0], []).append((factors[1:], c))
-        B.append("    {")
-        B.append("      float acc = %s;" % fl(consts))
-        for (b0, s0), rest in groups.items():
-            inner = f"t{tmp}"
-            tmp += 1
-            first = True
-            for factors, c in rest:
-                # product of the remaining factors
-                fs = list(factors)
-                expr = None
-                while fs:
-                    if len(fs) >= 2 and fs[0][0] == fs[1][0]:
-                        e = prod(fs[0][0], fs[0][1], fs[1][1])
-                        fs = fs[2:]
-                    else:
-                        e = seg(*fs[0])
-                        fs = fs[1:]
-                    if expr is None:
-                        expr = e
-                    else:
-                        v = f"q{tmp}"
-                        tmp += 1
-                        B.append(f"      const float {v} = {expr} * {e};")
-                        expr = v
-                if expr is None:
-                    expr = "1.f"
-                if first:
-                    B.append(f"      float {inner} = {fl(c)} * {expr};")
-                    first = False
+
+    def is_leaf(factors):
+        return len(factors) <= 1 or (len(factors) == 2 and factors[0][0] == factors[1][0])
+
+    def accumulate(terms, acc):
+        """Adds the sum of ``terms`` to the variable ``acc`` (None: a new one); returns its name."""
+        nonlocal tmp
+        deep = [f for f, _ in terms if not is_leaf(f)]
+        if not deep:
+            for factors, c in terms:
+                expr = "1.f" if not factors else seg(*factors[0]) if len(factors) == 1 else prod(factors[0][0], factors[0][1], factors[1][1])
+                if acc is None:
+                    acc, tmp = f"t{tmp}", tmp + 1
+                    B.append(f"      float {acc} = {fl(c)} * {expr};")
                 else:
-                    B.append(f"      {inner} = fmaf({fl(c)}, {expr}, {inner});")
-            B.append(f"      acc = fmaf({seg(b0, s0)}, {inner}, acc);")
-        B.append(f"      out({j}, {so}, acc);")
+                    B.append(f"      {acc} = fmaf({fl(c)}, {expr}, {acc});")
+            return acc
+        count = {}
+        for f in deep:
+            for q in dict.fromkeys(map(tuple, f)):
+                count[q] = count.get(q, 0) + 1
+        first = min(order.index(b) for b, _ in count)
+        v = max((q for q in count if q[0] == order[first]), key=lambda q: (count[q], -q[1]))
+        cofactor, rest = [], []
+        for f, c in terms:
+            if v in f:
+                f = list(f)
+                f.remove(v)
+                cofactor.append((f, c))
+            else:
+                rest.append((f, c))
+        inner = accumulate(cofactor, None)
+        if acc is None:
+            acc, tmp = f"t{tmp}", tmp + 1
+            B.append(f"      float {acc} = {seg(*v)} * {inner};")
+        else:
+            B.append(f"      {acc} = fmaf({seg(*v)}, {inner}, {acc});")
+        return accumulate(rest, acc) if rest else acc
+
+    # every segment is handed out, zero where no term feeds it: batched outputs are not cleared beforehand
+    for j, so in [(j, so) for j, o in enumerate(merged.outputs) for so in range(o.num_segments)]:
+        B.append("    {")
+        acc = accumulate(by_out[j, so], None) if (j, so) in by_out else "0.f"
+        B.append(f"      out({j}, {so}, {acc});")
         B.append("    }")
         L.extend(B)
         B.clear()

@@ -22,6 +22,7 @@ struct StaticBuf {
   int32_t index_is_64;
   int32_t row_size;  // elements per row
   int32_t vec;       // 1: segments have a channel axis, 0: scalar segments
+  int32_t mul_ir;    // 1: blocks of 1, 3, 5, ... segments, [channel][component] each
 };
 
 struct StaticParams {
@@ -30,8 +31,23 @@ struct StaticParams {
   int32_t extent;
 };
 
+// Segment s of a row of irreps 0, 1, 2, ... (one block each) lies in block l = floor(sqrt(s)), whose first segment
+// is l * l.  The generated code passes s as a literal, so this folds away.
+constexpr int kMaxL = 3;
+__host__ __device__ constexpr int block_of(int s) { return s < 1 ? 0 : s < 4 ? 1 : s < 9 ? 2 : 3; }
+
+// Channel-major buffers are read and written in place.  A thread's components of a block are contiguous, so a warp's
+// reads cover whole lines (the lines stay in L1 between the block's components); a block of an output goes through
+// shared memory, so that every store of a warp is 128 contiguous bytes: stored component by component, each 32-byte
+// sector would be written 2l+1 times.  A separate transposition of the rows in and out cost as much as the smaller
+// kernels themselves: a read and a write of every feature, output and both their gradients.  Bound by the FP32 issue
+// rate: 16,384 atoms x 128 channels of 0e+1o+2e+3o -> 0e+1o, degree 3, forward 93 us, weight gradient 109 us, feature
+// gradient 267 us; the step 470 us, with transposed copies and without the factored sums (gen_u1d_static.py) 820 us.
 template <class K>
 __global__ void __launch_bounds__(128) u1d_static_kernel(const __grid_constant__ StaticParams P) {
+  __shared__ float staging[4][32 * (2 * kMaxL + 1)];
+  float* const stage = staging[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
   const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (gid >= P.batch * P.extent) return;
   const int64_t z = gid / P.extent;
@@ -57,8 +73,29 @@ __global__ void __launch_bounds__(128) u1d_static_kernel(const __grid_constant__
     out_stride[j] = s.vec ? X : 1;
     out_atomic[j] = s.mode != CUEQ_BATCHED || (!s.vec && X > 1);
   }
-  auto in = [&](int b, int s) -> float { return __ldg(in_base[b] + s * in_stride[b]); };
+  auto in = [&](int b, int s) -> float {
+    const int l = block_of(s), first = l * l;
+    // in_base already points at channel u of segment 0
+    if (s < (kMaxL + 1) * (kMaxL + 1) && P.buf[b].mul_ir) return __ldg(in_base[b] + first * X + u * (2 * l) + (s - first));
+    return __ldg(in_base[b] + s * in_stride[b]);
+  };
+  float block[2 * kMaxL + 1];   // components of the output block being collected (constant indices only)
   auto out = [&](int j, int s, float v) {
+    const int l = block_of(s), first = l * l, d = 2 * l + 1;
+    if (s < (kMaxL + 1) * (kMaxL + 1) && P.buf[K::NUM_INPUTS + j].mul_ir) {
+      // X is a multiple of 32: the lanes of a warp hold 32 consecutive channels of one row, all or none of them here
+      block[s - first] = v;
+      if (s - first == d - 1) {
+#pragma unroll
+        for (int i = 0; i < d; ++i) stage[lane * d + i] = block[i];
+        __syncwarp();
+        float* p = out_base[j] + first * X + (u - lane) * (2 * l);   // the warp's run of the block, at this lane (out_base is at u)
+#pragma unroll
+        for (int t = 0; t < d; ++t) p[t * 32] = stage[t * 32 + lane];
+        __syncwarp();
+      }
+      return;
+    }
     float* p = out_base[j] + s * out_stride[j];
     if (out_atomic[j]) atomicAdd(p, v); else *p = v;
   };
@@ -110,6 +147,15 @@ extern "C" int cueq_b200_u1d_static_launch(int id, int64_t batch, int32_t extent
     if (s.mode == CUEQ_INDEXED && !s.index && batch > 0) return cueq::fail("u1d_static: indexed buffer %d has no index", b);
     P.buf[b].ptr = s.ptr; P.buf[b].index = s.index; P.buf[b].mode = s.mode; P.buf[b].index_is_64 = s.index_is_64;
     P.buf[b].vec = buffer_dim[b];
+    if (s.layout != 0 && s.layout != 1) return cueq::fail("u1d_static: buffer %d has invalid layout", b);
+    P.buf[b].mul_ir = s.layout;
+    if (s.layout) {
+      const int n = buffer_num_segments[b];
+      if (!buffer_dim[b] || (n != 1 && n != 4 && n != 9 && n != 16))
+        return cueq::fail("u1d_static: buffer %d cannot be channel-major (%d segments, channel axis %d)", b, n, buffer_dim[b]);
+      if (b >= e.num_inputs && (s.mode != CUEQ_BATCHED || extent % 32))
+        return cueq::fail("u1d_static: a channel-major output has to be batched with an extent that is a multiple of 32");
+    }
     P.buf[b].row_size = buffer_num_segments[b] * (buffer_dim[b] ? extent : 1);
   }
   if (batch == 0) return 0;

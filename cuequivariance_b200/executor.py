@@ -267,26 +267,37 @@ class StaticKernel:
     def __init__(self, kernel_id: int, name: str):
         self.kernel_id, self.name = kernel_id, name
 
+    @staticmethod
+    def _in_place(program: "Uniform1dProgram", cfg: CallConfig, b: int) -> bool:
+        """Whether the kernels address channel-major buffer ``b`` as it is: one block of each degree 0, 1, 2, ..., and for
+        an output whole warps on one row."""
+        n = program.num_inputs
+        natural = tuple((program.extent, 2 * l + 1) for l in range(len(cfg.layout(b))))  # noqa: E741
+        if not program.buffer_dim[b] or cfg.layout(b) != natural or len(natural) > 4 or program.buffer_num_segments[b] != len(natural) ** 2:
+            return False
+        return b < n or (cfg.outputs[b - n].mode == _lib.BATCHED and program.extent % 32 == 0)
+
     def try_run(self, program: "Uniform1dProgram", cfg: CallConfig, xs):
         from . import profiling
+        from .transpose import transpose_blocks
 
         if program.math_dtype != torch.float32 or any(x.dtype != torch.float32 for x in xs):
             return None
-        if any(cfg.layout(b) is not None for b in range(program.num_inputs + program.num_outputs)):
-            return None
         device = xs[0].device
+        nb = program.num_inputs + program.num_outputs
+        in_place = [cfg.layout(b) is not None and self._in_place(program, cfg, b) for b in range(nb)]
+        xs = [x if cfg.layout(i) is None or in_place[i] else transpose_blocks(x, cfg.layout(i), to_ir_mul=True) for i, x in enumerate(xs)]
         outs = [
             torch.zeros((spec.rows, program.row_sizes[program.num_inputs + j]), dtype=torch.float32, device=device)
             if spec.mode != _lib.BATCHED or program.buffer_dim[program.num_inputs + j] == 0
             else torch.empty((spec.rows, program.row_sizes[program.num_inputs + j]), dtype=torch.float32, device=device)
             for j, spec in enumerate(cfg.outputs)
         ]
-        nb = program.num_inputs + program.num_outputs
         bufs = (_lib.Buffer * nb)()
         keep = []
         for b, (t, spec) in enumerate(zip(list(xs) + outs, cfg.inputs + cfg.outputs)):
             bufs[b].ptr = t.data_ptr() if t.numel() else None
-            bufs[b].rows, bufs[b].mode, bufs[b].dtype = spec.rows, spec.mode, _lib.F32
+            bufs[b].rows, bufs[b].mode, bufs[b].dtype, bufs[b].layout = spec.rows, spec.mode, _lib.F32, int(in_place[b])
             if spec.mode == _lib.INDEXED:
                 idx = spec.index.contiguous()
                 keep.append(idx)
@@ -297,13 +308,22 @@ class StaticKernel:
             _lib.check(_lib.lib().cueq_b200_u1d_static_launch(
                 self.kernel_id, cfg.batch, program.extent, bufs, _lib.int32_array(program.buffer_dim),
                 _lib.int32_array(program.buffer_num_segments), nb, stream))
+        for j in range(program.num_outputs):
+            b = program.num_inputs + j
+            if cfg.layout(b) is not None and not in_place[b]:
+                outs[j] = transpose_blocks(outs[j], cfg.layout(b), to_ir_mul=False)
         return outs
 
     def derive(self, requires_gradient, has_cotangent):
         return None  # the derivative program is matched by its own digest
 
 
-SPLIT_STATIC_GRADIENTS = True   # one launch per gradient where each has a build-time kernel (see PolynomialFunction.backward)
+# One launch per gradient instead of one for all, where each gradient has a build-time kernel: for polynomials of more
+# than this many paths on more than this many (row, channel) pairs.  The two gradients of the largest symmetric
+# contraction (0e+1o+2e+3o -> 0e+1o, degree 3: 4,078 paths) take 209 registers together: 404 us against 269 + 110 us at
+# 16,384 x 128.  Smaller polynomials fit (the next one needs 80), and on few rows the launch itself is the time
+# (213 x 64: 288 us against 390 us per step).
+SPLIT_STATIC_PATHS, SPLIT_STATIC_ROWS = 1000, 1 << 18
 
 
 def attach_static(program: "Uniform1dProgram") -> None:
@@ -409,10 +429,8 @@ class PolynomialFunction(torch.autograd.Function):
             for j, g in enumerate(grad_outputs):
                 if g is not None:
                     cots.append(g.contiguous())
-            # A build-time straight-line kernel that produces several gradients at once can need more registers
-            # than a thread has (the symmetric contraction's weight + input gradient spills 0.8 KB per thread);
-            # where every single gradient has a straight-line kernel of its own, one launch per gradient is faster.
-            if SPLIT_STATIC_GRADIENTS and sum(needs) > 1 and isinstance(dprog._special, StaticKernel):
+            if (sum(needs) > 1 and isinstance(dprog._special, StaticKernel) and cfg.batch * dprog.extent >= SPLIT_STATIC_ROWS
+                    and sum(d.num_paths for _, d in dprog.flat.operations) > SPLIT_STATIC_PATHS):
                 singles = []
                 for i, n in enumerate(needs):
                     if n:

@@ -64,6 +64,9 @@ class SymmetricContraction(torch.nn.Module):
         self.method = "uniform_1d"
         self.transpose_in = TransposeIrrepsLayout(irreps_in, source=IrrepsLayout.parse(layout_in or layout), target=self.etp.inputs[1].layout, device=device)
         self.transpose_out = TransposeIrrepsLayout(irreps_out, source=self.etp.outputs[0].layout, target=IrrepsLayout.parse(layout_out or layout), device=device)
+        # the build-time kernels read and write mul_ir rows in place; everything else gets transposed copies
+        self._layouts = {b: tuple((m, ir.dim) for m, ir in irreps) for b, irreps, t in
+                         ((1, irreps_in, self.transpose_in), (2, irreps_out, self.transpose_out)) if t.f is not None}
         self.f = SegmentedPolynomial(self.etp.polynomial, method=self.method, math_dtype=math_dtype, name="symmetric_contraction")
 
     def extra_repr(self) -> str:
@@ -74,5 +77,7 @@ class SymmetricContraction(torch.nn.Module):
             weight = torch.einsum("zau,ab->zbu", self.weight, self.projection)
         else:
             weight = self.weight
+        if self._layouts and x.dtype == weight.dtype == torch.float32 and self.f.has_static_kernel(torch.float32):
+            return self.f([weight.flatten(1), x], input_indices={0: indices}, layouts=self._layouts)[0]
         out = self.f([weight.flatten(1), self.transpose_in(x)], input_indices={0: indices})
         return self.transpose_out(out[0])

@@ -131,6 +131,12 @@ class SegmentedPolynomial(nn.Module):
             self._programs[math_dtype] = prog
         return prog
 
+    def has_static_kernel(self, dtype: torch.dtype) -> bool:
+        """Whether a call whose operands all have this dtype runs on a kernel written out at build time."""
+        from .executor import StaticKernel
+
+        return self.math_dtype in (None, dtype) and isinstance(getattr(self._program(dtype), "_special", None), StaticKernel)
+
     def __reduce__(self):
         return (
             SegmentedPolynomial,

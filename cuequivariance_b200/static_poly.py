@@ -65,15 +65,21 @@ def digest(poly: Polynomial) -> str:
 
 
 def registered_polynomials() -> List[Tuple[str, Polynomial]]:
-    """(name, flattened polynomial) of everything that gets a static kernel: the MACE
-    symmetric contraction 0e+1o+2e+3o -> 0e+1o of degree 3 and its first derivatives."""
+    """(name, flattened polynomial) of everything that gets a static kernel: the MACE symmetric contractions
+    0e+1o[+2e[+3o]] -> 0e[+1o] of degree 2 and 3 - the shapes whose path tables ship with the package, so that the
+    digest cannot depend on the host that evaluates it - and their first derivatives, each alone and both together."""
     from . import descriptors
 
     out = []
-    e, _ = descriptors.symmetric_contraction("4x0e+4x1o+4x2e+4x3o", "4x0e+4x1o", (1, 2, 3))
-    fwd = e.polynomial.flatten_coefficient_modes().squeeze_modes()
-    out.append(("sc_l3_l1_d3_fwd", fwd))
-    out.append(("sc_l3_l1_d3_bwd_wx", fwd.backward([True, True], [True])))
-    out.append(("sc_l3_l1_d3_bwd_x", fwd.backward([False, True], [True])))
-    out.append(("sc_l3_l1_d3_bwd_w", fwd.backward([True, False], [True])))
+    for l_in in (1, 2, 3):
+        for l_out in (0, 1):
+            for degree in (2, 3):
+                irreps = ["+".join(f"4x{l}{'eo'[l % 2]}" for l in range(n + 1)) for n in (l_in, l_out)]  # noqa: E741
+                e, _ = descriptors.symmetric_contraction(*irreps, tuple(range(1, degree + 1)))
+                fwd = e.polynomial.flatten_coefficient_modes().squeeze_modes()
+                name = f"sc_l{l_in}_l{l_out}_d{degree}"
+                out.append((f"{name}_fwd", fwd))
+                out.append((f"{name}_bwd_wx", fwd.backward([True, True], [True])))
+                out.append((f"{name}_bwd_x", fwd.backward([False, True], [True])))
+                out.append((f"{name}_bwd_w", fwd.backward([True, False], [True])))
     return out

@@ -67,7 +67,8 @@ typedef struct {
   int32_t dtype;      /* CUEQ_F32 / F64 / BF16 / F16                                              */
   const void* index;  /* device pointer [batch] when mode == CUEQ_INDEXED, else NULL               */
   int32_t index_is_64; /* 1: int64 indices, 0: int32                                              */
-  int32_t reserved;
+  int32_t layout;     /* 0: segment after segment (ir_mul).  1: channel-major (mul_ir) blocks of 1, 3, 5, ...
+                         segments, [channel][component] each - cueq_b200_u1d_static_launch only           */
 } cueq_buffer;
 
 int cueq_b200_abi_version(void);
@@ -244,7 +245,9 @@ int cueq_b200_cw_backward(int group, const cueq_cw_args* args, void* stream);
  * accumulated with atomics unless batched), for polynomials whose straight-line code was
  * generated when the library was built - the counterpart of the per-polynomial NVRTC kernels of
  * the reference's closed op (CHANGELOG.md:38,49).  `digest` identifies the polynomial
- * (cuequivariance_b200/static_poly.py); _find returns a kernel id or -1. */
+ * (cuequivariance_b200/static_poly.py); _find returns a kernel id or -1.
+ * A buffer may be channel-major (cueq_buffer.layout = 1) when it has a channel axis and 1, 4, 9 or 16 segments;
+ * an output then has to be batched and the extent a multiple of 32. */
 int cueq_b200_u1d_static_find(const char* digest);
 const char* cueq_b200_u1d_static_name(int id);
 int cueq_b200_u1d_static_launch(int id, int64_t batch, int32_t extent, const cueq_buffer* buffers,
