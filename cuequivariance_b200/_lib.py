@@ -168,6 +168,26 @@ class GemmF32x3Args(C.Structure):
     ]
 
 
+class LinearPath(C.Structure):
+    _fields_ = [
+        ("u", C.c_int32), ("v", C.c_int32), ("d", C.c_int32), ("x_off", C.c_int32), ("out_off", C.c_int32), ("w_off", C.c_int32),
+        ("c", C.c_float), ("reserved", C.c_int32),
+    ]
+
+
+LINEAR_MAX_PATHS, LINEAR_MAX_CLASSES = 8, 64
+
+
+class LinearArgs(C.Structure):
+    _fields_ = [
+        ("x", C.c_void_p), ("w", C.c_void_p), ("out", C.c_void_p),
+        ("ldx", C.c_int64), ("ldo", C.c_int64), ("w_class_stride", C.c_int64),
+        ("bounds", C.POINTER(C.c_int32)), ("status", C.c_void_p),
+        ("num_paths", C.c_int32), ("num_classes", C.c_int32), ("x_mul_ir", C.c_int32), ("out_mul_ir", C.c_int32),
+        ("transposed", C.c_int32), ("struct_bytes", C.c_int32), ("paths", LinearPath * LINEAR_MAX_PATHS),
+    ]
+
+
 class GemmF32x3TnArgs(C.Structure):
     _fields_ = [
         ("A", C.c_void_p), ("B", C.c_void_p), ("C", C.c_void_p), ("colsum", C.c_void_p),
@@ -242,6 +262,8 @@ def lib() -> C.CDLL:
     L.cueq_b200_fctp_fused_gw.argtypes = [C.POINTER(FctpFusedGwArgs), C.c_void_p]
     L.cueq_b200_gemm_f32x3.argtypes = [C.POINTER(GemmF32x3Args), C.c_void_p]
     L.cueq_b200_gemm_f32x3_tn.argtypes = [C.POINTER(GemmF32x3TnArgs), C.c_void_p]
+    L.cueq_b200_linear_map.argtypes = [C.POINTER(LinearArgs), C.c_void_p]
+    L.cueq_b200_linear_gw.argtypes = [C.POINTER(LinearArgs), C.c_void_p]
     L.cueq_b200_selftest_bounded_wait.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p]
     if L.cueq_b200_abi_version() != 1:
         raise CueqError("libcueq_b200.so has an unexpected ABI version; rebuild it")

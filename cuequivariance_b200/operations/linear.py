@@ -8,7 +8,7 @@ from typing import Dict, Optional
 
 import torch
 
-from .. import descriptors
+from .. import _lib, descriptors
 from ..irreps import Irreps, IrrepsLayout
 from ..segmented_polynomial import SegmentedPolynomial
 from ..transpose import TransposeIrrepsLayout
@@ -152,6 +152,74 @@ class _GroupedDenseLinear(torch.autograd.Function):
         return None, None, gw, gx
 
 
+def _fused_paths(paths, num_in: int, num_out: int):
+    """What ``cueq_b200_linear_map`` / ``_gw`` need, or None when they do not take the shape: every multiplicity 32, 64,
+    96 or 128, irreps up to l = 3, and no block of rows in more than one path."""
+    if len(paths) > _lib.LINEAR_MAX_PATHS or any(u > 128 or v > 128 or d > 7 for (_, u, v, _, _, d, _) in paths):
+        return None
+    ins, outs = {p[3] for p in paths}, {p[4] for p in paths}
+    if len(ins) != len(paths) or len(outs) != len(paths):
+        return None
+    return {"paths": paths, "full_in": len(ins) == num_in, "full_out": len(outs) == num_out}
+
+
+def _aligned(t: torch.Tensor) -> torch.Tensor:
+    t = t.contiguous()
+    return t.clone() if t.data_ptr() % 16 else t
+
+
+class _FusedLinear(torch.autograd.Function):
+    """All irreps, components and weight classes of the layer in one launch per result (``csrc/linear_fused.cu``); rows stay
+    in the caller's layouts.  ``bounds``: row ranges of the classes, ``(0, rows)`` for one weight set."""
+
+    @staticmethod
+    def _launch(plan, which, bounds, x, w, out, transposed=0):
+        import ctypes as C
+
+        from .. import profiling
+
+        a = _lib.LinearArgs()
+        a.x, a.w, a.out = x.data_ptr(), w.data_ptr(), out.data_ptr()
+        a.bounds = _lib.int32_array(bounds)
+        a.status = _lib.status_word(x.device).data_ptr()
+        a.num_paths, a.num_classes = len(plan["paths"]), len(bounds) - 1
+        a.x_mul_ir, a.out_mul_ir = plan["mul_ir"] if not transposed else plan["mul_ir"][::-1]
+        a.transposed, a.struct_bytes = transposed, C.sizeof(a)
+        a.ldx, a.ldo = x.shape[1], (out if which == "map" else w).shape[1]
+        a.w_class_stride = (w if which == "map" else out).shape[1]
+        for q, (wo, u, v, xo, oo, d, c) in zip(a.paths, plan["paths"]):
+            q.u, q.v, q.d, q.x_off, q.out_off, q.w_off, q.c = u, v, d, xo, oo, wo, c
+        fn = _lib.lib().cueq_b200_linear_map if which == "map" else _lib.lib().cueq_b200_linear_gw
+        name = ("linear" if len(bounds) == 2 else "indexed_linear") + "_f32x3" + ("_gx" if transposed else "" if which == "map" else "_gw")
+        with torch.cuda.device(x.device), profiling.kernel(name):
+            _lib.check(fn(C.byref(a), C.c_void_p(torch.cuda.current_stream(x.device).cuda_stream)))
+
+    @staticmethod
+    def forward(ctx, plan, bounds, weight, x):
+        x, weight = _aligned(x), _aligned(weight)
+        all_rows = bounds[0] == 0 and bounds[-1] == x.shape[0]
+        out = (torch.empty if plan["full_out"] and all_rows else torch.zeros)((x.shape[0], plan["out_size"]), dtype=torch.float32, device=x.device)
+        _FusedLinear._launch(plan, "map", bounds, x, weight, out)
+        ctx.plan, ctx.bounds, ctx.all_rows = plan, bounds, all_rows
+        ctx.save_for_backward(weight, x)
+        return out
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx, gout):
+        plan, bounds = ctx.plan, ctx.bounds
+        weight, x = ctx.saved_tensors
+        gout = _aligned(gout)
+        gw = gx = None
+        if ctx.needs_input_grad[3]:
+            gx = (torch.empty_like if plan["full_in"] and ctx.all_rows else torch.zeros_like)(x)
+            _FusedLinear._launch(plan, "map", bounds, gout, weight, gx, transposed=1)
+        if ctx.needs_input_grad[2]:
+            gw = torch.zeros_like(weight)
+            _FusedLinear._launch(plan, "gw", bounds, x, gout, gw)
+        return None, None, gw, gx
+
+
 class Linear(torch.nn.Module):
     """``forward(x, weight=None, weight_indices=None)``; ``x``: ``[batch, irreps_in.dim]``;
     ``weight``: ``[1 or weight_classes, weight_numel]`` when shared (the module's own parameter
@@ -219,9 +287,13 @@ class Linear(torch.nn.Module):
             u, v = d.operands[0].segments[sw]
             dim = d.operands[1].segments[si][0]
             paths.append((offs[0][sw], u, v, offs[1][si], offs[2][so], dim, float(p.coefficients)))
-        self._dense_plan = None
+        self._dense_plan = self._fused_plan = None
         if paths and all(u % 32 == 0 and v % 32 == 0 for (_, u, v, _, _, _, _) in paths):
             self._dense_plan = {"paths": paths, "out_size": d.operands[2].size}
+            fused = _fused_paths(paths, d.operands[1].num_segments, d.operands[2].num_segments)
+            if fused is not None:
+                mul_ir = (int(self.transpose_in.f is not None), int(self.transpose_out.f is not None))
+                self._fused_plan = {**fused, "out_size": d.operands[2].size, "mul_ir": mul_ir}
         try:
             self.f = SegmentedPolynomial(e.polynomial, method=self.method, math_dtype=math_dtype, name="linear")
             self._generic_error = None
@@ -246,6 +318,15 @@ class Linear(torch.nn.Module):
             input_indices[0] = weight_indices
         if weight is None:
             raise ValueError("Weights should not be None")
+        if self._fused_plan is not None and DENSE_ROUTE and x.is_cuda and x.dim() == 2 and x.dtype == torch.float32 and weight.dtype == torch.float32 \
+                and x.shape[1] == self.irreps_in.dim and weight.shape[1] == self.weight_numel and x.shape[0] < 2**31:
+            if not input_indices and weight.shape[0] == 1 and x.shape[0] >= DENSE_MIN_ROWS:
+                return _FusedLinear.apply(self._fused_plan, (0, x.shape[0]), weight, x)
+            if input_indices and weight.shape[0] == self.weight_classes and self.weight_classes <= _lib.LINEAR_MAX_CLASSES \
+                    and (self.require_grouped or x.shape[0] >= DENSE_MIN_ROWS) and weight_indices.shape[0] == x.shape[0]:
+                bounds = class_bounds(weight_indices, self.weight_classes)
+                if bounds is not None:
+                    return _FusedLinear.apply(self._fused_plan, tuple(bounds), weight, x)
         xin = self.transpose_in(x)
         if (self._dense_plan is not None and DENSE_ROUTE and not input_indices and weight.shape[0] == 1 and xin.is_cuda
                 and xin.dtype == torch.float32 and weight.dtype == torch.float32 and xin.shape[0] >= DENSE_MIN_ROWS):

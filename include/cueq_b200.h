@@ -319,6 +319,37 @@ typedef struct {
 } cueq_gemm_f32x3_tn_args;
 int cueq_b200_gemm_f32x3_tn(const cueq_gemm_f32x3_tn_args* args, void* stream);
 
+/* Equivariant linear layer, all irreps and weight classes in one launch, in the accuracy of the GEMMs above
+ * (cuequivariance_torch/operations/linear.py:30-191; with classes primitives/segmented_polynomial_indexed_linear.py:116-156).
+ * A path maps u copies of an irrep of dimension d (1, 3, 5 or 7) onto v copies; u and v are 32, 64, 96 or 128, no two
+ * paths share a block of rows, offsets are in elements.  Class k owns the rows bounds[k] <= z < bounds[k + 1] and the
+ * weights at w + k * w_class_stride.
+ * linear_map: out[z, v, i] = c * sum_u W[u, v] x[z, u, i]; with `transposed` the input gradient: `x` holds the cotangent
+ *   rows (addressed by out_off), `out` the gradient rows (addressed by x_off).
+ * linear_gw:  out (the weight gradient, zeroed by the caller) [u, v] += c * sum_{z, i} x[z, u, i] g[z, v, i]; `w` = g. */
+#define CUEQ_LINEAR_MAX_PATHS 8
+#define CUEQ_LINEAR_MAX_CLASSES 64
+typedef struct {
+  int32_t u, v, d, x_off, out_off, w_off;
+  float c;
+  int32_t reserved;
+} cueq_linear_path;
+typedef struct {
+  const void* x;        /* device float32 [rows, ldx]                                              */
+  const void* w;        /* device float32 weights (linear_map) or g rows [rows, ldo] (linear_gw)   */
+  void* out;            /* device float32 [rows, ldo] (linear_map) or weight gradient (linear_gw)  */
+  int64_t ldx, ldo, w_class_stride;
+  const int32_t* bounds; /* host [num_classes + 1], ascending                                      */
+  void* status;         /* nullable device int32: 2 if a bounded wait ran out                      */
+  int32_t num_paths, num_classes;
+  int32_t x_mul_ir, out_mul_ir;   /* layouts of the rows `x` and of the rows `out` / `g`           */
+  int32_t transposed;
+  int32_t struct_bytes; /* sizeof(cueq_linear_args) as the caller declares it                      */
+  cueq_linear_path paths[CUEQ_LINEAR_MAX_PATHS];
+} cueq_linear_args;
+int cueq_b200_linear_map(const cueq_linear_args* args, void* stream);
+int cueq_b200_linear_gw(const cueq_linear_args* args, void* stream);
+
 /* ---- fully connected ("uvw") tensor product: kernels around the tensor-core GEMM -----------------
  *
  * For one path of uvw,iu,jv,kw+ijk (cue.descriptors.fully_connected_tensor_product,
