@@ -168,6 +168,26 @@ class GemmF32x3Args(C.Structure):
     ]
 
 
+FCTP_TRI_MAX_PATHS = 24
+
+
+class FctpTriPath(C.Structure):
+    _fields_ = [
+        ("a_src", C.c_int32), ("a_off", C.c_int32), ("na", C.c_int32), ("q_src", C.c_int32), ("q_off", C.c_int32), ("nb", C.c_int32),
+        ("b_row0", C.c_int32), ("coef", C.c_float * 125),
+    ]
+
+
+class FctpTriArgs(C.Structure):
+    _fields_ = [
+        ("a", C.c_void_p * 2), ("qt", C.c_void_p * 2), ("b_hi", C.c_void_p), ("b_lo", C.c_void_p), ("out", C.c_void_p),
+        ("paths", C.POINTER(FctpTriPath)), ("status", C.c_void_p),
+        ("lda", C.c_int64 * 2), ("zp", C.c_int64), ("b_rows", C.c_int64), ("ldo", C.c_int64), ("batch", C.c_int64),
+        ("dtype", C.c_int32), ("channels", C.c_int32), ("out_off", C.c_int32), ("nc", C.c_int32), ("num_paths", C.c_int32),
+        ("splits", C.c_int32), ("struct_bytes", C.c_int32), ("reserved", C.c_int32),
+    ]
+
+
 class LinearPath(C.Structure):
     _fields_ = [
         ("u", C.c_int32), ("v", C.c_int32), ("d", C.c_int32), ("x_off", C.c_int32), ("out_off", C.c_int32), ("w_off", C.c_int32),
@@ -262,6 +282,10 @@ def lib() -> C.CDLL:
     L.cueq_b200_fctp_fused_gw.argtypes = [C.POINTER(FctpFusedGwArgs), C.c_void_p]
     L.cueq_b200_gemm_f32x3.argtypes = [C.POINTER(GemmF32x3Args), C.c_void_p]
     L.cueq_b200_gemm_f32x3_tn.argtypes = [C.POINTER(GemmF32x3TnArgs), C.c_void_p]
+    L.cueq_b200_fctp_tri.argtypes = [C.POINTER(FctpTriArgs), C.c_void_p]
+    L.cueq_b200_fctp_tri_weights.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int, C.POINTER(C.c_int32), C.POINTER(C.c_int32),
+                                             C.c_void_p, C.c_void_p, C.c_void_p]
+    L.cueq_b200_fctp_tri_transpose.argtypes = [C.c_void_p, C.c_int, C.c_int64, C.c_int32, C.c_int64, C.c_void_p, C.c_int64, C.c_void_p]
     L.cueq_b200_linear_map.argtypes = [C.POINTER(LinearArgs), C.c_void_p]
     L.cueq_b200_linear_gw.argtypes = [C.POINTER(LinearArgs), C.c_void_p]
     L.cueq_b200_selftest_bounded_wait.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p]

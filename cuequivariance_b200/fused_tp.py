@@ -33,6 +33,7 @@ from typing import List, Optional
 import numpy as np
 import torch
 
+from . import _lib
 from .executor import Uniform1dProgram
 from .polynomial import Polynomial
 
@@ -111,7 +112,7 @@ class _TensorCoreUVW(torch.autograd.Function):
     def _launch_build(owner, k, x1, x2, Z, B):
         import ctypes as C
 
-        from . import _lib, profiling
+        from . import profiling
 
         a = owner._fctp_args(k, x1, x2, B)
         a.z = Z.data_ptr()
@@ -124,7 +125,7 @@ class _TensorCoreUVW(torch.autograd.Function):
               c_is_zero=0):
         import ctypes as C
 
-        from . import _lib, profiling
+        from . import profiling
 
         g = _lib.GemmArgs()
         g.A, g.B, g.C = A.data_ptr(), Bm.data_ptr(), Cptr
@@ -141,9 +142,12 @@ class _TensorCoreUVW(torch.autograd.Function):
         d, off = owner.d, owner.offsets
         B = x1.shape[0]
         dev = x1.device
-        from . import _lib
-
         status = _lib.status_word(dev)
+        if FUSED and owner._tri_channels(torch.bfloat16):
+            out = owner.tri_map(2, w, (x1.to(torch.bfloat16), x2.to(torch.bfloat16)), "fctp_fused_forward")
+            ctx.owner, ctx.status = owner, status
+            ctx.save_for_backward(w, x1, x2)
+            return out.to(x1.dtype)
         if FUSED and owner._fused_tasks() is not None:
             out = owner._fused_forward(w, x1, x2, status)
             ctx.owner, ctx.status = owner, status
@@ -173,7 +177,7 @@ class _TensorCoreUVW(torch.autograd.Function):
     def backward(ctx, gout):
         import ctypes as C
 
-        from . import _lib, profiling
+        from . import profiling
 
         owner = ctx.owner
         w, x1, x2 = ctx.saved_tensors
@@ -183,6 +187,13 @@ class _TensorCoreUVW(torch.autograd.Function):
         status = ctx.status
         fused_x = FUSED and owner._fused_tasks() is not None and owner._fused_units(1) is not None and owner._fused_wunits() is not None
         gx1f = gx2f = gwf = None
+        if FUSED and owner._tri_channels(torch.bfloat16) and (need_x1 or need_x2):
+            gout16 = gout.to(torch.bfloat16)
+            if need_x1:
+                gx1f = owner.tri_map(0, w, (x2.to(torch.bfloat16), gout16), "fctp_fused_gx1")
+            if need_x2:
+                gx2f = owner.tri_map(1, w, (x1.to(torch.bfloat16), gout16), "fctp_fused_gx2")
+            need_x1 = need_x2 = False
         if fused_x and (need_x1 or need_x2 or need_w):
             gout16 = gout.to(torch.bfloat16).contiguous()
             x1b, x2b = x1.to(torch.bfloat16).contiguous(), x2.to(torch.bfloat16).contiguous()
@@ -279,14 +290,128 @@ class DenseUVW:
                 return False
         return True
 
+    # -- tri-linear route: the output and both input gradients without a coupled operand ---------
+    def _tri_channels(self, dtype) -> int:
+        """The common multiplicity when ``cueq_b200_fctp_tri`` takes the product in this dtype, else 0."""
+        d = self.d
+        muls = {m for p in d.paths for m in d.operands[0].segments[p.indices[0]]}
+        muls |= {s[1] for op in d.operands[1:] for s in op.segments}
+        if len(muls) != 1 or not d.paths or len(d.paths) > _lib.FCTP_TRI_MAX_PATHS:
+            return 0
+        (c,) = muls
+        if any(n not in (1, 3, 5) for p in d.paths for n in p.coefficients.shape):
+            return 0
+        # bf16 with 64 channels has kernels of its own (fctp_fused.cu), which are faster: 5.4 against 6.2 ms for the output
+        # and both input gradients of 32,768 samples of 64x(0e+1o+2e).  Other shapes used to write the coupled operand to
+        # memory: the same sums in float32 took 23 ms, 10 ms here.
+        return c if c in ((128,) if dtype == torch.bfloat16 else (32, 64, 96)) else 0
+
+    def _tri_plan(self, which: int):
+        """Path tables for the derivative of the trilinear form with respect to operand ``which`` (0: x1, 1: x2, 2: the
+        output's cotangent, i.e. the output itself): per irrep of the result ``(offset, dimension, paths)``, plus the
+        weight offsets and axis orders of all paths and the set of operands that are needed transposed."""
+        key = f"_tri{which}"
+        if hasattr(self, key):
+            return getattr(self, key)
+        d, off = self.d, self.offsets
+        others = [ax for ax in range(3) if ax != which]
+        groups, w_off, order, transposed = {}, [], [], set()
+        for k, p in enumerate(d.paths):
+            sw, segs = p.indices[0], p.indices[1:]
+            dims = p.coefficients.shape
+            a = min(others, key=lambda ax: dims[ax])                 # contracted on the tensor cores, once per component
+            q = others[0] if a == others[1] else others[1]
+            t = _lib.FctpTriPath()
+            t.a_src, t.a_off, t.na = others.index(a), off[1 + a][segs[a]], dims[a]
+            t.q_src, t.q_off, t.nb = others.index(q), off[1 + q][segs[q]], dims[q]
+            c = d.operands[0].segments[sw][0]
+            t.b_row0 = k * c * c
+            coef = p.coefficients.transpose(a, q, which)
+            for i, j, kk in np.ndindex(*coef.shape):
+                t.coef[(i * 5 + j) * 5 + kk] = float(coef[i, j, kk])
+            transposed.add(t.q_src)
+            w_off.append(off[0][sw])
+            order.append(100 * a + 10 * q + which)
+            groups.setdefault(segs[which], []).append(t)
+        launches = [(off[1 + which][s], d.operands[1 + which].segments[s][0], (_lib.FctpTriPath * len(ts))(*ts), len(ts)) for s, ts in groups.items()]
+        launches.sort(key=lambda t: -t[1])
+        full = len(groups) == d.operands[1 + which].num_segments
+        res = (launches, _lib.int32_array(w_off), _lib.int32_array(order), transposed, full)
+        setattr(self, key, res)
+        return res
+
+    @staticmethod
+    def _tri_splits(tiles: int, c: int) -> int:
+        """Into how many thread blocks the sum over q is divided.  A block takes an SM for itself, so ``tiles`` blocks come
+        in waves of 148; a division pays while it fills the last wave (1 % per doubling for the additions)."""
+        nq = 4 if c == 32 else 2
+        valid = [s for s in (1, 2, 4, 8, 16) if c % s == 0 and (c // s) % nq == 0]
+        return min(valid, key=lambda s: -(-tiles * s // 148) / s * (1 + 0.01 * s.bit_length()))
+
+    def tri_map(self, which: int, w, operands, name: str) -> torch.Tensor:
+        """float32 derivative of the trilinear form with respect to operand ``which``; ``operands``: the rows of the two
+        other operands (float32 or both bf16, ir_mul), in the order (x1, x2, cotangent)."""
+        import ctypes as C
+
+        from . import profiling
+        from .executor import dtype_code
+
+        L = _lib.lib()
+        dt = operands[0].dtype
+        c = self._tri_channels(dt)
+        launches, w_off, order, transposed, full = self._tri_plan(which)
+        dev = operands[0].device
+        xs = [x.contiguous() for x in operands]
+        xs = [x.clone() if x.data_ptr() % 16 else x for x in xs]
+        B, bf16 = xs[0].shape[0], dt == torch.bfloat16
+        size = self.d.operands[1 + which].size
+        n = len(self.d.paths)
+        w = w.detach().contiguous()
+        if w.dtype not in (torch.float32, torch.bfloat16):
+            w = w.to(torch.bfloat16 if bf16 else torch.float32)
+        hi = torch.empty((n * c * c, c), dtype=dt, device=dev)
+        lo = None if bf16 else torch.empty_like(hi)
+        step = min(B, max(128, 2**30 // max(x.shape[1] for x in xs) // 128 * 128))   # transposed operands of 4 GB at most
+        rt = c if c <= 64 else c // 2
+        with torch.cuda.device(dev):
+            stream = C.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
+            with profiling.kernel("fctp_tri_weights"):
+                _lib.check(L.cueq_b200_fctp_tri_weights(w.data_ptr(), dtype_code(w.dtype), dtype_code(dt), c, n, w_off, order, hi.data_ptr(),
+                                                        None if lo is None else lo.data_ptr(), stream))
+            tiles = -(-step // 128) * (c // rt)
+            splits = self._tri_splits(tiles, c)
+            out = (torch.empty if full and splits == 1 else torch.zeros)((B, size), dtype=torch.float32, device=dev)
+            for b0 in range(0, B, step):
+                nb = min(step, B - b0)
+                zp = -(-nb // 128) * 128
+                a = _lib.FctpTriArgs()
+                keep = []
+                for s, x in enumerate(xs):
+                    xb = x[b0 : b0 + nb]
+                    a.a[s], a.lda[s] = xb.data_ptr(), x.shape[1]
+                    if s in transposed:
+                        t = torch.empty((x.shape[1], zp), dtype=torch.float32, device=dev)
+                        with profiling.kernel("fctp_tri_transpose"):
+                            _lib.check(L.cueq_b200_fctp_tri_transpose(xb.data_ptr(), dtype_code(dt), nb, x.shape[1], x.shape[1], t.data_ptr(), zp, stream))
+                        a.qt[s] = t.data_ptr()
+                        keep.append(t)
+                a.b_hi, a.b_lo, a.b_rows = hi.data_ptr(), None if lo is None else lo.data_ptr(), hi.shape[0]
+                a.status = _lib.status_word(dev).data_ptr()
+                a.out, a.ldo, a.zp, a.batch = out[b0].data_ptr(), size, zp, nb
+                a.dtype, a.channels, a.splits, a.struct_bytes = dtype_code(dt), c, splits, C.sizeof(a)
+                for o, nc, paths, np_ in launches:
+                    a.out_off, a.nc, a.num_paths = o, nc, np_
+                    a.paths = C.cast(paths, C.POINTER(_lib.FctpTriPath))
+                    with profiling.kernel(name):
+                        _lib.check(L.cueq_b200_fctp_tri(C.byref(a), stream))
+        return out
+
     # -- fused route: coupled operand built in shared memory ------------------------------------
     def _fused_tasks(self):
         """Task table for the fused kernels, or None if the shape is outside what they cover
         (all multiplicities 64, irrep dimensions 1/3/5, at most 4 paths per output irrep)."""
         if hasattr(self, "_tasks"):
             return self._tasks
-        from . import _lib
-
         d, off = self.d, self.offsets
         self._tasks = None
         by_out = {}
@@ -325,8 +450,6 @@ class DenseUVW:
         key = f"_units{which}"
         if hasattr(self, key):
             return getattr(self, key)
-        from . import _lib
-
         d, off = self.d, self.offsets
         units = []
         for p in d.paths:
@@ -357,7 +480,7 @@ class DenseUVW:
     def _fused_gx(self, which, w16, xb, gout16, status):
         import ctypes as C
 
-        from . import _lib, profiling
+        from . import profiling
 
         units = self._fused_units(which)
         B = xb.shape[0]
@@ -375,8 +498,6 @@ class DenseUVW:
     def _fused_wunits(self):
         if hasattr(self, "_wunits"):
             return self._wunits
-        from . import _lib
-
         d, off = self.d, self.offsets
         units = []
         for p in d.paths:
@@ -396,7 +517,7 @@ class DenseUVW:
     def _fused_gw(self, w, x1b, x2b, gout16, status):
         import ctypes as C
 
-        from . import _lib, profiling
+        from . import profiling
 
         units = self._fused_wunits()
         gw = torch.zeros((w.numel() // 64, 64), dtype=torch.float32, device=w.device)
@@ -413,7 +534,7 @@ class DenseUVW:
     def _fused_forward(self, w, x1, x2, status):
         import ctypes as C
 
-        from . import _lib, profiling
+        from . import profiling
 
         tasks = self._fused_tasks()
         B = x1.shape[0]
@@ -439,7 +560,6 @@ class DenseUVW:
     def _fctp_args(self, k, x1, x2, B):
         import ctypes as C
 
-        from . import _lib
         from .executor import dtype_code
 
         d, off, p = self.d, self.offsets, self.d.paths[k]
@@ -518,7 +638,7 @@ class DenseUVW:
         """Z[:, col0 : col0 + U*V] (rows (z, k), pitch ldz) = coupled operand of path k, float32."""
         import ctypes as C
 
-        from . import _lib, profiling
+        from . import profiling
 
         a = self._fctp_args(k, x1, x2, x1.shape[0])
         a.z = Z.data_ptr() + 4 * col0
@@ -535,6 +655,8 @@ class DenseUVW:
         GEMM per component k against the stacked weight blocks."""
         from .dense import gemm_f32x3, split_tf32
 
+        if self._tri_channels(torch.float32) and x1.shape[0]:
+            return self.tri_map(2, w, (x1, x2), "fctp_f32_forward")
         d, off = self.d, self.offsets
         B, dev = x1.shape[0], x1.device
         out = torch.zeros((B, self.out_size), dtype=torch.float32, device=dev)
@@ -604,9 +726,11 @@ class DenseUVW:
         """(dPhi/dx1, dPhi/dx2): per path gZ = g W^T by one GEMM per component, folded against the other operand."""
         import ctypes as C
 
-        from . import _lib, profiling
+        from . import profiling
         from .dense import gemm_f32x3, split_tf32
 
+        if self._tri_channels(torch.float32) and x1.shape[0]:
+            return self.tri_map(0, w, (x2, g), "fctp_f32_gx"), self.tri_map(1, w, (x1, g), "fctp_f32_gx")
         d, off = self.d, self.offsets
         B, dev = x1.shape[0], x1.device
         gx1 = torch.zeros(x1.shape, dtype=torch.float32, device=dev)

@@ -319,6 +319,39 @@ typedef struct {
 } cueq_gemm_f32x3_tn_args;
 int cueq_b200_gemm_f32x3_tn(const cueq_gemm_f32x3_tn_args* args, void* stream);
 
+/* Fully connected product (uvw,iu,jv,kw+ijk, shared weights): output or input gradient, one irrep of the result per call.
+ * R (the result), P and Q are the operands x1, x2, out / cotangent in the roles
+ *   R[z, c, r] (+)= sum over paths, p, q, a, b of coef[a][b][c] W[p, q, r] P[z, a, p] Q[z, b, q]
+ * All multiplicities are `channels` (32, 64, 96 in float32; 128 in bf16), irreps have dimension 1, 3 or 5.  P rows come
+ * as they are (ir_mul), Q transposed ([column][sample], cueq_b200_fctp_tri_transpose), the weights as rows ((q, r), p)
+ * (cueq_b200_fctp_tri_weights; row block k * channels^2 belongs to path k).  With splits > 1 the sum over q is divided among that
+ * many thread blocks and the result (zeroed by the caller) is added to. */
+#define CUEQ_FCTP_TRI_MAX_PATHS 24
+typedef struct {
+  int32_t a_src, a_off, na;   /* P: operand 0 or 1, its first column, its components                */
+  int32_t q_src, q_off, nb;   /* Q: likewise                                                       */
+  int32_t b_row0;             /* first weight row of the path                                      */
+  float coef[125];            /* [a][b][c], pitch 5                                                */
+} cueq_fctp_tri_path;
+typedef struct {
+  const void* a[2];     /* device rows [batch, lda], 16-byte aligned, of type `dtype`              */
+  const void* qt[2];    /* device float32 [columns, zp], 16-byte aligned; zp: a multiple of 128, >= batch */
+  const void* b_hi;     /* device [b_rows, channels]: TF32 halves (float32) or bf16                */
+  const void* b_lo;
+  void* out;            /* device float32 [batch, ldo]                                             */
+  const cueq_fctp_tri_path* paths;   /* host                                                       */
+  void* status;         /* nullable device int32: 2 if a bounded wait ran out                      */
+  int64_t lda[2], zp, b_rows, ldo, batch;
+  int32_t dtype, channels, out_off, nc, num_paths, splits;
+  int32_t struct_bytes; /* sizeof(cueq_fctp_tri_args) as the caller declares it                    */
+  int32_t reserved;
+} cueq_fctp_tri_args;
+int cueq_b200_fctp_tri(const cueq_fctp_tri_args* args, void* stream);
+/* order[k] = 100 * (axis of p) + 10 * (axis of q) + (axis of r), axes of W[u][v][w]: 0, 1, 2; w_off in elements */
+int cueq_b200_fctp_tri_weights(const void* w, int w_dtype, int dtype, int channels, int num_paths, const int32_t* w_off,
+                               const int32_t* order, void* hi, void* lo, void* stream);
+int cueq_b200_fctp_tri_transpose(const void* x, int dtype, int64_t batch, int32_t cols, int64_t ld, float* y, int64_t zp, void* stream);
+
 /* Equivariant linear layer, all irreps and weight classes in one launch, in the accuracy of the GEMMs above
  * (cuequivariance_torch/operations/linear.py:30-191; with classes primitives/segmented_polynomial_indexed_linear.py:116-156).
  * A path maps u copies of an irrep of dimension d (1, 3, 5 or 7) onto v copies; u and v are 32, 64, 96 or 128, no two
