@@ -218,7 +218,7 @@ class Uniform1dProgram:
                 torch.zeros((spec.rows, self.row_sizes[self.num_inputs + j]), dtype=self.math_dtype, device=device)
                 for j, spec in enumerate(cfg.outputs)
             ]
-            if cfg.batch > 0:
+            if cfg.batch > 0 and self.flat.operations:    # a derivative that vanishes has none
                 self._launch_generic(cfg, xs, outs, device)
             for j in range(self.num_outputs):
                 lay = cfg.layout(self.num_inputs + j)
@@ -413,6 +413,9 @@ class PolynomialFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, program: Uniform1dProgram, cfg: CallConfig, *inputs):
         ctx.program, ctx.cfg = program, cfg
+        # An output without a cotangent is left out of the derivative polynomial.  Materialised as zeros, the missing
+        # cotangents of the first-order gradients cost a double backward two more forward and two more backward passes.
+        ctx.set_materialize_grads(False)
         ctx.save_for_backward(*inputs)
         return tuple(program.run(cfg, [x.detach() for x in inputs]))
 
