@@ -188,6 +188,21 @@ class FctpTriArgs(C.Structure):
     ]
 
 
+class FctpGwPath(C.Structure):
+    _fields_ = [
+        ("x_row", C.c_int32), ("na", C.c_int32), ("y_row", C.c_int32), ("nb", C.c_int32), ("t_row", C.c_int32), ("ne", C.c_int32),
+        ("w_off", C.c_int32), ("order", C.c_int32), ("coef", C.c_float * 125),
+    ]
+
+
+class FctpGwArgs(C.Structure):
+    _fields_ = [
+        ("t", C.c_void_p), ("t_hi", C.c_void_p), ("t_lo", C.c_void_p), ("gw", C.c_void_p), ("paths", C.POINTER(FctpGwPath)),
+        ("status", C.c_void_p), ("rows", C.c_int64), ("zp", C.c_int64), ("batch", C.c_int64),
+        ("channels", C.c_int32), ("num_paths", C.c_int32), ("struct_bytes", C.c_int32), ("reserved", C.c_int32),
+    ]
+
+
 class LinearPath(C.Structure):
     _fields_ = [
         ("u", C.c_int32), ("v", C.c_int32), ("d", C.c_int32), ("x_off", C.c_int32), ("out_off", C.c_int32), ("w_off", C.c_int32),
@@ -285,7 +300,9 @@ def lib() -> C.CDLL:
     L.cueq_b200_fctp_tri.argtypes = [C.POINTER(FctpTriArgs), C.c_void_p]
     L.cueq_b200_fctp_tri_weights.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int, C.POINTER(C.c_int32), C.POINTER(C.c_int32),
                                              C.c_void_p, C.c_void_p, C.c_void_p]
-    L.cueq_b200_fctp_tri_transpose.argtypes = [C.c_void_p, C.c_int, C.c_int64, C.c_int32, C.c_int64, C.c_void_p, C.c_int64, C.c_void_p]
+    L.cueq_b200_fctp_tri_transpose.argtypes = [C.c_void_p, C.c_int, C.c_int64, C.c_int32, C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p,
+                                               C.c_int64, C.c_void_p]
+    L.cueq_b200_fctp_gw.argtypes = [C.POINTER(FctpGwArgs), C.c_void_p]
     L.cueq_b200_linear_map.argtypes = [C.POINTER(LinearArgs), C.c_void_p]
     L.cueq_b200_linear_gw.argtypes = [C.POINTER(LinearArgs), C.c_void_p]
     L.cueq_b200_selftest_bounded_wait.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p]

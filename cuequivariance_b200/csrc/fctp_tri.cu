@@ -17,8 +17,9 @@
 // float32: P and W are split into TF32 halves (P on chip, W by fctp_tri_weights), three passes, small terms first, so
 // that an accumulation chain has K / 8 <= 12 additions at full magnitude; all further sums are float32 FMAs.
 // bf16: one pass; Y stays in float32, where the route before rounded the products of the inputs to bf16.
-// What bounds it: float32 - the MMAs (27 * 64^3 * 3 multiply-adds per sample and launch set) and the L2 traffic of W
-// (2 MB per path component and 128 samples); bf16 - the CUDA cores' multiply-adds.
+// What bounds it, per launch set at 32,768 samples of 64x(0e+1o+2e), float32: 3.5 ms.  The MMAs alone need 1.2 ms (27 * 64^3 * 3
+// multiply-adds per sample); they wait for the weight blocks, 64 KB per 128 columns, of which two fit beside the operand
+// tile, and with five components of the result for the multiply-adds of the consumers.
 #include <cuda.h>
 
 #include <cstring>
@@ -382,9 +383,10 @@ __global__ void __launch_bounds__(256) fctp_tri_weights_kernel(const __grid_cons
   }
 }
 
-// rows [batch][ld] -> float32 [cols][zp], zeros for batch <= z < zp
+// rows [batch][ld] -> float32 [cols][zp], as they are and / or as TF32 halves; zeros for batch <= z < zp
 template <class T>
-__global__ void __launch_bounds__(256) fctp_tri_transpose_kernel(const T* __restrict__ x, float* __restrict__ y, int batch, int cols, int64_t ld, int64_t zp) {
+__global__ void __launch_bounds__(256) fctp_tri_transpose_kernel(const T* __restrict__ x, float* __restrict__ y, float* __restrict__ y_hi,
+                                                                 float* __restrict__ y_lo, int batch, int cols, int64_t ld, int64_t zp) {
   __shared__ float tile[32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, z0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
 #pragma unroll
@@ -395,7 +397,16 @@ __global__ void __launch_bounds__(256) fctp_tri_transpose_kernel(const T* __rest
   __syncthreads();
 #pragma unroll
   for (int k = 0; k < 32; k += 8)
-    if (c0 + ty + k < cols) y[(int64_t)(c0 + ty + k) * zp + z0 + tx] = tile[tx][ty + k];
+    if (c0 + ty + k < cols) {
+      const int64_t at = (int64_t)(c0 + ty + k) * zp + z0 + tx;
+      const float v = tile[tx][ty + k];
+      if (y) y[at] = v;
+      if (y_hi) {
+        const float h = tf32_hi(v);
+        y_hi[at] = h;
+        y_lo[at] = tf32_hi(v - h);
+      }
+    }
 }
 
 int make_map(CUtensorMap* map, bool bf16, const void* base, int64_t rows, int C, int box_rows) {
@@ -515,13 +526,14 @@ extern "C" int cueq_b200_fctp_tri_weights(const void* w, int w_dtype, int dtype,
   return 0;
 }
 
-extern "C" int cueq_b200_fctp_tri_transpose(const void* x, int dtype, int64_t batch, int32_t cols, int64_t ld, float* y, int64_t zp, void* stream) {
-  if (!x || !y) return cueq::fail("fctp tri: null operand");
+extern "C" int cueq_b200_fctp_tri_transpose(const void* x, int dtype, int64_t batch, int32_t cols, int64_t ld, float* y, float* y_hi, float* y_lo,
+                                            int64_t zp, void* stream) {
+  if (!x || (!y && !y_hi) || (!y_hi != !y_lo)) return cueq::fail("fctp tri: null operand");
   if (batch < 1 || cols < 1 || zp % 32 || zp < batch || zp > 2147483647LL - 32 || (cols + 31) / 32 > 65535) return cueq::fail("fctp tri: invalid shape");
   const dim3 grid((unsigned)(zp / 32), (unsigned)((cols + 31) / 32));
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (dtype == CUEQ_F32) fctp_tri_transpose_kernel<float><<<grid, 256, 0, st>>>((const float*)x, y, (int)batch, cols, ld, zp);
-  else if (dtype == CUEQ_BF16) fctp_tri_transpose_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>((const __nv_bfloat16*)x, y, (int)batch, cols, ld, zp);
+  if (dtype == CUEQ_F32) fctp_tri_transpose_kernel<float><<<grid, 256, 0, st>>>((const float*)x, y, y_hi, y_lo, (int)batch, cols, ld, zp);
+  else if (dtype == CUEQ_BF16) fctp_tri_transpose_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>((const __nv_bfloat16*)x, y, y_hi, y_lo, (int)batch, cols, ld, zp);
   else return cueq::fail("fctp tri: float32 or bf16 operands");
   CUEQ_CUDA_OK(cudaGetLastError());
   return 0;

@@ -392,7 +392,8 @@ class DenseUVW:
                     if s in transposed:
                         t = torch.empty((x.shape[1], zp), dtype=torch.float32, device=dev)
                         with profiling.kernel("fctp_tri_transpose"):
-                            _lib.check(L.cueq_b200_fctp_tri_transpose(xb.data_ptr(), dtype_code(dt), nb, x.shape[1], x.shape[1], t.data_ptr(), zp, stream))
+                            _lib.check(L.cueq_b200_fctp_tri_transpose(xb.data_ptr(), dtype_code(dt), nb, x.shape[1], x.shape[1], t.data_ptr(), None, None,
+                                                                      zp, stream))
                         a.qt[s] = t.data_ptr()
                         keep.append(t)
                 a.b_hi, a.b_lo, a.b_rows = hi.data_ptr(), None if lo is None else lo.data_ptr(), hi.shape[0]
@@ -405,6 +406,57 @@ class DenseUVW:
                     with profiling.kernel(name):
                         _lib.check(L.cueq_b200_fctp_tri(C.byref(a), stream))
         return out
+
+    def _tri_gw_paths(self):
+        if hasattr(self, "_gw_paths"):
+            return self._gw_paths
+        d, off = self.d, self.offsets
+        row0 = np.concatenate([[0], np.cumsum([op.size for op in d.operands[1:]])]).tolist()
+        arr = (_lib.FctpGwPath * len(d.paths))()
+        for t, p in zip(arr, d.paths):
+            sw, segs, dims = p.indices[0], p.indices[1:], p.coefficients.shape
+            e = min((2, 1, 0), key=lambda ax: dims[ax])              # fewest passes on the tensor cores; the output's axis for ties
+            x, y = (0, 1) if e == 2 else (1 - e, 2)                  # a contiguous axis in t or y
+            row = lambda ax: row0[ax] + off[1 + ax][segs[ax]]  # noqa: E731
+            t.x_row, t.na, t.y_row, t.nb, t.t_row, t.ne = row(x), dims[x], row(y), dims[y], row(e), dims[e]
+            t.w_off, t.order = off[0][sw], 100 * x + 10 * y + e
+            coef = p.coefficients.transpose(e, x, y)
+            for i, j, k in np.ndindex(*coef.shape):
+                t.coef[(i * 5 + j) * 5 + k] = float(coef[i, j, k])
+        self._gw_paths = (arr, row0)
+        return self._gw_paths
+
+    def tri_gw(self, operands, name: str) -> torch.Tensor:
+        """float32 weight gradient from the rows of (x1, x2, cotangent) (float32, ir_mul)."""
+        import ctypes as C
+
+        from . import profiling
+
+        L = _lib.lib()
+        paths, row0 = self._tri_gw_paths()
+        xs = [x.contiguous() for x in operands]
+        dev, B, rows = xs[0].device, xs[0].shape[0], row0[-1]
+        gw = torch.zeros((1, self.d.operands[0].size), dtype=torch.float32, device=dev)
+        step = min(B, max(128, 2**28 // rows // 128 * 128))          # 1 GB for each of the three transposed arrays
+        with torch.cuda.device(dev):
+            stream = C.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
+            for b0 in range(0, B, step):
+                nb = min(step, B - b0)
+                zp = -(-nb // 128) * 128
+                t = torch.empty((3, rows, zp), dtype=torch.float32, device=dev)
+                for x, r in zip(xs, row0):
+                    with profiling.kernel("fctp_tri_transpose"):
+                        _lib.check(L.cueq_b200_fctp_tri_transpose(x[b0 : b0 + nb].data_ptr(), _lib.F32, nb, x.shape[1], x.shape[1], t[0, r].data_ptr(),
+                                                                  t[1, r].data_ptr(), t[2, r].data_ptr(), zp, stream))
+                a = _lib.FctpGwArgs()
+                a.t, a.t_hi, a.t_lo, a.gw = t[0].data_ptr(), t[1].data_ptr(), t[2].data_ptr(), gw.data_ptr()
+                a.paths = C.cast(paths, C.POINTER(_lib.FctpGwPath))
+                a.status = _lib.status_word(dev).data_ptr()
+                a.rows, a.zp, a.batch = rows, zp, nb
+                a.channels, a.num_paths, a.struct_bytes = self._tri_channels(torch.float32), len(self.d.paths), C.sizeof(a)
+                with profiling.kernel(name):
+                    _lib.check(L.cueq_b200_fctp_gw(C.byref(a), stream))
+        return gw
 
     # -- fused route: coupled operand built in shared memory ------------------------------------
     def _fused_tasks(self):
@@ -696,6 +748,8 @@ class DenseUVW:
         """dPhi/dw: per path  gW[(u,v), w] = sum_(z,k) Z[(z,k),(u,v)] g[z, k, w]  (reduction over rows)."""
         from .dense import gemm_f32x3_tn
 
+        if self._tri_channels(torch.float32) and x1.shape[0]:
+            return self.tri_gw((x1, x2, g), "fctp_f32_gw")
         d, off = self.d, self.offsets
         B, dev = x1.shape[0], x1.device
         gw = torch.zeros((1, d.operands[0].size), dtype=torch.float32, device=dev)

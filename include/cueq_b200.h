@@ -350,7 +350,33 @@ int cueq_b200_fctp_tri(const cueq_fctp_tri_args* args, void* stream);
 /* order[k] = 100 * (axis of p) + 10 * (axis of q) + (axis of r), axes of W[u][v][w]: 0, 1, 2; w_off in elements */
 int cueq_b200_fctp_tri_weights(const void* w, int w_dtype, int dtype, int channels, int num_paths, const int32_t* w_off,
                                const int32_t* order, void* hi, void* lo, void* stream);
-int cueq_b200_fctp_tri_transpose(const void* x, int dtype, int64_t batch, int32_t cols, int64_t ld, float* y, int64_t zp, void* stream);
+/* y (nullable): the transposed rows; y_hi, y_lo (nullable together): their TF32 halves */
+int cueq_b200_fctp_tri_transpose(const void* x, int dtype, int64_t batch, int32_t cols, int64_t ld, float* y, float* y_hi, float* y_lo,
+                                 int64_t zp, void* stream);
+
+/* The weight gradient of the same product, float32: gw[x, y, t] += sum over samples, a, b, e of
+ *   coef[e][a][b] X[z, a, x] Y[z, b, y] T[z, e, t],   x, y, t = the axes u, v, w in the order given per path.
+ * All operands transposed and stacked: row = column of x1, x2 or the cotangent; sums run over K blocks of 32 samples, so the
+ * columns batch..zp of `t`, `t_hi`, `t_lo` hold zeros.  gw is zeroed by the caller. */
+typedef struct {
+  int32_t x_row, na, y_row, nb, t_row, ne;   /* first stacked row and components of X, Y, T        */
+  int32_t w_off;              /* first weight of the path                                          */
+  int32_t order;              /* 100 * (axis of x) + 10 * (axis of y) + (axis of t)                */
+  float coef[125];            /* [e][a][b], pitch 5                                                */
+} cueq_fctp_gw_path;
+typedef struct {
+  const void* t;        /* device float32 [rows, zp]                                               */
+  const void* t_hi;     /* their TF32 halves                                                       */
+  const void* t_lo;
+  void* gw;             /* device float32 weights, accumulated into                                */
+  const cueq_fctp_gw_path* paths;    /* host                                                       */
+  void* status;         /* nullable device int32: 2 if a bounded wait ran out                      */
+  int64_t rows, zp, batch;
+  int32_t channels, num_paths;
+  int32_t struct_bytes; /* sizeof(cueq_fctp_gw_args) as the caller declares it                     */
+  int32_t reserved;
+} cueq_fctp_gw_args;
+int cueq_b200_fctp_gw(const cueq_fctp_gw_args* args, void* stream);
 
 /* Equivariant linear layer, all irreps and weight classes in one launch, in the accuracy of the GEMMs above
  * (cuequivariance_torch/operations/linear.py:30-191; with classes primitives/segmented_polynomial_indexed_linear.py:116-156).
