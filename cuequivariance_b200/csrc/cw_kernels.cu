@@ -132,6 +132,23 @@ extern "C" int cueq_b200_cw_backward(int g, const cueq_cw_args* a, void* stream)
   return kGroups[g]->bwd(p, coef, a->x1_mul_ir, pick_cpl(a), masked, reinterpret_cast<cudaStream_t>(stream));
 }
 
+// All groups of a polynomial by one call: the constant part of each group's arguments comes from `templates`, which the
+// caller keeps, tensors and sizes from `call`.  The groups are queued one after the other, as by separate calls.
+extern "C" int cueq_b200_cw_run(int backward, int num_groups, const int32_t* groups, const cueq_cw_args* templates, const cueq_cw_args* call,
+                                void* stream) {
+  if (num_groups < 0 || (num_groups && (!groups || !templates || !call))) return cueq::fail("channelwise: null argument");
+  for (int i = 0; i < num_groups; ++i) {
+    cueq_cw_args a = templates[i];
+    a.w = call->w; a.x1 = call->x1; a.x2 = call->x2; a.out = call->out;
+    a.gout = call->gout; a.gw = call->gw; a.gx1 = call->gx1; a.gx2 = call->gx2;
+    a.senders = call->senders; a.order = call->order; a.rowptr = call->rowptr;
+    a.num_receivers = call->num_receivers; a.recv_mod = call->recv_mod;
+    a.x1_mul_ir = call->x1_mul_ir; a.out_mul_ir = call->out_mul_ir;
+    if (int rc = backward ? cueq_b200_cw_backward(groups[i], &a, stream) : cueq_b200_cw_forward(groups[i], &a, stream)) return rc;
+  }
+  return 0;
+}
+
 // ---- forward without caller-provided scratch ----------------------------------------------------
 //
 // cueq_b200_cw_forward needs two pieces of device memory besides its inputs and outputs: the

@@ -266,6 +266,7 @@ class StaticKernel:
 
     def __init__(self, kernel_id: int, name: str):
         self.kernel_id, self.name = kernel_id, name
+        self._kept: dict = {}     # per (layouts, output modes): what a call does with its buffers
 
     @staticmethod
     def _in_place(program: "Uniform1dProgram", cfg: CallConfig, b: int) -> bool:
@@ -284,33 +285,37 @@ class StaticKernel:
         if program.math_dtype != torch.float32 or any(x.dtype != torch.float32 for x in xs):
             return None
         device = xs[0].device
-        nb = program.num_inputs + program.num_outputs
-        in_place = [cfg.layout(b) is not None and self._in_place(program, cfg, b) for b in range(nb)]
-        xs = [x if cfg.layout(i) is None or in_place[i] else transpose_blocks(x, cfg.layout(i), to_ir_mul=True) for i, x in enumerate(xs)]
-        outs = [
-            torch.zeros((spec.rows, program.row_sizes[program.num_inputs + j]), dtype=torch.float32, device=device)
-            if spec.mode != _lib.BATCHED or program.buffer_dim[program.num_inputs + j] == 0
-            else torch.empty((spec.rows, program.row_sizes[program.num_inputs + j]), dtype=torch.float32, device=device)
-            for j, spec in enumerate(cfg.outputs)
-        ]
+        n_in = program.num_inputs
+        specs = cfg.inputs + cfg.outputs
+        # what a call does with its buffers depends on their layouts and modes only
+        key = (cfg.layouts, tuple(s.mode for s in cfg.outputs))
+        kept = self._kept.get(key)
+        if kept is None:
+            in_place = [cfg.layout(b) is not None and self._in_place(program, cfg, b) for b in range(len(specs))]
+            zeroed = [s.mode != _lib.BATCHED or program.buffer_dim[n_in + j] == 0 for j, s in enumerate(cfg.outputs)]
+            kept = (in_place, [cfg.layout(b) is not None and not f for b, f in enumerate(in_place)], zeroed,
+                    _lib.int32_array(program.buffer_dim), _lib.int32_array(program.buffer_num_segments))
+            self._kept[key] = kept
+        in_place, transposed, zeroed, dims, segments = kept
+        xs = [transpose_blocks(x, cfg.layout(i), to_ir_mul=True) if transposed[i] else x for i, x in enumerate(xs)]
+        outs = [(torch.zeros if z else torch.empty)((spec.rows, program.row_sizes[n_in + j]), dtype=torch.float32, device=device)
+                for j, (spec, z) in enumerate(zip(cfg.outputs, zeroed))]
+        nb = len(specs)
         bufs = (_lib.Buffer * nb)()
         keep = []
-        for b, (t, spec) in enumerate(zip(list(xs) + outs, cfg.inputs + cfg.outputs)):
-            bufs[b].ptr = t.data_ptr() if t.numel() else None
-            bufs[b].rows, bufs[b].mode, bufs[b].dtype, bufs[b].layout = spec.rows, spec.mode, _lib.F32, int(in_place[b])
+        for buf, t, spec, placed in zip(bufs, xs + outs, specs, in_place):
+            buf.ptr, buf.rows, buf.mode, buf.dtype, buf.layout = t.data_ptr(), spec.rows, spec.mode, _lib.F32, placed
             if spec.mode == _lib.INDEXED:
                 idx = spec.index.contiguous()
                 keep.append(idx)
-                bufs[b].index = idx.data_ptr() if idx.numel() else None
-                bufs[b].index_is_64 = 1 if idx.dtype == torch.int64 else 0
-        stream = C.c_void_p(torch.cuda.current_stream(device).cuda_stream)
-        with torch.cuda.device(device), profiling.kernel(f"u1d_static[{self.name}]"):
-            _lib.check(_lib.lib().cueq_b200_u1d_static_launch(
-                self.kernel_id, cfg.batch, program.extent, bufs, _lib.int32_array(program.buffer_dim),
-                _lib.int32_array(program.buffer_num_segments), nb, stream))
+                buf.index = idx.data_ptr()
+                buf.index_is_64 = idx.dtype == torch.int64
+        with _lib.on_device(device), profiling.kernel(f"u1d_static[{self.name}]"):
+            _lib.check(_lib.lib().cueq_b200_u1d_static_launch(self.kernel_id, cfg.batch, program.extent, bufs, dims, segments, nb,
+                                                              torch.cuda.current_stream(device).cuda_stream))
         for j in range(program.num_outputs):
             b = program.num_inputs + j
-            if cfg.layout(b) is not None and not in_place[b]:
+            if transposed[b]:
                 outs[j] = transpose_blocks(outs[j], cfg.layout(b), to_ir_mul=False)
         return outs
 

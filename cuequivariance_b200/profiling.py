@@ -19,6 +19,10 @@ def enable(flag: bool = True) -> None:
     _enabled = flag
 
 
+def enabled() -> bool:
+    return _enabled
+
+
 def reset() -> None:
     global launch_count
     _records.clear()

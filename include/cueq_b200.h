@@ -238,6 +238,10 @@ const char* cueq_b200_cw_group_signature(int group);
 int cueq_b200_cw_group_info(int group, int32_t* d1, int32_t* num_paths, int32_t* num_pairs, int32_t* num_terms);
 int cueq_b200_cw_forward(int group, const cueq_cw_args* args, void* stream);
 int cueq_b200_cw_backward(int group, const cueq_cw_args* args, void* stream);
+/* num_groups forward (backward = 0) or backward launches: group i runs with templates[i], except for the tensors (w, x1, x2,
+ * out, gout, gw, gx1, gx2), senders, order, rowptr, num_receivers, recv_mod and the two layouts, which come from `call`. */
+int cueq_b200_cw_run(int backward, int num_groups, const int32_t* groups, const cueq_cw_args* templates, const cueq_cw_args* call,
+                     void* stream);
 
 /* ---- kernels written out at build time for known polynomials ---------------------------------
  *
