@@ -13,6 +13,7 @@ LIB_PATH = Path(__file__).resolve().parent / "libcueq_b200.so"
 F32, F64, BF16, F16 = 0, 1, 2, 3
 SHARED, BATCHED, INDEXED = 0, 1, 2
 MAX_BUFFERS, MAX_OPERANDS = 16, 8
+CSR_SMALL_EDGES, CSR_SMALL_ROWS = 4096, 65536
 
 
 class U1dDesc(C.Structure):
@@ -280,6 +281,8 @@ def lib() -> C.CDLL:
     L.cueq_b200_sh_backward.argtypes = [C.POINTER(ShArgs), C.c_void_p]
     L.cueq_b200_cw_forward.argtypes = [C.c_int, C.POINTER(CwArgs), C.c_void_p]
     L.cueq_b200_cw_backward.argtypes = [C.c_int, C.POINTER(CwArgs), C.c_void_p]
+    L.cueq_b200_csr_rowptr.argtypes = [C.c_void_p, C.c_int, C.c_int64, C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p]
+    L.cueq_b200_csr_small.argtypes = [C.c_void_p, C.c_int, C.c_int64, C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p]
     L.cueq_b200_cw_run.argtypes = [C.c_int, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]
     L.cueq_b200_cw_forward_noalloc.argtypes = [C.c_int, C.POINTER(CwNoAllocArgs), C.c_void_p]
     L.cueq_b200_u1d_static_find.argtypes = [C.c_char_p]

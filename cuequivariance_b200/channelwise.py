@@ -74,19 +74,47 @@ class _CsrCache:
         for k, ref, val in self.entries:
             if k == key and ref is index:
                 return val
-        idx = index if index.dtype == torch.int32 else index.to(torch.int32)
-        if idx.numel() > 1 and not bool((idx[1:] >= idx[:-1]).all()):
-            sorted_idx, order = torch.sort(idx, stable=True)
-            order = order.to(torch.int32)
+        if index.is_cuda and index.dtype in (torch.int32, torch.int64):
+            order, rowptr = self._rows_cuda(index.contiguous(), num_rows)
         else:
-            sorted_idx, order = idx, None
-        bounds = torch.arange(num_rows + 1, device=index.device, dtype=torch.int32)
-        rowptr = torch.searchsorted(sorted_idx.contiguous(), bounds, right=False).to(torch.int32)
+            idx = index if index.dtype == torch.int32 else index.to(torch.int32)
+            if idx.numel() > 1 and not bool((idx[1:] >= idx[:-1]).all()):
+                sorted_idx, order = torch.sort(idx, stable=True)
+                order = order.to(torch.int32)
+            else:
+                sorted_idx, order = idx, None
+            bounds = torch.arange(num_rows + 1, device=index.device, dtype=torch.int32)
+            rowptr = torch.searchsorted(sorted_idx.contiguous(), bounds, right=False).to(torch.int32)
         val = (order, rowptr)
         self.entries.append((key, index, val))
         if len(self.entries) > self.capacity:
             self.entries.pop(0)
         return val
+
+    @staticmethod
+    def _rows_cuda(index, num_rows: int):
+        """(order or None, rowptr).  A short list: one kernel, nothing read back (its order is given even if it ascends).
+        A longer one: one kernel and one read of its flag where the index ascends, as edge lists of neighbour searches do,
+        a stable sort in between where it does not."""
+        import torch
+
+        from . import _lib
+
+        L, n, is64 = _lib.lib(), index.numel(), int(index.dtype == torch.int64)
+        rowptr = torch.empty(num_rows + 1, dtype=torch.int32, device=index.device)
+        with _lib.on_device(index.device):
+            stream = torch.cuda.current_stream(index.device).cuda_stream
+            if n <= _lib.CSR_SMALL_EDGES and num_rows <= _lib.CSR_SMALL_ROWS:
+                order = torch.empty(n, dtype=torch.int32, device=index.device)
+                _lib.check(L.cueq_b200_csr_small(index.data_ptr(), is64, n, num_rows, order.data_ptr(), rowptr.data_ptr(), stream))
+                return order, rowptr
+            flag = torch.zeros(1, dtype=torch.int32, device=index.device)
+            _lib.check(L.cueq_b200_csr_rowptr(index.data_ptr(), is64, n, num_rows, rowptr.data_ptr(), flag.data_ptr(), stream))
+            if not flag.item():
+                return None, rowptr
+            index, order = torch.sort(index if not is64 else index.to(torch.int32), stable=True)
+            _lib.check(L.cueq_b200_csr_rowptr(index.data_ptr(), 0, n, num_rows, rowptr.data_ptr(), flag.data_ptr(), stream))
+        return order.to(torch.int32), rowptr
 
     def get_passes(self, receivers, senders, num_rows: int, num_senders: int, passes: int):
         """CSR over (pass, receiver) rows, pass = which of ``passes`` equal ranges the sender

@@ -233,6 +233,12 @@ typedef struct {
   int32_t reserved;
 } cueq_cw_args;
 
+/* Row pointers [rows + 1] of an ascending receiver index [n]: rowptr[r] = first position with index >= r.  *descends (zeroed
+ * by the caller) becomes 1 if the index does not ascend; the row pointers are then of no use. */
+int cueq_b200_csr_rowptr(const void* index, int index_is_64, int64_t n, int64_t rows, int32_t* rowptr, int32_t* descends, void* stream);
+/* The same for any index of at most 4,096 entries and 65,536 rows, with the stable order [n] of its positions by receiver. */
+int cueq_b200_csr_small(const void* index, int index_is_64, int64_t n, int64_t rows, int32_t* order, int32_t* rowptr, void* stream);
+
 int cueq_b200_cw_num_groups(void);
 const char* cueq_b200_cw_group_signature(int group);
 int cueq_b200_cw_group_info(int group, int32_t* d1, int32_t* num_paths, int32_t* num_pairs, int32_t* num_terms);
