@@ -58,7 +58,7 @@ class CwArgs(C.Structure):
         ("w_offset", C.c_int32 * 8), ("out_offset", C.c_int32 * 8),
         ("x1_mul_ir", C.c_int32), ("out_mul_ir", C.c_int32), ("channels_per_lane", C.c_int32), ("staging", C.c_int32),
         ("status", C.c_void_p), ("recv_mod", C.c_int32), ("variant", C.c_int32),
-        ("path_mask", C.c_int32), ("x2_width", C.c_int32), ("dtype", C.c_int32), ("reserved", C.c_int32),
+        ("path_mask", C.c_int32), ("x2_width", C.c_int32), ("dtype", C.c_int32), ("mean_degree", C.c_int32),
     ]
 
 

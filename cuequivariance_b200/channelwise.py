@@ -422,6 +422,7 @@ class _ChannelwiseBase:
         ts, tj, tc = tabs[which]
         a.tab_start, a.tab_j, a.tab_c = ts.data_ptr(), tj.data_ptr(), tc.data_ptr()
         a.num_receivers = nrecv
+        a.mean_degree = tensors["w"].shape[0] // max(nrecv, 1)
         if x1_is_block:
             # may be a column slice of a wider tensor (several irrep blocks gathered together); a
             # gradient block, if any, must then be the matching slice of an equally wide tensor
@@ -476,6 +477,7 @@ class _ChannelwiseBase:
         if order is not None:
             a.order = order.data_ptr()
         a.rowptr, a.num_receivers, a.recv_mod = rowptr.data_ptr(), nrecv, recv_mod
+        a.mean_degree = w.shape[0] // max(nrecv, 1)
         a.x1_mul_ir, a.out_mul_ir = int(common["x1_mul_ir"]), int(mul_ir)
         with _lib.on_device(dev):
             _lib.check(_lib.lib().cueq_b200_cw_run(int(which == "bwd_tab"), n, groups, arr, C.byref(a), torch.cuda.current_stream(dev).cuda_stream))

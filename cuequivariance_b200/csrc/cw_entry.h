@@ -54,7 +54,7 @@ struct GroupEntry {
   int (*fwd)(const CwParams&, int mul_ir, int cpl, bool masked, cudaStream_t);
   int (*bwd)(const CwParams&, const CwCoef&, int mul_ir, int cpl, bool masked, cudaStream_t);
   int (*fwd_bulk)(const CwParams&, int mul_ir, int cpl, cudaStream_t);
-  int (*bwd_block)(const CwParams&, const CwCoef&, int mul_ir, int bulk, bool masked, cudaStream_t);
+  int (*bwd_block)(const CwParams&, const CwCoef&, int mul_ir, int cpl, int bulk, bool masked, cudaStream_t);
 };
 struct GroupEntry64 {
   int (*fwd)(const CwParamsT<double>&, int mul_ir, cudaStream_t);

@@ -119,16 +119,19 @@ extern "C" int cueq_b200_cw_backward(int g, const cueq_cw_args* a, void* stream)
   std::memset(&coef, 0, sizeof(coef));
   for (int t = 0; t < kGroups[g]->nterm; ++t) coef.c[t] = static_cast<const float*>(a->bwd_coef)[t];
   if (a->variant < 0 || a->variant > 3) return cueq::fail("channelwise backward: variant must be 0 (automatic), 1, 2 or 3");
-  // one thread block per receiver needs the four-channel layout (extent a multiple of 4 is given);
-  // it is the default from 128 channels on, where a warp's 128 channels are all in use
+  // One thread block per receiver, four channels per thread where a warp's 128 channels are all in use, else two.  With two
+  // and few edges per receiver the cotangent row is staged by a block for too little work; 100,000 edges, lmax 3, one warp
+  // against one block per receiver: 64 channels, 20 edges 680 / 536 us, 5 edges 720 / 757 us; 32 channels, 5 edges
+  // 1371 / 687 us; 2,000 edges on 100 receivers, 64 channels: 153 / 51 us.
+  const bool few = a->mean_degree > 0 && a->mean_degree < 8 && a->extent > 32 && a->extent % 128;
   const bool masked = is_masked(p, *kGroups[g]);
-  const bool block_per_receiver = a->variant >= 2 || (a->variant == 0 && a->channels_per_lane != 2 && a->extent % 128 == 0);
+  const bool block_per_receiver = a->variant >= 2 || (a->variant == 0 && a->channels_per_lane != 2 && !few);
   if (a->variant == 3 && a->extent % 128) return cueq::fail("channelwise backward: variant 3 needs a multiple of 128 channels");
   // bulk reductions pay from three components per channel on (one 1.5 KB operation instead of three vector
   // reductions per lane); for the scalar block (512 bytes per edge) the vector reductions are faster
   const bool bulk = a->variant == 3 || (a->variant == 0 && kGroups[g]->d1 >= 3);
   if (block_per_receiver)
-    return kGroups[g]->bwd_block(p, coef, a->x1_mul_ir, bulk, masked, reinterpret_cast<cudaStream_t>(stream));
+    return kGroups[g]->bwd_block(p, coef, a->x1_mul_ir, a->variant >= 2 || a->extent % 128 == 0 ? 4 : 2, bulk, masked, reinterpret_cast<cudaStream_t>(stream));
   return kGroups[g]->bwd(p, coef, a->x1_mul_ir, pick_cpl(a), masked, reinterpret_cast<cudaStream_t>(stream));
 }
 
@@ -142,7 +145,7 @@ extern "C" int cueq_b200_cw_run(int backward, int num_groups, const int32_t* gro
     a.w = call->w; a.x1 = call->x1; a.x2 = call->x2; a.out = call->out;
     a.gout = call->gout; a.gw = call->gw; a.gx1 = call->gx1; a.gx2 = call->gx2;
     a.senders = call->senders; a.order = call->order; a.rowptr = call->rowptr;
-    a.num_receivers = call->num_receivers; a.recv_mod = call->recv_mod;
+    a.num_receivers = call->num_receivers; a.recv_mod = call->recv_mod; a.mean_degree = call->mean_degree;
     a.x1_mul_ir = call->x1_mul_ir; a.out_mul_ir = call->out_mul_ir;
     if (int rc = backward ? cueq_b200_cw_backward(groups[i], &a, stream) : cueq_b200_cw_forward(groups[i], &a, stream)) return rc;
   }

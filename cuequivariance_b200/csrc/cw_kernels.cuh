@@ -61,10 +61,13 @@ __device__ __forceinline__ void to_array(const float4& v, float (&a)[4]) { a[0] 
 __device__ __forceinline__ void to_array(const float2& v, float (&a)[2]) { a[0] = v.x; a[1] = v.y; }
 __device__ __forceinline__ void to_array(const double2& v, double (&a)[2]) { a[0] = v.x; a[1] = v.y; }
 
-template <int N>
-__device__ __forceinline__ float4 make_vec(const float (&f)[N], int t) { return make_float4(f[t], f[t + 1], f[t + 2], f[t + 3]); }
-template <int N>
-__device__ __forceinline__ double2 make_vec(const double (&f)[N], int t) { return make_double2(f[t], f[t + 1]); }
+template <int C, int N, class T>
+__device__ __forceinline__ Vec<C, T> make_vec(const T (&f)[N], int t) {
+  Vec<C, T> v;
+  v.x = f[t]; v.y = f[t + 1];
+  if constexpr (C == 4) { v.z = f[t + 2]; v.w = f[t + 3]; }
+  return v;
+}
 
 template <int BYTES>
 __device__ __forceinline__ void cp_async(void* smem_dst, const void* gmem_src) {
@@ -643,9 +646,8 @@ struct StageGSplit {
   }
 };
 
-template <class T, class G, bool MUL_IR, bool BULK_RED, bool NEED_GX2, bool MASKED>
-__global__ void __launch_bounds__(kWarps * 32, sizeof(T) == 8 ? 2 : 3) cw_bwd_block_kernel(const __grid_constant__ CwParamsT<T> p, const __grid_constant__ CwCoefT<T> coef) {
-  constexpr int C = 16 / (int)sizeof(T);
+template <class T, class G, int C, bool MUL_IR, bool BULK_RED, bool NEED_GX2, bool MASKED>
+__global__ void __launch_bounds__(kWarps * 32, sizeof(T) == 8 ? 2 : C == 2 ? 4 : 3) cw_bwd_block_kernel(const __grid_constant__ CwParamsT<T> p, const __grid_constant__ CwCoefT<T> coef) {
   // BULK_RED (mul_ir rows only): the x1 gradient of an edge - the 32 lanes' C*D1 values are one contiguous run of
   // the sender's row - leaves as ONE bulk reduction per warp and edge instead of D1 vector reductions per lane.
   // Its shared-memory source is the slot the edge's x1 block was staged in (free once X is in registers); the
@@ -744,7 +746,7 @@ __global__ void __launch_bounds__(kWarps * 32, sizeof(T) == 8 ? 2 : 3) cw_bwd_bl
           __syncwarp();                                              // every lane has taken its X out of the slot
           Vec<C, T>* slot = reinterpret_cast<Vec<C, T>*>(st + S::kX2);
 #pragma unroll
-          for (int t = 0; t < G::D1; ++t) slot[lane * G::D1 + t] = make_vec(f, C * t);
+          for (int t = 0; t < G::D1; ++t) slot[lane * G::D1 + t] = make_vec<C>(f, C * t);
           fence_proxy_async();
           __syncwarp();
           if (lane == 0)
@@ -840,41 +842,41 @@ int launch_bwd(const CwParams& p, const CwCoef& coef, int mul_ir, int cpl, bool 
   return masked ? launch_bwd_m<G, true>(p, coef, mul_ir, cpl, st) : launch_bwd_m<G, false>(p, coef, mul_ir, cpl, st);
 }
 
-template <class T, class G, bool A, bool BULK, bool GX2, bool MASKED>
+template <class T, class G, int C, bool A, bool BULK, bool GX2, bool MASKED>
 int launch_bwd_block_t(const CwParamsT<T>& p, const CwCoefT<T>& coef, cudaStream_t st) {
-  constexpr int C = 16 / (int)sizeof(T);
   using S = Smem<G, C, T>;
   const size_t smem = sizeof(T) * (S::kGrow + kWarps * S::kPerWarpFwd);
   static cueq::PerDeviceFlag configured;
   if (!configured.get()) {
-    CUEQ_CUDA_OK(cudaFuncSetAttribute(cw_bwd_block_kernel<T, G, A, BULK, GX2, MASKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CUEQ_CUDA_OK(cudaFuncSetAttribute(cw_bwd_block_kernel<T, G, C, A, BULK, GX2, MASKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     configured.set();
   }
   // blocks walk the receivers with a grid stride; many short-lived blocks (a few receivers each) let the hardware
   // balance the uneven edge counts better than eight waves of long ones (l = 3 launch 3.48 -> 3.40 ms)
   const int cap = 148 * 96;
   dim3 grid(p.num_receivers < cap ? p.num_receivers : cap, (p.extent + 32 * C - 1) / (32 * C));
-  cw_bwd_block_kernel<T, G, A, BULK, GX2, MASKED><<<grid, kWarps * 32, smem, st>>>(p, coef);
+  cw_bwd_block_kernel<T, G, C, A, BULK, GX2, MASKED><<<grid, kWarps * 32, smem, st>>>(p, coef);
   CUEQ_CUDA_OK(cudaGetLastError());
   return 0;
 }
 
 // bulk: the x1 gradient leaves as one bulk reduction per warp and edge; needs mul_ir rows whose blocks start on
 // 16-byte boundaries (checked here: a misaligned bulk operation is an illegal instruction, not an error code)
-template <class T, class G, bool MASKED>
+template <class T, class G, int C, bool MASKED>
 int launch_bwd_block_m(const CwParamsT<T>& p, const CwCoefT<T>& coef, int mul_ir, int bulk, cudaStream_t st) {
-  constexpr int C = 16 / (int)sizeof(T);
-  const bool aligned = (reinterpret_cast<uintptr_t>(p.gx1) % 16 == 0) && (p.x1_stride % C == 0) && (p.x1_off % C == 0) && (p.extent % (32 * C) == 0);
+  constexpr int V = 16 / (int)sizeof(T);
+  const bool aligned = (reinterpret_cast<uintptr_t>(p.gx1) % 16 == 0) && (p.x1_stride % V == 0) && (p.x1_off % V == 0) && (p.extent % (32 * C) == 0);
   // the x2-gradient partials are a third of the arithmetic: a launch that does not need them runs without
   if (bulk && mul_ir && p.need_gx1 && aligned)
-    return p.need_gx2 ? launch_bwd_block_t<T, G, true, true, true, MASKED>(p, coef, st) : launch_bwd_block_t<T, G, true, true, false, MASKED>(p, coef, st);
-  if (mul_ir) return p.need_gx2 ? launch_bwd_block_t<T, G, true, false, true, MASKED>(p, coef, st) : launch_bwd_block_t<T, G, true, false, false, MASKED>(p, coef, st);
-  return p.need_gx2 ? launch_bwd_block_t<T, G, false, false, true, MASKED>(p, coef, st) : launch_bwd_block_t<T, G, false, false, false, MASKED>(p, coef, st);
+    return p.need_gx2 ? launch_bwd_block_t<T, G, C, true, true, true, MASKED>(p, coef, st) : launch_bwd_block_t<T, G, C, true, true, false, MASKED>(p, coef, st);
+  if (mul_ir) return p.need_gx2 ? launch_bwd_block_t<T, G, C, true, false, true, MASKED>(p, coef, st) : launch_bwd_block_t<T, G, C, true, false, false, MASKED>(p, coef, st);
+  return p.need_gx2 ? launch_bwd_block_t<T, G, C, false, false, true, MASKED>(p, coef, st) : launch_bwd_block_t<T, G, C, false, false, false, MASKED>(p, coef, st);
 }
 
 template <class G>
-int launch_bwd_block(const CwParams& p, const CwCoef& coef, int mul_ir, int bulk, bool masked, cudaStream_t st) {
-  return masked ? launch_bwd_block_m<float, G, true>(p, coef, mul_ir, bulk, st) : launch_bwd_block_m<float, G, false>(p, coef, mul_ir, bulk, st);
+int launch_bwd_block(const CwParams& p, const CwCoef& coef, int mul_ir, int cpl, int bulk, bool masked, cudaStream_t st) {
+  if (cpl == 2) return masked ? launch_bwd_block_m<float, G, 2, true>(p, coef, mul_ir, bulk, st) : launch_bwd_block_m<float, G, 2, false>(p, coef, mul_ir, bulk, st);
+  return masked ? launch_bwd_block_m<float, G, 4, true>(p, coef, mul_ir, bulk, st) : launch_bwd_block_m<float, G, 4, false>(p, coef, mul_ir, bulk, st);
 }
 
 // float64: two channels per thread, one form of each kernel (it walks the path mask whether or not all paths are there)
@@ -884,7 +886,7 @@ int launch_fwd_f64(const CwParamsT<double>& p, int mul_ir, cudaStream_t st) {
 }
 template <class G>
 int launch_bwd_f64(const CwParamsT<double>& p, const CwCoefT<double>& coef, int mul_ir, cudaStream_t st) {
-  return launch_bwd_block_m<double, G, true>(p, coef, mul_ir, 1, st);
+  return launch_bwd_block_m<double, G, 2, true>(p, coef, mul_ir, 1, st);
 }
 
 }  // namespace

@@ -219,8 +219,9 @@ typedef struct {
   void* status;         /* nullable device int32: set to 1 if a bounded wait on a bulk copy ran out */
   int32_t recv_mod;     /* backward only: if > 0 the CSR has several rows per receiver (row r belongs to
                            receiver r % recv_mod), used to visit the edges in sender-range passes        */
-  int32_t variant;      /* backward only: 0 = the library chooses (3 from 128 channels on for x1 degrees >= 1,
-                           2 for the scalar block, 1 otherwise); 1 = one warp per receiver (2 or 4 channels
+  int32_t variant;      /* backward only: 0 = the library chooses (multiples of 128 channels: 3 for x1 degrees >= 1, 2 for
+                           the scalar block; other channel counts: the same with two channels per thread, or 1
+                           where receivers have few edges, see mean_degree); 1 = one warp per receiver (2 or 4 channels
                            per thread); 2 = one thread block per receiver: its warps share the staged
                            cotangent row and split the receiver's edges, four channels per thread;
                            3 = as 2, with the x1 gradient of an edge leaving as one bulk reduction
@@ -230,7 +231,7 @@ typedef struct {
                            keep the full group's numbering, entries of absent paths have no terms           */
   int32_t x2_width;     /* components of an x2 row: 1, 4, 9 or 16 (0: 16)                               */
   int32_t dtype;        /* CUEQ_F32, or CUEQ_F64: two channels per thread, staging / variant ignored    */
-  int32_t reserved;
+  int32_t mean_degree;    /* backward: edges per receiver, rounded down (0: unknown); picks the division of the work */
 } cueq_cw_args;
 
 /* Row pointers [rows + 1] of an ascending receiver index [n]: rowptr[r] = first position with index >= r.  *descends (zeroed
@@ -245,7 +246,8 @@ int cueq_b200_cw_group_info(int group, int32_t* d1, int32_t* num_paths, int32_t*
 int cueq_b200_cw_forward(int group, const cueq_cw_args* args, void* stream);
 int cueq_b200_cw_backward(int group, const cueq_cw_args* args, void* stream);
 /* num_groups forward (backward = 0) or backward launches: group i runs with templates[i], except for the tensors (w, x1, x2,
- * out, gout, gw, gx1, gx2), senders, order, rowptr, num_receivers, recv_mod and the two layouts, which come from `call`. */
+ * out, gout, gw, gx1, gx2), senders, order, rowptr, num_receivers, recv_mod, mean_degree and the two layouts, which come from
+ * `call`. */
 int cueq_b200_cw_run(int backward, int num_groups, const int32_t* groups, const cueq_cw_args* templates, const cueq_cw_args* call,
                      void* stream);
 
