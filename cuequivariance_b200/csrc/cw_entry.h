@@ -44,6 +44,7 @@ struct CwParamsT {
   int recv_mod;             // backward: CSR rows are (pass, receiver) pairs; the cotangent row is row % recv_mod (0: off)
   unsigned path_mask;       // bit q: path q of the group belongs to the polynomial (MASKED kernels)
   int nx2;                  // components of an x2 row (MASKED kernels; 16 otherwise)
+  int overlap;              // launch: may start while the kernel before it in the stream, a group of the same call, still runs
 };
 using CwParams = CwParamsT<float>;
 

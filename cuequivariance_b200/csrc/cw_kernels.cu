@@ -76,17 +76,21 @@ extern "C" int cueq_b200_cw_group_info(int g, int32_t* d1, int32_t* npath, int32
   return 0;
 }
 
-extern "C" int cueq_b200_cw_forward(int g, const cueq_cw_args* a, void* stream) {
+namespace {
+
+int run_forward(int g, const cueq_cw_args* a, int overlap, void* stream) {
   if (g < 0 || g >= kNumGroups) return cueq::fail("channelwise: group %d out of range", g);
   if (a && a->dtype == CUEQ_F64) {
     CwParamsT<double> p;
     if (int rc = fill_params(a, *kGroups[g], p, kGroups[g]->nterm_fwd)) return rc;
+    p.overlap = overlap;
     if (!p.w || !p.x1 || !p.x2 || !p.out) return cueq::fail("channelwise forward: null tensor");
     return p.num_receivers == 0 ? 0 : kGroups64[g]->fwd(p, a->x1_mul_ir, reinterpret_cast<cudaStream_t>(stream));
   }
   if (a && a->dtype != CUEQ_F32) return cueq::fail("channelwise: float32 or float64 operands");
   CwParams p;
   if (int rc = fill_params(a, *kGroups[g], p, kGroups[g]->nterm_fwd)) return rc;
+  p.overlap = overlap;
   if (!p.w || !p.x1 || !p.x2 || !p.out) return cueq::fail("channelwise forward: null tensor");
   if (p.num_receivers == 0) return 0;
   p.status = reinterpret_cast<int*>(a->status);
@@ -96,11 +100,12 @@ extern "C" int cueq_b200_cw_forward(int g, const cueq_cw_args* a, void* stream) 
   return kGroups[g]->fwd(p, a->x1_mul_ir, pick_cpl(a), masked, reinterpret_cast<cudaStream_t>(stream));
 }
 
-extern "C" int cueq_b200_cw_backward(int g, const cueq_cw_args* a, void* stream) {
+int run_backward(int g, const cueq_cw_args* a, int overlap, void* stream) {
   if (g < 0 || g >= kNumGroups) return cueq::fail("channelwise: group %d out of range", g);
   if (a && a->dtype == CUEQ_F64) {
     CwParamsT<double> p;
     if (int rc = fill_params(a, *kGroups[g], p, kGroups[g]->nterm)) return rc;
+    p.overlap = overlap;
     if (!p.w || !p.x1 || !p.x2 || !p.gout) return cueq::fail("channelwise backward: null tensor");
     if (!a->bwd_coef) return cueq::fail("channelwise backward: null coefficient table");
     p.recv_mod = a->recv_mod;
@@ -111,6 +116,7 @@ extern "C" int cueq_b200_cw_backward(int g, const cueq_cw_args* a, void* stream)
   if (a && a->dtype != CUEQ_F32) return cueq::fail("channelwise: float32 or float64 operands");
   CwParams p;
   if (int rc = fill_params(a, *kGroups[g], p, kGroups[g]->nterm)) return rc;
+  p.overlap = overlap;
   if (!p.w || !p.x1 || !p.x2 || !p.gout) return cueq::fail("channelwise backward: null tensor");
   if (!a->bwd_coef) return cueq::fail("channelwise backward: null coefficient table");
   if (p.num_receivers == 0) return 0;
@@ -135,8 +141,15 @@ extern "C" int cueq_b200_cw_backward(int g, const cueq_cw_args* a, void* stream)
   return kGroups[g]->bwd(p, coef, a->x1_mul_ir, pick_cpl(a), masked, reinterpret_cast<cudaStream_t>(stream));
 }
 
+}  // namespace
+
+extern "C" int cueq_b200_cw_forward(int g, const cueq_cw_args* a, void* stream) { return run_forward(g, a, 0, stream); }
+
+extern "C" int cueq_b200_cw_backward(int g, const cueq_cw_args* a, void* stream) { return run_backward(g, a, 0, stream); }
+
 // All groups of a polynomial by one call: the constant part of each group's arguments comes from `templates`, which the
-// caller keeps, tensors and sizes from `call`.  The groups are queued one after the other, as by separate calls.
+// caller keeps, tensors and sizes from `call`.  Every group but the first may start before the one in front of it has
+// ended (cw_kernels.cuh, launch_kernel).
 extern "C" int cueq_b200_cw_run(int backward, int num_groups, const int32_t* groups, const cueq_cw_args* templates, const cueq_cw_args* call,
                                 void* stream) {
   if (num_groups < 0 || (num_groups && (!groups || !templates || !call))) return cueq::fail("channelwise: null argument");
@@ -147,7 +160,7 @@ extern "C" int cueq_b200_cw_run(int backward, int num_groups, const int32_t* gro
     a.senders = call->senders; a.order = call->order; a.rowptr = call->rowptr;
     a.num_receivers = call->num_receivers; a.recv_mod = call->recv_mod; a.mean_degree = call->mean_degree;
     a.x1_mul_ir = call->x1_mul_ir; a.out_mul_ir = call->out_mul_ir;
-    if (int rc = backward ? cueq_b200_cw_backward(groups[i], &a, stream) : cueq_b200_cw_forward(groups[i], &a, stream)) return rc;
+    if (int rc = backward ? run_backward(groups[i], &a, i > 0, stream) : run_forward(groups[i], &a, i > 0, stream)) return rc;
   }
   return 0;
 }

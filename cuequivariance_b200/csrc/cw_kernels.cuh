@@ -107,6 +107,8 @@ __device__ __forceinline__ void red_add_hint(double* addr, const double (&v)[2],
   asm volatile("red.global.add.L2::cache_hint.f64 [%0], %1, %2;\n" ::"l"(addr), "d"(v[0]), "l"(policy) : "memory");
   asm volatile("red.global.add.L2::cache_hint.f64 [%0], %1, %2;\n" ::"l"(addr + 1), "d"(v[1]), "l"(policy) : "memory");
 }
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
@@ -338,6 +340,7 @@ template <class T> constexpr int kFwdMinBlocks = sizeof(T) == 8 ? 2 : CW_MINBLOC
 
 template <class T, class G, int C, bool MUL_IR, bool MASKED>
 __global__ void __launch_bounds__(kWarps * 32, kFwdMinBlocks<T>) cw_fwd_kernel(const __grid_constant__ CwParamsT<T> p) {
+  let_next_start();
   extern __shared__ __align__(16) unsigned char smem_bytes[];
   T* smem = reinterpret_cast<T*>(smem_bytes);
   using S = Smem<G, C, T>;
@@ -384,6 +387,7 @@ __global__ void __launch_bounds__(kWarps * 32, kFwdMinBlocks<T>) cw_fwd_kernel(c
     }
     if (active) StoreOut<G, C, 0, MUL_IR, MASKED, T>::run(p.out + (int64_t)n * p.out_stride, p, ch, acc);
   }
+  wait_for_previous();
 }
 
 // ---- forward, staging by bulk copies ----------------------------------------------------------
@@ -556,6 +560,7 @@ __device__ __forceinline__ T reduce16(T (&r)[16], int lane) {
 
 template <class G, int C, bool MUL_IR, bool MASKED>
 __global__ void __launch_bounds__(kWarps * 32, CW_MINBLOCKS) cw_bwd_kernel(const __grid_constant__ CwParams p, const __grid_constant__ CwCoef coef) {
+  let_next_start();
   extern __shared__ __align__(16) float smem[];
   using S = Smem<G, C>;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -617,6 +622,7 @@ __global__ void __launch_bounds__(kWarps * 32, CW_MINBLOCKS) cw_bwd_kernel(const
       __syncwarp();
     }
   }
+  wait_for_previous();
 }
 
 // ---- backward, one thread block per receiver ---------------------------------------------------
@@ -648,6 +654,7 @@ struct StageGSplit {
 
 template <class T, class G, int C, bool MUL_IR, bool BULK_RED, bool NEED_GX2, bool MASKED>
 __global__ void __launch_bounds__(kWarps * 32, sizeof(T) == 8 ? 2 : C == 2 ? 4 : 3) cw_bwd_block_kernel(const __grid_constant__ CwParamsT<T> p, const __grid_constant__ CwCoefT<T> coef) {
+  let_next_start();
   // BULK_RED (mul_ir rows only): the x1 gradient of an edge - the 32 lanes' C*D1 values are one contiguous run of
   // the sender's row - leaves as ONE bulk reduction per warp and edge instead of D1 vector reductions per lane.
   // Its shared-memory source is the slot the edge's x1 block was staged in (free once X is in registers); the
@@ -763,9 +770,32 @@ __global__ void __launch_bounds__(kWarps * 32, sizeof(T) == 8 ? 2 : C == 2 ? 4 :
     }
   }
   if (kBulk && lane == 0) bulk_wait_all();                           // shared memory stays allocated until the last reduction is done
+  wait_for_previous();
 }
 
 // ---- launchers ----------------------------------------------------------------------------------
+// The groups of one call read the same inputs and write different columns (the x2 gradient adds up), so a group need not
+// wait for the one before it: its blocks fill the SMs that the other's last wave leaves idle.  Every kernel lets its
+// successor start at once and ends only when its predecessor has, so that the end of the last group is the end of all.
+// Only a launch that says so starts early; the first group of a call waits for everything before it as usual.
+// 65,536 unsorted edges on 4,096 nodes, 128 channels, forward: 244 -> 220 us; 40,003 edges, 96 channels, lmax 2, forward and
+// gradients: 402 -> 340 us.  The groups' parts of the x2 gradient then add up in no fixed order, as those of x1 always did.
+template <class... Params, class... Args>
+int launch_kernel(void (*kernel)(Params...), dim3 grid, size_t smem, cudaStream_t st, int overlap, const Args&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(kWarps * 32);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = overlap ? 1 : 0;
+  CUEQ_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, args...));
+  return 0;
+}
+
 int grid_x(int num_receivers) {
   const int want = (num_receivers + kWarps - 1) / kWarps;
   const int cap = 148 * 32;
@@ -781,9 +811,7 @@ int launch_fwd_t(const CwParamsT<T>& p, cudaStream_t st) {
     configured.set();
   }
   dim3 grid(grid_x(p.num_receivers), (p.extent + 32 * C - 1) / (32 * C));
-  cw_fwd_kernel<T, G, C, A, MASKED><<<grid, kWarps * 32, smem, st>>>(p);
-  CUEQ_CUDA_OK(cudaGetLastError());
-  return 0;
+  return launch_kernel(cw_fwd_kernel<T, G, C, A, MASKED>, grid, smem, st, p.overlap, p);
 }
 
 template <class G, int C, bool A>
@@ -826,9 +854,7 @@ int launch_bwd_t(const CwParams& p, const CwCoef& coef, cudaStream_t st) {
     configured.set();
   }
   dim3 grid(grid_x(p.num_receivers), (p.extent + 32 * C - 1) / (32 * C));
-  cw_bwd_kernel<G, C, A, MASKED><<<grid, kWarps * 32, smem, st>>>(p, coef);
-  CUEQ_CUDA_OK(cudaGetLastError());
-  return 0;
+  return launch_kernel(cw_bwd_kernel<G, C, A, MASKED>, grid, smem, st, p.overlap, p, coef);
 }
 
 template <class G, bool MASKED>
@@ -855,9 +881,7 @@ int launch_bwd_block_t(const CwParamsT<T>& p, const CwCoefT<T>& coef, cudaStream
   // balance the uneven edge counts better than eight waves of long ones (l = 3 launch 3.48 -> 3.40 ms)
   const int cap = 148 * 96;
   dim3 grid(p.num_receivers < cap ? p.num_receivers : cap, (p.extent + 32 * C - 1) / (32 * C));
-  cw_bwd_block_kernel<T, G, C, A, BULK, GX2, MASKED><<<grid, kWarps * 32, smem, st>>>(p, coef);
-  CUEQ_CUDA_OK(cudaGetLastError());
-  return 0;
+  return launch_kernel(cw_bwd_block_kernel<T, G, C, A, BULK, GX2, MASKED>, grid, smem, st, p.overlap, p, coef);
 }
 
 // bulk: the x1 gradient leaves as one bulk reduction per warp and edge; needs mul_ir rows whose blocks start on
