@@ -262,6 +262,7 @@ class DenseUVW:
         self.out_size = d.operands[3].size
         self._flat = {}
         self._wcache = {}
+        self._tri_mul = {}
 
     def _weights_bf16(self, w: torch.Tensor, transposed: bool) -> torch.Tensor:
         """The shared weights as bf16 rows of 64, in ``[u][v][w]`` order or (``transposed``) ``[v][u][w]``.  The same
@@ -293,6 +294,12 @@ class DenseUVW:
     # -- tri-linear route: the output and both input gradients without a coupled operand ---------
     def _tri_channels(self, dtype) -> int:
         """The common multiplicity when ``cueq_b200_fctp_tri`` takes the product in this dtype, else 0."""
+        c = self._tri_mul.get(dtype)
+        if c is None:
+            c = self._tri_mul[dtype] = self._find_tri_channels(dtype)
+        return c
+
+    def _find_tri_channels(self, dtype) -> int:
         d = self.d
         muls = {m for p in d.paths for m in d.operands[0].segments[p.indices[0]]}
         muls |= {s[1] for op in d.operands[1:] for s in op.segments}
