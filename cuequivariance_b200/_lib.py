@@ -279,6 +279,7 @@ def lib() -> C.CDLL:
     L.cueq_b200_sh_width.argtypes = [C.c_uint32]
     L.cueq_b200_sh_forward.argtypes = [C.POINTER(ShArgs), C.c_void_p]
     L.cueq_b200_sh_backward.argtypes = [C.POINTER(ShArgs), C.c_void_p]
+    L.cueq_b200_sh_second.argtypes = [C.POINTER(ShArgs), C.c_void_p, C.c_int64, C.c_void_p, C.c_int64, C.c_void_p]
     L.cueq_b200_cw_forward.argtypes = [C.c_int, C.POINTER(CwArgs), C.c_void_p]
     L.cueq_b200_cw_backward.argtypes = [C.c_int, C.POINTER(CwArgs), C.c_void_p]
     L.cueq_b200_csr_rowptr.argtypes = [C.c_void_p, C.c_int, C.c_int64, C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p]

@@ -8,7 +8,8 @@
 // trip through memory, and so do the cotangents on the way back.  Here one thread owns one vector: it
 // reads 3 numbers and writes sum(2l+1) (forward), or reads 3 + sum(2l+1) and writes 3 (backward:
 // g_vec = P (J^T g) / |v| with P = 1 - n n^T the projector that differentiating the normalisation gives).
-// Memory-bound by construction: 12 + 4 sum(2l+1) bytes per edge each way in float32.
+// Memory-bound by construction: 12 + 4 sum(2l+1) bytes per edge each way in float32.  The derivative of the backward pass
+// (forces inside a training loss) is a third kernel.
 #include "common.cuh"
 #include "generated/sh_poly.cuh"
 
@@ -36,6 +37,19 @@ __device__ __forceinline__ void vjp_all(T x, T y, T z, unsigned mask, const T* _
 
 constexpr int kMaxOut = 25;   // 1 + 3 + 5 + 7 + 9
 
+// A value and its derivative along one direction: the generated polynomials, evaluated on these, give second derivatives.
+template <typename T>
+struct Dual {
+  T v, d;
+  Dual() = default;
+  __device__ __forceinline__ explicit Dual(double c) : v(T(c)), d(T(0)) {}
+  __device__ __forceinline__ Dual(T v_, T d_) : v(v_), d(d_) {}
+  __device__ __forceinline__ Dual& operator+=(const Dual& o) { v += o.v; d += o.d; return *this; }
+};
+template <typename T> __device__ __forceinline__ Dual<T> operator+(const Dual<T>& a, const Dual<T>& b) { return Dual<T>(a.v + b.v, a.d + b.d); }
+template <typename T> __device__ __forceinline__ Dual<T> operator-(const Dual<T>& a, const Dual<T>& b) { return Dual<T>(a.v - b.v, a.d - b.d); }
+template <typename T> __device__ __forceinline__ Dual<T> operator*(const Dual<T>& a, const Dual<T>& b) { return Dual<T>(a.v * b.v, a.d * b.v + a.v * b.d); }
+
 template <typename T>
 __device__ __forceinline__ T inv_norm(T x, T y, T z) {
   // torch.nn.functional.normalize: v / max(|v|, 1e-12)
@@ -61,29 +75,76 @@ __global__ void __launch_bounds__(256) sh_forward_kernel(const T* __restrict__ v
   }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256) sh_backward_kernel(const T* __restrict__ vec, const T* __restrict__ gout, T* __restrict__ gvec,
+// The derivatives are evaluated in float64 for float32 vectors too: a gradient is a sum of up to 24 partly cancelling terms
+// (and a second derivative has three times as many), it is differentiated again in a force loss, and the kernels wait for
+// memory either way.  Error of the forces / of the force loss's gradient against float64, 20,000 edges: 8.3e-8 / 1.1e-7, in
+// float32 2.1e-7 / 4.3e-7, by the polynomials that a loss on forces used before 1.7e-7 / 3.1e-7.
+template <typename IO, typename T = double>
+__global__ void __launch_bounds__(256) sh_backward_kernel(const IO* __restrict__ vec, const IO* __restrict__ gout, IO* __restrict__ gvec,
                                                           int64_t rows, int64_t ld_vec, int64_t ld_g, int64_t ld_gvec, unsigned mask,
                                                           int width, int normalize) {
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < rows; r += (int64_t)gridDim.x * blockDim.x) {
-    T x = vec[r * ld_vec], y = vec[r * ld_vec + 1], z = vec[r * ld_vec + 2];
+    T x = T(vec[r * ld_vec]), y = T(vec[r * ld_vec + 1]), z = T(vec[r * ld_vec + 2]);
     T s = T(1);
     if (normalize) {
       s = inv_norm(x, y, z);
       x *= s; y *= s; z *= s;
     }
     T g[kMaxOut];
-    const T* src = gout + r * ld_g;
+    const IO* src = gout + r * ld_g;
 #pragma unroll
-    for (int k = 0; k < kMaxOut; ++k) g[k] = k < width ? src[k] : T(0);
+    for (int k = 0; k < kMaxOut; ++k) g[k] = k < width ? T(src[k]) : T(0);
     T gx = T(0), gy = T(0), gz = T(0);
     vjp_all(x, y, z, mask, g, gx, gy, gz);
     if (normalize) {   // d(v/|v|) = (1 - n n^T) dv / |v|
       const T dot = gx * x + gy * y + gz * z;
       gx = (gx - dot * x) * s; gy = (gy - dot * y) * s; gz = (gz - dot * z) * s;
     }
-    T* dst = gvec + r * ld_gvec;
-    dst[0] = gx; dst[1] = gy; dst[2] = gz;
+    IO* dst = gvec + r * ld_gvec;
+    dst[0] = IO(gx); dst[1] = IO(gy); dst[2] = IO(gz);
+  }
+}
+
+// Derivative of <h, g_vec(vec, g)>: with respect to g it is the derivative of the harmonics along h, with respect to vec
+// that of g_vec along h (the Hessian of <g, Y> is symmetric).  One pass, 24 + 8 sum(2l+1) + 12 bytes per vector in float32;
+// before, the gradient was rebuilt as a polynomial over normalised vectors whenever it had to be differentiable, some fifty
+// kernels and their autograd nodes: a force loss on 65,536 edges 2015 us, 1638 us with this kernel.
+template <typename IO, typename T = double>
+__global__ void __launch_bounds__(256) sh_second_kernel(const IO* __restrict__ vec, const IO* __restrict__ gout, const IO* __restrict__ h,
+                                                        IO* __restrict__ gvec, IO* __restrict__ gg, int64_t rows, int64_t ld_vec, int64_t ld_g,
+                                                        int64_t ld_h, int64_t ld_gvec, int64_t ld_gg, unsigned mask, int width, int normalize) {
+  using D = Dual<T>;
+  for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < rows; r += (int64_t)gridDim.x * blockDim.x) {
+    const IO *v = vec + r * ld_vec, *w = h + r * ld_h;
+    D x{T(v[0]), T(w[0])}, y{T(v[1]), T(w[1])}, z{T(v[2]), T(w[2])};
+    D s(T(1), T(0));
+    if (normalize) {
+      const D n2 = x * x + y * y + z * z;
+      const T i = inv_norm(x.v, y.v, z.v);
+      // d(1 / |v|) = -d(|v|^2) / (2 |v|^3); constant where the norm is clamped
+      s = D(i, n2.v > T(1e-24) ? T(-0.5) * n2.d * i * i * i : T(0));
+      x = x * s; y = y * s; z = z * s;
+    }
+    {
+      D out[kMaxOut];
+      eval_all(x, y, z, mask, out);
+      IO* dst = gg + r * ld_gg;
+#pragma unroll
+      for (int k = 0; k < kMaxOut; ++k)
+        if (k < width) dst[k] = IO(out[k].d);
+    }
+    D g[kMaxOut];
+    const IO* src = gout + r * ld_g;
+#pragma unroll
+    for (int k = 0; k < kMaxOut; ++k) g[k] = D(k < width ? T(src[k]) : T(0), T(0));
+    D gx(T(0), T(0)), gy(T(0), T(0)), gz(T(0), T(0));
+    vjp_all(x, y, z, mask, g, gx, gy, gz);
+    if (normalize) {
+      const D dot = gx * x + gy * y + gz * z;
+      gx = (gx - dot * x) * s; gy = (gy - dot * y) * s; gz = (gz - dot * z) * s;
+    }
+    IO* dst = gvec + r * ld_gvec;
+    dst[0] = IO(gx.d); dst[1] = IO(gy.d); dst[2] = IO(gz.d);
   }
 }
 
@@ -137,6 +198,22 @@ extern "C" int cueq_b200_sh_backward(const cueq_sh_args* a, void* stream) {
   else
     sh_backward_kernel<double><<<grid_for(a->rows), 256, 0, st>>>((const double*)a->vec, (const double*)a->y, (double*)a->gvec, a->rows, a->ld_vec,
                                                                     a->ld_y, a->ld_gvec, a->ls_mask, w, a->normalize);
+  CUEQ_CUDA_OK(cudaGetLastError());
+  return 0;
+}
+
+extern "C" int cueq_b200_sh_second(const cueq_sh_args* a, const void* h, int64_t ld_h, void* gg, int64_t ld_gg, void* stream) {
+  if (int rc = check(a)) return rc;
+  if (!a->gvec || !h || !gg) return cueq::fail("spherical harmonics second derivative: null tensor");
+  if (a->rows == 0) return 0;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  const int w = width_of(a->ls_mask);
+  if (a->dtype == CUEQ_F32)
+    sh_second_kernel<float><<<grid_for(a->rows), 256, 0, st>>>((const float*)a->vec, (const float*)a->y, (const float*)h, (float*)a->gvec, (float*)gg, a->rows,
+                                                                 a->ld_vec, a->ld_y, ld_h, a->ld_gvec, ld_gg, a->ls_mask, w, a->normalize);
+  else
+    sh_second_kernel<double><<<grid_for(a->rows), 256, 0, st>>>((const double*)a->vec, (const double*)a->y, (const double*)h, (double*)a->gvec, (double*)gg,
+                                                                  a->rows, a->ld_vec, a->ld_y, ld_h, a->ld_gvec, ld_gg, a->ls_mask, w, a->normalize);
   CUEQ_CUDA_OK(cudaGetLastError());
   return 0;
 }

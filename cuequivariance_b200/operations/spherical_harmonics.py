@@ -16,7 +16,7 @@ FUSED = True       # degrees 0..4, float32/float64 CUDA tensors: the fused kerne
 FUSED_LMAX = 4
 
 
-def _launch(which: str, vec, y, gvec, mask: int, normalize: bool):
+def _launch(which: str, vec, y, gvec, mask: int, normalize: bool, h=None, gg=None):
     import ctypes as C
 
     from .. import _lib, profiling
@@ -28,15 +28,16 @@ def _launch(which: str, vec, y, gvec, mask: int, normalize: bool):
     a.ld_gvec = gvec.stride(0) if gvec is not None else 0
     a.ls_mask, a.normalize = mask, 1 if normalize else 0
     a.dtype = _lib.F32 if vec.dtype == torch.float32 else _lib.F64
-    fn = _lib.lib().cueq_b200_sh_forward if which == "forward" else _lib.lib().cueq_b200_sh_backward
-    with torch.cuda.device(vec.device), profiling.kernel(f"sh_fused_{which}"):
-        _lib.check(fn(C.byref(a), C.c_void_p(torch.cuda.current_stream(vec.device).cuda_stream)))
+    L, stream = _lib.lib(), C.c_void_p(torch.cuda.current_stream(vec.device).cuda_stream)
+    with _lib.on_device(vec.device), profiling.kernel(f"sh_fused_{which}"):
+        if which == "second":
+            _lib.check(L.cueq_b200_sh_second(C.byref(a), h.data_ptr(), h.stride(0), gg.data_ptr(), gg.stride(0), stream))
+        else:
+            _lib.check((L.cueq_b200_sh_forward if which == "forward" else L.cueq_b200_sh_backward)(C.byref(a), stream))
 
 
 class _FusedSH(torch.autograd.Function):
-    """Forward and first derivative on the fused kernels.  When the derivative itself has to be
-    differentiable (``create_graph=True``, e.g. forces inside a training loss) the backward pass is
-    evaluated through the polynomial executor instead, which is differentiable to any order."""
+    """Forward and first derivative on the fused kernels; the derivative is differentiable (forces inside a training loss)."""
 
     @staticmethod
     def forward(ctx, module, vec):
@@ -50,15 +51,34 @@ class _FusedSH(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         (vec,) = ctx.saved_tensors
-        module = ctx.module
-        if torch.is_grad_enabled():
-            with torch.enable_grad():
-                y = module._polynomial_route(vec)
-                (gv,) = torch.autograd.grad(y, vec, g, create_graph=True)
-            return None, gv
+        return None, _FusedSHGrad.apply(ctx.module, vec, g)
+
+
+class _FusedSHGrad(torch.autograd.Function):
+    """Gradient to the vectors; its own derivative is one kernel.  Where that in turn has to be differentiable, the
+    harmonics are evaluated through the polynomial executor, which is differentiable to any order."""
+
+    @staticmethod
+    def forward(ctx, module, vec, g):
         gv = torch.empty((vec.shape[0], 3), dtype=vec.dtype, device=vec.device)
         _launch("backward", vec.contiguous(), g.contiguous(), gv, module.mask, module.normalize)
-        return None, gv
+        ctx.module = module
+        ctx.save_for_backward(vec, g)
+        return gv
+
+    @staticmethod
+    def backward(ctx, h):
+        vec, g = ctx.saved_tensors
+        module = ctx.module
+        if torch.is_grad_enabled():
+            y = module._polynomial_route(vec)
+            (gv,) = torch.autograd.grad(y, vec, g, create_graph=True)
+            wanted = [t for t, need in zip((vec, g), ctx.needs_input_grad[1:]) if need]
+            grads = iter(torch.autograd.grad(gv, wanted, h, create_graph=True, allow_unused=True))
+            return (None, *(next(grads) if need else None for need in ctx.needs_input_grad[1:]))
+        gvec, gg = torch.empty((vec.shape[0], 3), dtype=vec.dtype, device=vec.device), torch.empty_like(g, memory_format=torch.contiguous_format)
+        _launch("second", vec.contiguous(), g.contiguous(), gvec, module.mask, module.normalize, h.contiguous(), gg)
+        return None, gvec, gg
 
 
 class SphericalHarmonics(nn.Module):

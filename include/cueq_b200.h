@@ -169,6 +169,9 @@ typedef struct {
 int cueq_b200_sh_width(uint32_t ls_mask);
 int cueq_b200_sh_forward(const cueq_sh_args* args, void* stream);
 int cueq_b200_sh_backward(const cueq_sh_args* args, void* stream);
+/* Second derivative: with `y` = g, the cotangent of the harmonics, and h [rows, 3], a cotangent of g_vec: gvec receives the
+ * gradient of <h, g_vec> with respect to the vectors, gg [rows, width] the one with respect to g. */
+int cueq_b200_sh_second(const cueq_sh_args* args, const void* h, int64_t ld_h, void* gg, int64_t ld_gg, void* stream);
 
 /* ---- channelwise ("uvu") tensor product, specialised kernels --------------------------------
  *
