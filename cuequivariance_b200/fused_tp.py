@@ -17,13 +17,16 @@ Two routes:
     TMA + tcgen05 GEMM (float32 accumulation in TMEM); the backward runs two more GEMMs per
     path (weight gradient with both operands MN-major, so nothing is transposed in memory;
     gradient of Z) and a kernel that folds the gradient of Z back onto x1 and x2.  First
-    derivatives only.  ``Z`` makes a round trip through HBM; building its tiles directly in
-    shared memory inside the GEMM is the remaining step.
-  - float32 inputs: the same decomposition in float32 accuracy.  ``Z`` is written in float32 (the
-    paths that feed one output irrep side by side, so one GEMM per output component contracts them
-    all) and contracted by this library's three-pass TF32 tcgen05 GEMMs (``dense.gemm_f32x3`` and
-    its row-reduction twin for the weight gradient); differentiable to any order, because every
-    derivative of a tri-linear map is again one of the same four contractions.
+    derivatives only.  ``Z`` makes a round trip through HBM.
+    With 64 channels its tiles are built in shared memory instead (``csrc/fctp_fused.cu``), with 128 the output
+    and the input gradients take the kernels of the float32 route.
+  - float32 inputs, all multiplicities 32, 64 or 96 and l <= 2: ``csrc/fctp_tri.cu`` (output and input gradients: one
+    operand is contracted with the weights on the tensor cores, the other folded in from TMEM) and
+    ``csrc/fctp_gw.cu`` (weight gradient), three TF32 passes; nothing of the size of ``Z`` is in memory.  Other shapes:
+    ``Z`` is written in float32 (the paths that feed one output irrep side by side, so one GEMM per output component
+    contracts them all) and contracted by this library's three-pass TF32 tcgen05 GEMMs (``dense.gemm_f32x3`` and its
+    row-reduction twin for the weight gradient).  Differentiable to any order, because every derivative of a
+    tri-linear map is again one of the same four contractions.
   - float64 inputs and per-sample weights: the generic kernel on the fully flattened product.
 """
 from __future__ import annotations
@@ -143,8 +146,10 @@ class _TensorCoreUVW(torch.autograd.Function):
         B = x1.shape[0]
         dev = x1.device
         status = _lib.status_word(dev)
-        if FUSED and owner._tri_channels(torch.bfloat16):
-            out = owner.tri_map(2, w, (x1.to(torch.bfloat16), x2.to(torch.bfloat16)), "fctp_fused_forward")
+        # operands that hold more than bf16 keep it on the other routes
+        ctx.tri = FUSED and x1.dtype == x2.dtype == torch.bfloat16 and owner._tri_channels(torch.bfloat16) > 0
+        if ctx.tri:
+            out = owner.tri_map(2, w, (x1, x2), "fctp_fused_forward")
             ctx.owner, ctx.status = owner, status
             ctx.save_for_backward(w, x1, x2)
             return out.to(x1.dtype)
@@ -187,12 +192,12 @@ class _TensorCoreUVW(torch.autograd.Function):
         status = ctx.status
         fused_x = FUSED and owner._fused_tasks() is not None and owner._fused_units(1) is not None and owner._fused_wunits() is not None
         gx1f = gx2f = gwf = None
-        if FUSED and owner._tri_channels(torch.bfloat16) and (need_x1 or need_x2):
+        if ctx.tri and (need_x1 or need_x2):
             gout16 = gout.to(torch.bfloat16)
             if need_x1:
-                gx1f = owner.tri_map(0, w, (x2.to(torch.bfloat16), gout16), "fctp_fused_gx1")
+                gx1f = owner.tri_map(0, w, (x2, gout16), "fctp_fused_gx1")
             if need_x2:
-                gx2f = owner.tri_map(1, w, (x1.to(torch.bfloat16), gout16), "fctp_fused_gx2")
+                gx2f = owner.tri_map(1, w, (x1, gout16), "fctp_fused_gx2")
             need_x1 = need_x2 = False
         if fused_x and (need_x1 or need_x2 or need_w):
             gout16 = gout.to(torch.bfloat16).contiguous()

@@ -226,9 +226,10 @@ class Linear(torch.nn.Module):
     when ``internal_weights``), ``[batch, weight_numel]`` otherwise; ``weight_indices``:
     ``[batch]`` class ids, required when ``weight_classes > 1``.
 
-    float32 with one weight set and multiplicities that are multiples of 32 runs as float32-accurate
-    tensor-core GEMMs (``dense.gemm_f32x3`` / ``gemm_f32x3_tn``; first derivatives only); everything else
-    runs on the generic kernel over the polynomial ``uv,iu,iv``
+    float32 with multiplicities 32, 64, 96 or 128 and no two paths on one block of rows runs as one float32-accurate
+    tensor-core launch per result, all irreps and (sorted) weight classes included (``csrc/linear_fused.cu``); other
+    multiples of 32 as one GEMM per irrep and component (``dense.gemm_f32x3`` / ``gemm_f32x3_tn``); first derivatives
+    only.  Everything else runs on the generic kernel over the polynomial ``uv,iu,iv``
     flattened over ``u``.  There is no ``naive`` method and no fallback."""
 
     def __init__(
