@@ -15,7 +15,7 @@
 // once per component of the smaller operand (35 against 27 blocks of 64^3 per sample).
 //
 // float32: P and W are split into TF32 halves (P on chip, W by fctp_tri_weights), three passes, small terms first, so
-// that an accumulation chain has K / 8 <= 12 additions at full magnitude; all further sums are float32 FMAs.
+// that an accumulation chain has K / 8 <= 8 additions at full magnitude; all further sums are float32 FMAs.
 // bf16: one pass; Y stays in float32, where the route before rounded the products of the inputs to bf16.
 // What bounds it, per launch set at 32,768 samples of 64x(0e+1o+2e), float32: 3.5 ms.  The MMAs alone need 1.2 ms (27 * 64^3 * 3
 // multiply-adds per sample); they wait for the weight blocks, 64 KB per 128 columns, of which two fit beside the operand
@@ -58,7 +58,7 @@ struct Cfg {
   static constexpr int RT = C <= 64 ? C : C / 2;       // channels of the result per thread block
   static constexpr int RPT = RT / 4;                   // per thread
   static constexpr int NQ = RT == 32 ? 4 : 2;          // q values per accumulator
-  static constexpr int NT = NQ * RT;                   // accumulator columns: 128 (C = 96: 96)
+  static constexpr int NT = NQ * RT;                   // accumulator columns: 128
   static constexpr int KB = BF16 ? 64 : 32;            // elements per 128-byte operand row
   static constexpr int NKB = C / KB;
   static constexpr int kTwin = BF16 ? 1 : 2;           // hi (and lo)
@@ -111,17 +111,6 @@ __device__ __forceinline__ void tmem_ld(unsigned t, float (&y)[8]) {
 #pragma unroll
   for (int c = 0; c < 8; ++c) y[c] = __uint_as_float(v[c]);
 }
-__device__ __forceinline__ void tmem_ld(unsigned t, float (&y)[12]) {
-  unsigned v[12];
-#pragma unroll
-  for (int k = 0; k < 12; k += 4)
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];\n"
-                 : "=r"(v[k]), "=r"(v[k + 1]), "=r"(v[k + 2]), "=r"(v[k + 3]) : "r"(t + k));
-  asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-#pragma unroll
-  for (int c = 0; c < 12; ++c) y[c] = __uint_as_float(v[c]);
-}
-
 template <bool BF16, int C, int NC>
 __global__ void __launch_bounds__(kThreads, 1) fctp_tri_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_constant__ CUtensorMap map_lo,
                                                                const __grid_constant__ TriParams p) {
@@ -499,7 +488,6 @@ extern "C" int cueq_b200_fctp_tri(const cueq_fctp_tri_args* a, void* stream) {
   } else {
     if (C == 32) return launch<false, 32>(a, p, st);
     if (C == 64) return launch<false, 64>(a, p, st);
-    if (C == 96) return launch<false, 96>(a, p, st);
   }
   return cueq::fail("fctp tri: %d channels are not covered", C);
 }

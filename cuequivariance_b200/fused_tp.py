@@ -20,9 +20,9 @@ Two routes:
     derivatives only.  ``Z`` makes a round trip through HBM.
     With 64 channels its tiles are built in shared memory instead (``csrc/fctp_fused.cu``), with 128 the output
     and the input gradients take the kernels of the float32 route.
-  - float32 inputs, all multiplicities 32, 64 or 96 and l <= 2: ``csrc/fctp_tri.cu`` (output and input gradients: one
+  - float32 inputs, l <= 2: ``csrc/fctp_tri.cu`` (output and input gradients, all multiplicities 32 or 64: one
     operand is contracted with the weights on the tensor cores, the other folded in from TMEM) and
-    ``csrc/fctp_gw.cu`` (weight gradient), three TF32 passes; nothing of the size of ``Z`` is in memory.  Other shapes:
+    ``csrc/fctp_gw.cu`` (weight gradient, all multiplicities 32, 64 or 96), three TF32 passes; nothing of the size of ``Z`` is in memory.  Other shapes:
     ``Z`` is written in float32 (the paths that feed one output irrep side by side, so one GEMM per output component
     contracts them all) and contracted by this library's three-pass TF32 tcgen05 GEMMs (``dense.gemm_f32x3`` and its
     row-reduction twin for the weight gradient).  Differentiable to any order, because every derivative of a
@@ -267,7 +267,7 @@ class DenseUVW:
         self.out_size = d.operands[3].size
         self._flat = {}
         self._wcache = {}
-        self._tri_mul = {}
+        self._tri_mul = None
 
     def _weights_bf16(self, w: torch.Tensor, transposed: bool) -> torch.Tensor:
         """The shared weights as bf16 rows of 64, in ``[u][v][w]`` order or (``transposed``) ``[v][u][w]``.  The same
@@ -299,12 +299,24 @@ class DenseUVW:
     # -- tri-linear route: the output and both input gradients without a coupled operand ---------
     def _tri_channels(self, dtype) -> int:
         """The common multiplicity when ``cueq_b200_fctp_tri`` takes the product in this dtype, else 0."""
-        c = self._tri_mul.get(dtype)
-        if c is None:
-            c = self._tri_mul[dtype] = self._find_tri_channels(dtype)
-        return c
+        c = self._common_multiplicity()
+        # bf16 with 64 channels has kernels of its own (fctp_fused.cu), which are faster: 5.4 against 6.2 ms for the output
+        # and both input gradients of 32,768 samples of 64x(0e+1o+2e).  Other shapes used to write the coupled operand to
+        # memory: the same sums in float32 took 23 ms, 10 ms here.  float32 with 96 channels stays there: chains of twelve
+        # additions in the tensor core, input gradients 3.8e-7 off where the memory route is 2.5e-7 off.
+        return c if c in ((128,) if dtype == torch.bfloat16 else (32, 64)) else 0
 
-    def _find_tri_channels(self, dtype) -> int:
+    def _gw_channels(self) -> int:
+        """Likewise for ``cueq_b200_fctp_gw`` (float32)."""
+        c = self._common_multiplicity()
+        return c if c in (32, 64, 96) else 0
+
+    def _common_multiplicity(self) -> int:
+        if self._tri_mul is None:
+            self._tri_mul = self._find_multiplicity()
+        return self._tri_mul
+
+    def _find_multiplicity(self) -> int:
         d = self.d
         muls = {m for p in d.paths for m in d.operands[0].segments[p.indices[0]]}
         muls |= {s[1] for op in d.operands[1:] for s in op.segments}
@@ -313,10 +325,7 @@ class DenseUVW:
         (c,) = muls
         if any(n not in (1, 3, 5) for p in d.paths for n in p.coefficients.shape):
             return 0
-        # bf16 with 64 channels has kernels of its own (fctp_fused.cu), which are faster: 5.4 against 6.2 ms for the output
-        # and both input gradients of 32,768 samples of 64x(0e+1o+2e).  Other shapes used to write the coupled operand to
-        # memory: the same sums in float32 took 23 ms, 10 ms here.
-        return c if c in ((128,) if dtype == torch.bfloat16 else (32, 64, 96)) else 0
+        return c
 
     def _tri_plan(self, which: int):
         """Path tables for the derivative of the trilinear form with respect to operand ``which`` (0: x1, 1: x2, 2: the
@@ -465,7 +474,7 @@ class DenseUVW:
                 a.paths = C.cast(paths, C.POINTER(_lib.FctpGwPath))
                 a.status = _lib.status_word(dev).data_ptr()
                 a.rows, a.zp, a.batch = rows, zp, nb
-                a.channels, a.num_paths, a.struct_bytes = self._tri_channels(torch.float32), len(self.d.paths), C.sizeof(a)
+                a.channels, a.num_paths, a.struct_bytes = self._gw_channels(), len(self.d.paths), C.sizeof(a)
                 with profiling.kernel(name):
                     _lib.check(L.cueq_b200_fctp_gw(C.byref(a), stream))
         return gw
@@ -760,7 +769,7 @@ class DenseUVW:
         """dPhi/dw: per path  gW[(u,v), w] = sum_(z,k) Z[(z,k),(u,v)] g[z, k, w]  (reduction over rows)."""
         from .dense import gemm_f32x3_tn
 
-        if self._tri_channels(torch.float32) and x1.shape[0]:
+        if self._gw_channels() and x1.shape[0]:
             return self.tri_gw((x1, x2, g), "fctp_f32_gw")
         d, off = self.d, self.offsets
         B, dev = x1.shape[0], x1.device

@@ -337,7 +337,7 @@ int cueq_b200_gemm_f32x3_tn(const cueq_gemm_f32x3_tn_args* args, void* stream);
 /* Fully connected product (uvw,iu,jv,kw+ijk, shared weights): output or input gradient, one irrep of the result per call.
  * R (the result), P and Q are the operands x1, x2, out / cotangent in the roles
  *   R[z, c, r] (+)= sum over paths, p, q, a, b of coef[a][b][c] W[p, q, r] P[z, a, p] Q[z, b, q]
- * All multiplicities are `channels` (32, 64, 96 in float32; 128 in bf16), irreps have dimension 1, 3 or 5.  P rows come
+ * All multiplicities are `channels` (32, 64 in float32; 128 in bf16), irreps have dimension 1, 3 or 5.  P rows come
  * as they are (ir_mul), Q transposed ([column][sample], cueq_b200_fctp_tri_transpose), the weights as rows ((q, r), p)
  * (cueq_b200_fctp_tri_weights; row block k * channels^2 belongs to path k).  With splits > 1 the sum over q is divided among that
  * many thread blocks and the result (zeroed by the caller) is added to. */

