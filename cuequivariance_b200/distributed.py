@@ -94,6 +94,13 @@ def all_gather_rows(x: torch.Tensor, group=None) -> torch.Tensor:
     return _AllGatherRows.apply(x, group)
 
 
+def _x1_gradient(plan, rows: int, device) -> torch.Tensor:
+    """Rows for the node-feature gradient, to be filled block by block.  An irrep of x1 that couples to nothing has no
+    group, so nobody writes its columns: they are zero."""
+    covered = sum(g["x1_width"] for g in plan.groups) == plan.row_sizes[1]
+    return (torch.empty if covered else torch.zeros)((rows, plan.row_sizes[1]), dtype=torch.float32, device=device)
+
+
 BUNDLES = 0   # exchanges per direction in the pipelined path (0: one per irrep, 1: one collective, 2: two bundles)
 
 
@@ -192,7 +199,7 @@ class _PipelinedShardedChannelwise(torch.autograd.Function):
         if need_x1:
             for wk in works:
                 wk.wait()
-            gx1 = torch.empty((ctx.n_local, plan.row_sizes[1]), dtype=torch.float32, device=gout.device)
+            gx1 = _x1_gradient(plan, ctx.n_local, gout.device)
             for bi, (a, b, off, width) in enumerate(bundles):
                 gx1[:, off : off + width] = pieces[bi]
         return None, None, gx1, gx2, gw, None, None
@@ -536,7 +543,7 @@ class _PeerCopyShardedChannelwise(torch.autograd.Function):
                 partial[l], ready[l] = gl, ex.handshake([ex.push(pieces, (done,))])
         gx1 = None
         if need_x1:
-            gx1 = torch.empty((n_local, plan.row_sizes[1]), dtype=torch.float32, device=dev)
+            gx1 = _x1_gradient(plan, n_local, dev)
             for l, g in enumerate(groups):
                 main.wait_event(ready[l])
                 gx1[:, g["x1_off"] : g["x1_off"] + g["x1_width"]] = ex.stage[l].sum(0)
