@@ -404,7 +404,8 @@ class _ChannelwiseBase:
                 t.w_offset[q] = g["w_off"][q]
                 t.out_offset[q] = g["out_off"][q]
             keep = None
-            t.path_mask, t.x2_width, t.dtype = g["mask"], plan.row_sizes[2], _lib.F64 if f64 else _lib.F32
+            # x2 holds l = 0, 1, 2, ... in order and no path of a group reads beyond l = 3: the first 16 components of a wider row
+            t.path_mask, t.x2_width, t.dtype = g["mask"], min(plan.row_sizes[2], 16), _lib.F64 if f64 else _lib.F32
             if which == "bwd_tab":
                 keep = ((C.c_double if f64 else C.c_float) * g["nterm"])(*g["bwd_tab"][2])
                 t.bwd_coef = C.cast(keep, C.c_void_p)

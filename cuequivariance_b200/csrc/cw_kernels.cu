@@ -19,9 +19,10 @@ int pick_cpl(const cueq_cw_args* a) {
   return a->extent >= 64 ? 2 : 4;
 }
 
-// A polynomial with all paths of the group and 16-element x2 rows takes the kernels that know so at compile time.
+// A polynomial with all paths of the group and 16-element x2 rows takes the kernels that know so at compile time and copy a
+// row 16 bytes at a time; rows at another pitch (harmonics beyond l = 3 that no path reads) go element by element as well.
 template <class T>
-bool is_masked(const CwParamsT<T>& p, const GroupEntry& g) { return p.path_mask != (1u << g.npath) - 1u || p.nx2 != g.nx2; }
+bool is_masked(const CwParamsT<T>& p, const GroupEntry& g) { return p.path_mask != (1u << g.npath) - 1u || p.nx2 != g.nx2 || (p.x2_stride & 3); }
 
 template <class T>
 int fill_params(const cueq_cw_args* a, const GroupEntry& g, CwParamsT<T>& p, int expected_terms) {
@@ -55,7 +56,6 @@ int fill_params(const cueq_cw_args* a, const GroupEntry& g, CwParamsT<T>& p, int
   p.path_mask = a->path_mask ? (unsigned)a->path_mask : all;
   p.nx2 = a->x2_width ? a->x2_width : g.nx2;
   if ((p.path_mask & ~all) || p.nx2 < 1 || p.nx2 > g.nx2) return cueq::fail("channelwise: path mask or x2 width outside the group");
-  if (!is_masked(p, g) && (a->x2_stride & 3)) return cueq::fail("channelwise: x2 row stride must be a multiple of 4 elements");
   if (ptrs & 15) return cueq::fail("channelwise: tensors must be 16-byte aligned");
   p.need_gw = a->gw != nullptr; p.need_gx1 = a->gx1 != nullptr; p.need_gx2 = a->gx2 != nullptr;
   return 0;

@@ -232,7 +232,7 @@ typedef struct {
                            rows, 128 | extent; falls back to 2 where the rows are not 16-byte aligned)        */
   int32_t path_mask;    /* bit q: path q of the group is part of the polynomial (0: all are); tables and offsets
                            keep the full group's numbering, entries of absent paths have no terms           */
-  int32_t x2_width;     /* components of an x2 row: 1, 4, 9 or 16 (0: 16)                               */
+  int32_t x2_width;     /* components of an x2 row that the paths read: 1, 4, 9 or 16 (0: 16)            */
   int32_t dtype;        /* CUEQ_F32, or CUEQ_F64: two channels per thread, staging / variant ignored    */
   int32_t mean_degree;    /* backward: edges per receiver, rounded down (0: unknown); picks the division of the work */
 } cueq_cw_args;
