@@ -195,8 +195,15 @@ class ChannelwisePlan:
         self.row_sizes = row_sizes          # (w, x1, x2, out) elements per row
         self.x1_blocks = x1_blocks          # ((mul, dim), ...) of x1
         self.out_blocks = out_blocks
+        self.complete = all(g["mask"] == (1 << g["npath"]) - 1 for g in groups)   # whole groups of the library
         self._dev: dict = {}
         self._templates: dict = {}          # constant launch arguments, see _ChannelwiseBase._run_groups
+
+    def takes(self, dtype) -> bool:
+        """Whether the kernels of this dtype take the channel count: 16-byte accesses along the channels."""
+        import torch
+
+        return (dtype == torch.float32 and self.extent % 4 == 0) or (dtype == torch.float64 and self.extent % 2 == 0)
 
     def tables_on(self, device, dtype=None):
         import torch
@@ -344,9 +351,7 @@ class _ChannelwiseBase:
         from . import _lib
 
         plan = self.plan
-        if program.math_dtype not in (torch.float32, torch.float64) or any(x.dtype != program.math_dtype for x in xs):
-            return None
-        if plan.extent % 4 and program.math_dtype == torch.float32:
+        if not plan.takes(program.math_dtype) or any(x.dtype != program.math_dtype for x in xs):
             return None
         w_s, x1_s, x2_s = cfg.inputs[0], cfg.inputs[1], cfg.inputs[2]
         if w_s.mode != _lib.BATCHED or x2_s.mode != _lib.BATCHED or x1_s.mode == _lib.SHARED:

@@ -573,7 +573,8 @@ class ReceiverShardedChannelWise(torch.nn.Module):
 
     def _handler(self, x1_local, x2, weight):
         """The specialised-kernel handler if the pipelined path applies (float32, mul_ir
-        layouts, per-edge weights, one launch per irrep of x1), else None."""
+        layouts, per-edge weights, one launch per irrep of x1), else None.  Only products of whole kernel groups take
+        it: the path is first-order only, and the others can be differentiated twice through the all-gather."""
         if not self.pipelined or not x1_local.is_cuda or x1_local.dtype != torch.float32:
             return None
         if x2.dtype != torch.float32 or weight.dtype != torch.float32 or weight.shape[0] != x2.shape[0]:
@@ -582,6 +583,8 @@ class ReceiverShardedChannelWise(torch.nn.Module):
         special = getattr(prog, "_special", None)
         lay = getattr(self.tp, "_layouts", {})
         if special is None or not hasattr(special, "launch_forward_group") or 1 not in lay or 3 not in lay:
+            return None
+        if not special.plan.complete or not special.plan.takes(torch.float32):
             return None
         offs = [g["x1_off"] for g in special.plan.groups]
         if len(set(offs)) != len(offs):
