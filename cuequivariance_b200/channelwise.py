@@ -58,14 +58,34 @@ def group_signature(l1: int, paths: Sequence[Tuple[int, int]]) -> str:
 
 
 # ---- run-time side ----------------------------------------------------------------------------
+def _capturing(device) -> bool:
+    """Whether the work that this call enqueues on ``device`` is being recorded into a CUDA graph."""
+    import torch
+
+    from . import _lib
+
+    if device.type != "cuda":
+        return torch.cuda.is_available() and torch.cuda.is_current_stream_capturing()
+    with _lib.on_device(device):
+        return torch.cuda.is_current_stream_capturing()
+
+
 class _CsrCache:
     """Receiver index -> (order or None, rowptr).  Keyed on the tensor's storage address and
     version counter, so in-place updates of the index are noticed; the cache holds a
-    reference to the tensor, which keeps that address from being recycled."""
+    reference to the tensor, which keeps that address from being recycled.  What is made while a CUDA graph is
+    being captured belongs to the graph (it holds nothing before the first replay) and is not kept."""
 
     def __init__(self, capacity: int = 8):
         self.capacity = capacity
         self.entries: list = []
+
+    def _keep(self, key, index, val):
+        if not _capturing(index.device):
+            self.entries.append((key, index, val))
+            if len(self.entries) > self.capacity:
+                self.entries.pop(0)
+        return val
 
     def get(self, index, num_rows: int):
         import torch
@@ -85,11 +105,7 @@ class _CsrCache:
                 sorted_idx, order = idx, None
             bounds = torch.arange(num_rows + 1, device=index.device, dtype=torch.int32)
             rowptr = torch.searchsorted(sorted_idx.contiguous(), bounds, right=False).to(torch.int32)
-        val = (order, rowptr)
-        self.entries.append((key, index, val))
-        if len(self.entries) > self.capacity:
-            self.entries.pop(0)
-        return val
+        return self._keep(key, index, (order, rowptr))
 
     @staticmethod
     def _rows_cuda(index, num_rows: int):
@@ -131,11 +147,7 @@ class _CsrCache:
         sorted_rows, order = torch.sort(rows, stable=True)
         bounds = torch.arange(passes * num_rows + 1, device=receivers.device, dtype=torch.int64)
         rowptr = torch.searchsorted(sorted_rows.contiguous(), bounds, right=False).to(torch.int32)
-        val = (order.to(torch.int32), rowptr)
-        self.entries.append((key, receivers, val))
-        if len(self.entries) > self.capacity:
-            self.entries.pop(0)
-        return val
+        return self._keep(key, receivers, (order.to(torch.int32), rowptr))
 
     def int32(self, index):
         import torch
@@ -146,11 +158,7 @@ class _CsrCache:
         for k, ref, val in self.entries:
             if k == key and ref is index:
                 return val
-        val = index.to(torch.int32).contiguous()
-        self.entries.append((key, index, val))
-        if len(self.entries) > self.capacity:
-            self.entries.pop(0)
-        return val
+        return self._keep(key, index, index.to(torch.int32).contiguous())
 
 
 _CSR = _CsrCache()
@@ -379,8 +387,9 @@ class _ChannelwiseBase:
             rp = _IDENTITY_ROWPTR.get(key)
             if rp is None:
                 rp = torch.arange(batch + 1, dtype=torch.int32, device=device)
-                _IDENTITY_ROWPTR.clear()
-                _IDENTITY_ROWPTR[key] = rp
+                if not _capturing(device):
+                    _IDENTITY_ROWPTR.clear()
+                    _IDENTITY_ROWPTR[key] = rp
             return None, rp, batch
         return None
 
