@@ -152,15 +152,18 @@ class _GroupedDenseLinear(torch.autograd.Function):
         return None, None, gw, gx
 
 
-def _fused_paths(paths, num_in: int, num_out: int):
+def _fused_paths(paths, x_op, out_op):
     """What ``cueq_b200_linear_map`` / ``_gw`` need, or None when they do not take the shape: every multiplicity 32, 64,
-    96 or 128, irreps up to l = 3, and no block of rows in more than one path."""
+    96 or 128, irreps up to l = 3, no block of rows in more than one path, and every row and block on a 16-byte boundary
+    (irreps without a path may have any multiplicity)."""
     if len(paths) > _lib.LINEAR_MAX_PATHS or any(u > 128 or v > 128 or d > 7 for (_, u, v, _, _, d, _) in paths):
+        return None
+    if x_op.size % 4 or out_op.size % 4 or any(xo % 4 or oo % 4 for (_, _, _, xo, oo, _, _) in paths):
         return None
     ins, outs = {p[3] for p in paths}, {p[4] for p in paths}
     if len(ins) != len(paths) or len(outs) != len(paths):
         return None
-    return {"paths": paths, "full_in": len(ins) == num_in, "full_out": len(outs) == num_out}
+    return {"paths": paths, "full_in": len(ins) == x_op.num_segments, "full_out": len(outs) == out_op.num_segments}
 
 
 def _aligned(t: torch.Tensor) -> torch.Tensor:
@@ -291,7 +294,7 @@ class Linear(torch.nn.Module):
         self._dense_plan = self._fused_plan = None
         if paths and all(u % 32 == 0 and v % 32 == 0 for (_, u, v, _, _, _, _) in paths):
             self._dense_plan = {"paths": paths, "out_size": d.operands[2].size}
-            fused = _fused_paths(paths, d.operands[1].num_segments, d.operands[2].num_segments)
+            fused = _fused_paths(paths, d.operands[1], d.operands[2])
             if fused is not None:
                 mul_ir = (int(self.transpose_in.f is not None), int(self.transpose_out.f is not None))
                 self._fused_plan = {**fused, "out_size": d.operands[2].size, "mul_ir": mul_ir}
