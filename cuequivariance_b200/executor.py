@@ -454,6 +454,9 @@ class PolynomialFunction(torch.autograd.Function):
             for i, n in enumerate(needs):
                 if n:
                     grads[i] = next(it)
+        elif any(needs):
+            # nothing arrived (a function behind this one returned None): zeros, as materialised cotangents would give
+            grads = [torch.zeros_like(x) if n else None for x, n in zip(inputs, needs)]
         return (None, None, *grads)
 
 
