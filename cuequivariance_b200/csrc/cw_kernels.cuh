@@ -267,10 +267,14 @@ struct MTerms {
       }
     }
   }
+  // MASKED: an entry with one term does not read a second one, so that an infinite or undefined component of x2 reaches only
+  // the paths that use it, as on the table-driven kernel that takes what these kernels do not.
+  template <bool MASKED>
   __device__ __forceinline__ void compute(T* M, const T* x2row, int lane) const {
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      const T m = fma(c[r][1], x2row[j[r] >> 16], c[r][0] * x2row[j[r] & 0xffffu]);
+      T m = c[r][0] * x2row[j[r] & 0xffffu];
+      if (!MASKED || c[r][1] != T(0)) m = fma(c[r][1], x2row[j[r] >> 16], m);
       if (N % 32 == 0 || r + 1 < R || lane + 32 * r < NPAD) M[lane + 32 * r] = m;
     }
   }
@@ -375,7 +379,7 @@ __global__ void __launch_bounds__(kWarps * 32, kFwdMinBlocks<T>) cw_fwd_kernel(c
         cp_async_wait<0>();
       }
       __syncwarp();
-      mt.compute(Msm, st, lane);
+      mt.template compute<MASKED>(Msm, st, lane);
       __syncwarp();
       if (active) {
         const Vec<C, T>* stage = reinterpret_cast<const Vec<C, T>*>(st + S::kX2);
@@ -481,7 +485,7 @@ __global__ void __launch_bounds__(kWarps * 32, C == 2 ? CW_MINBLOCKS : 2) cw_fwd
       if (pos + 1 < end && lane == 0)
         bulk_issue_edge<G, C, MUL_IR>(p, stages + (s ^ 1) * S::kPerStage, bars + (s ^ 1), pos + 1, c0, nch);
       mbar_wait(bars + s, (it >> 1) & 1, p.status);
-      mt.compute(Msm, st, lane);
+      mt.template compute<false>(Msm, st, lane);
       __syncwarp();
       if (active) {
         const float* xs = st + S::kX2;
@@ -597,7 +601,7 @@ __global__ void __launch_bounds__(kWarps * 32, CW_MINBLOCKS) cw_bwd_kernel(const
       }
       const int eid = cur.eid;
       __syncwarp();
-      mt.compute(Msm, st, lane);
+      mt.template compute<MASKED>(Msm, st, lane);
       __syncwarp();
       float r[16];
 #pragma unroll
@@ -715,7 +719,7 @@ __global__ void __launch_bounds__(kWarps * 32, sizeof(T) == 8 ? 2 : C == 2 ? 4 :
       }
       const int eid = cur.eid;
       __syncwarp();
-      mt.compute(Msm, st, lane);
+      mt.template compute<MASKED>(Msm, st, lane);
       __syncwarp();
       if (kBulk) {
         // the other slot is the source of the previous edge's reduction: refill it only after that has been read
