@@ -29,12 +29,16 @@ def sources() -> list[Path]:
     return sorted(CSRC.glob("*.cu")) + sorted((CSRC / "generated").glob("*.cu"))
 
 
+def headers() -> list[Path]:
+    """Everything a translation unit may include: all of it is a dependency of every object."""
+    return list(CSRC.rglob("*.cuh")) + list(CSRC.rglob("*.h")) + list((ROOT / "include").glob("*.h"))
+
+
 def _stale() -> bool:
     if not LIB.exists():
         return True
     t = LIB.stat().st_mtime
-    deps = list(CSRC.rglob("*.cu")) + list(CSRC.rglob("*.cuh")) + list((ROOT / "include").glob("*.h"))
-    return any(d.stat().st_mtime > t for d in deps)
+    return any(d.stat().st_mtime > t for d in list(CSRC.rglob("*.cu")) + headers())
 
 
 def generate() -> None:
@@ -59,9 +63,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     for src in sources():
         obj = objdir / (src.stem + ".o")
         objs.append(obj)
-        if not force and obj.exists() and obj.stat().st_mtime > max(
-            [src.stat().st_mtime] + [h.stat().st_mtime for h in list(CSRC.rglob("*.cuh")) + list((ROOT / "include").glob("*.h"))]
-        ):
+        if not force and obj.exists() and obj.stat().st_mtime > max(d.stat().st_mtime for d in [src, *headers()]):
             continue
         cmd = [nvcc, *NVCC_FLAGS, "-c", str(src), "-o", str(obj)] + (["-Xptxas", "-v"] if verbose else [])
         procs.append((src, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
