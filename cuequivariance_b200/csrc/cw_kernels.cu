@@ -149,7 +149,9 @@ extern "C" int cueq_b200_cw_backward(int g, const cueq_cw_args* a, void* stream)
 
 // All groups of a polynomial by one call: the constant part of each group's arguments comes from `templates`, which the
 // caller keeps, tensors and sizes from `call`.  Every group but the first may start before the one in front of it has
-// ended (cw_kernels.cuh, launch_kernel).
+// ended (cw_kernels.cuh, launch_kernel), unless that would leave the x2 gradient's sum in no fixed order: where one block of
+// channels holds them all, a group adds one value to a component, the first two in either order (0 + a + b), the others
+// each after the groups before.  Several blocks of channels add in no fixed order anyway.
 extern "C" int cueq_b200_cw_run(int backward, int num_groups, const int32_t* groups, const cueq_cw_args* templates, const cueq_cw_args* call,
                                 void* stream) {
   if (num_groups < 0 || (num_groups && (!groups || !templates || !call))) return cueq::fail("channelwise: null argument");
@@ -160,7 +162,9 @@ extern "C" int cueq_b200_cw_run(int backward, int num_groups, const int32_t* gro
     a.senders = call->senders; a.order = call->order; a.rowptr = call->rowptr;
     a.num_receivers = call->num_receivers; a.recv_mod = call->recv_mod; a.mean_degree = call->mean_degree;
     a.x1_mul_ir = call->x1_mul_ir; a.out_mul_ir = call->out_mul_ir;
-    if (int rc = backward ? run_backward(groups[i], &a, i > 0, stream) : run_forward(groups[i], &a, i > 0, stream)) return rc;
+    const bool one_block = a.extent <= (a.dtype == CUEQ_F32 && a.extent % 128 == 0 ? 128 : 64);
+    const int overlap = i > 0 && !(backward && a.gx2 && one_block && i > 1);
+    if (int rc = backward ? run_backward(groups[i], &a, overlap, stream) : run_forward(groups[i], &a, overlap, stream)) return rc;
   }
   return 0;
 }
