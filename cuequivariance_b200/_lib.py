@@ -182,7 +182,7 @@ class FctpTriPath(C.Structure):
 class FctpTriArgs(C.Structure):
     _fields_ = [
         ("a", C.c_void_p * 2), ("qt", C.c_void_p * 2), ("b_hi", C.c_void_p), ("b_lo", C.c_void_p), ("out", C.c_void_p),
-        ("paths", C.POINTER(FctpTriPath)), ("status", C.c_void_p),
+        ("parts", C.c_void_p), ("paths", C.POINTER(FctpTriPath)), ("status", C.c_void_p),
         ("lda", C.c_int64 * 2), ("zp", C.c_int64), ("b_rows", C.c_int64), ("ldo", C.c_int64), ("batch", C.c_int64),
         ("dtype", C.c_int32), ("channels", C.c_int32), ("out_off", C.c_int32), ("nc", C.c_int32), ("num_paths", C.c_int32),
         ("splits", C.c_int32), ("struct_bytes", C.c_int32), ("reserved", C.c_int32),

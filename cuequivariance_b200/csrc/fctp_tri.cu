@@ -47,7 +47,7 @@ struct TriParams {
   const void* a[2];
   const float* qt[2];
   float* out;
-  int64_t lda[2], zp, ldo;
+  int64_t lda[2], zp, ldo, part;   // part: distance of the partial results of two divisions of the sum
   int batch, out_off, num_paths, splits;
   int* status;
   TriPath path[kMaxPaths];
@@ -314,17 +314,12 @@ __global__ void __launch_bounds__(kThreads, 1) fctp_tri_kernel(const __grid_cons
       }
     }
     if (!dead && status_clean(p.status) && z < p.batch) {
-      float* row = p.out + (int64_t)z * p.ldo + p.out_off + rpart * K::RT + g * K::RPT;
+      float* row = p.out + blockIdx.z * p.part + (int64_t)z * p.ldo + p.out_off + rpart * K::RT + g * K::RPT;
 #pragma unroll
       for (int c = 0; c < NC; ++c)
 #pragma unroll
-        for (int j = 0; j < K::RPT; j += 4) {
-          float* dst = row + c * C + j;
-          if (p.splits > 1)
-            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"l"(dst), "f"(acc[c][j]), "f"(acc[c][j + 1]), "f"(acc[c][j + 2]), "f"(acc[c][j + 3]) : "memory");
-          else
-            *reinterpret_cast<float4*>(dst) = make_float4(acc[c][j], acc[c][j + 1], acc[c][j + 2], acc[c][j + 3]);
-        }
+        for (int j = 0; j < K::RPT; j += 4)
+          *reinterpret_cast<float4*>(row + c * C + j) = make_float4(acc[c][j], acc[c][j + 1], acc[c][j + 2], acc[c][j + 3]);
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -332,6 +327,24 @@ __global__ void __launch_bounds__(kThreads, 1) fctp_tri_kernel(const __grid_cons
   if (warp == 17) {
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(512u) : "memory");
+  }
+}
+
+// The divisions of a sum, added in their order: the result does not depend on which thread block was faster.  Bound by memory
+// (a read of every partial result); added by red.global.add into the result instead, the last bits changed from call to call.
+// A block holds 256 / cols whole rows.
+__global__ void __launch_bounds__(256) fctp_tri_sum_kernel(const float4* __restrict__ parts, float* __restrict__ out, int64_t rows, int cols, int splits,
+                                                           int64_t ldo, const int* status) {
+  const int per = blockDim.x / cols, r = threadIdx.x / cols, c = threadIdx.x - r * cols;
+  if (r >= per || !status_clean(status)) return;                      // after a wait that ran out the parts are incomplete
+  for (int64_t z = (int64_t)blockIdx.x * per + r; z < rows; z += (int64_t)gridDim.x * per) {
+    const float4* src = parts + z * cols + c;
+    float4 v = __ldcs(src);
+    for (int s = 1; s < splits; ++s) {
+      const float4 a = __ldcs(src + s * rows * cols);
+      v.x += a.x; v.y += a.y; v.z += a.z; v.w += a.w;
+    }
+    *reinterpret_cast<float4*>(out + z * ldo + 4 * c) = v;
   }
 }
 
@@ -435,12 +448,27 @@ int launch(const cueq_fctp_tri_args* a, TriParams& p, cudaStream_t st) {
   CUtensorMap hi, lo;
   if (int rc = make_map(&hi, BF16, a->b_hi, a->b_rows, C, K::NT)) return rc;
   if (int rc = make_map(&lo, BF16, BF16 ? a->b_hi : a->b_lo, a->b_rows, C, K::NT)) return rc;
+  float* const out = p.out + p.out_off;
+  const int64_t ldo = p.ldo;
+  if (p.splits > 1) {
+    if (!a->parts) return cueq::fail("fctp tri: a divided sum needs room for its partial results");
+    p.out = (float*)a->parts;
+    p.out_off = 0;
+    p.ldo = (int64_t)a->nc * C;
+    p.part = p.ldo * p.batch;
+  }
+  int rc;
   switch (a->nc) {
-    case 1: return launch_c<BF16, C, 1>(hi, lo, p, st);
-    case 3: return launch_c<BF16, C, 3>(hi, lo, p, st);
-    case 5: return launch_c<BF16, C, 5>(hi, lo, p, st);
+    case 1: rc = launch_c<BF16, C, 1>(hi, lo, p, st); break;
+    case 3: rc = launch_c<BF16, C, 3>(hi, lo, p, st); break;
+    case 5: rc = launch_c<BF16, C, 5>(hi, lo, p, st); break;
     default: return cueq::fail("fctp tri: irreps of dimension 1, 3 or 5 only");
   }
+  if (rc || p.splits == 1) return rc;
+  const int cols = (int)(p.ldo / 4), per = 256 / cols, blocks = (p.batch + per - 1) / per;
+  fctp_tri_sum_kernel<<<blocks < 148 * 16 ? blocks : 148 * 16, 256, 0, st>>>((const float4*)a->parts, out, p.batch, cols, p.splits, ldo, p.status);
+  CUEQ_CUDA_OK(cudaGetLastError());
+  return 0;
 }
 
 }  // namespace
@@ -454,7 +482,7 @@ extern "C" int cueq_b200_fctp_tri(const cueq_fctp_tri_args* a, void* stream) {
   if (!bf16 && a->dtype != CUEQ_F32) return cueq::fail("fctp tri: float32 or bf16 operands");
   if (!bf16 && !a->b_lo) return cueq::fail("fctp tri: null operand");
   const int C = a->channels, unit = bf16 ? 8 : 4;
-  if ((((uintptr_t)a->out | (uintptr_t)a->b_hi | (uintptr_t)a->b_lo | (uintptr_t)a->a[0] | (uintptr_t)a->a[1] | (uintptr_t)a->qt[0] | (uintptr_t)a->qt[1]) & 15) || a->ldo % 4 || a->out_off % 4)
+  if ((((uintptr_t)a->out | (uintptr_t)a->parts | (uintptr_t)a->b_hi | (uintptr_t)a->b_lo | (uintptr_t)a->a[0] | (uintptr_t)a->a[1] | (uintptr_t)a->qt[0] | (uintptr_t)a->qt[1]) & 15) || a->ldo % 4 || a->out_off % 4)
     return cueq::fail("fctp tri: operands and rows must be 16-byte aligned");
   TriParams p;
   std::memset(&p, 0, sizeof(p));

@@ -401,7 +401,8 @@ class DenseUVW:
                                                         None if lo is None else lo.data_ptr(), stream))
             tiles = -(-step // 128) * (c // rt)
             splits = self._tri_splits(tiles, c)
-            out = (torch.empty if full and splits == 1 else torch.zeros)((B, size), dtype=torch.float32, device=dev)
+            out = (torch.empty if full else torch.zeros)((B, size), dtype=torch.float32, device=dev)
+            parts = torch.empty(splits * step * c * max(t[1] for t in launches), dtype=torch.float32, device=dev) if splits > 1 else None
             for b0 in range(0, B, step):
                 nb = min(step, B - b0)
                 zp = -(-nb // 128) * 128
@@ -416,6 +417,7 @@ class DenseUVW:
                             _lib.check(L.cueq_b200_fctp_tri_transpose(xb.data_ptr(), dtype_code(dt), nb, x.shape[1], x.shape[1], t.data_ptr(), None, None,
                                                                       zp, stream))
                         a.qt[s] = t.data_ptr()
+                a.parts = None if parts is None else parts.data_ptr()
                         keep.append(t)
                 a.b_hi, a.b_lo, a.b_rows = hi.data_ptr(), None if lo is None else lo.data_ptr(), hi.shape[0]
                 a.status = _lib.status_word(dev).data_ptr()

@@ -340,7 +340,7 @@ int cueq_b200_gemm_f32x3_tn(const cueq_gemm_f32x3_tn_args* args, void* stream);
  * All multiplicities are `channels` (32, 64 in float32; 128 in bf16), irreps have dimension 1, 3 or 5.  P rows come
  * as they are (ir_mul), Q transposed ([column][sample], cueq_b200_fctp_tri_transpose), the weights as rows ((q, r), p)
  * (cueq_b200_fctp_tri_weights; row block k * channels^2 belongs to path k).  With splits > 1 the sum over q is divided among that
- * many thread blocks and the result (zeroed by the caller) is added to. */
+ * many thread blocks, whose partial results are added in a fixed order.  The columns of the irrep are overwritten. */
 #define CUEQ_FCTP_TRI_MAX_PATHS 24
 typedef struct {
   int32_t a_src, a_off, na;   /* P: operand 0 or 1, its first column, its components                */
@@ -354,6 +354,7 @@ typedef struct {
   const void* b_hi;     /* device [b_rows, channels]: TF32 halves (float32) or bf16                */
   const void* b_lo;
   void* out;            /* device float32 [batch, ldo]                                             */
+  void* parts;          /* splits > 1: device float32 [splits, batch, nc * channels], 16-byte aligned, overwritten */
   const cueq_fctp_tri_path* paths;   /* host                                                       */
   void* status;         /* nullable device int32: 2 if a bounded wait ran out                      */
   int64_t lda[2], zp, b_rows, ldo, batch;

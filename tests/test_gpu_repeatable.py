@@ -33,3 +33,21 @@ def test_channelwise_output_and_edge_gradients(mul, l_in, l_sh, layout):
         return [out.detach(), *torch.autograd.grad(out, [w, x2], cot)]
 
     _same(step, ("out", "gw", "gx2"))
+
+
+@pytest.mark.parametrize("mul,lmax,batch,dtype", [(32, 2, 200, "float32"), (64, 2, 300, "float32"), (64, 2, 5000, "float32"), (96, 1, 300, "float32"),
+                                                  (128, 2, 300, "bfloat16")])
+def test_fully_connected_output_and_input_gradients(mul, lmax, batch, dtype):
+    s = "+".join(f"{mul}x{ir}" for ir in LS[: lmax + 1])
+    m = cb.FullyConnectedTensorProduct(s, s, s, layout=cb.ir_mul, internal_weights=False, shared_weights=True)
+    torch.manual_seed(0)
+    dt = getattr(torch, dtype)
+    x1, x2, cot = (torch.randn(batch, m.irreps_in1.dim, device=DEV).to(dt) for _ in range(3))
+    w = torch.randn(1, m.weight_numel, device=DEV).to(dt)
+    x1.requires_grad_(True), x2.requires_grad_(True)
+
+    def step():
+        out = m(x1, x2, w)
+        return [out.detach(), *(torch.autograd.grad(out, [x1, x2], cot) if mul != 96 else ())]   # 96: gradients folded by atomics
+
+    _same(step, ("out", "gx1", "gx2"))
