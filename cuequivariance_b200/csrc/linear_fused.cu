@@ -3,7 +3,7 @@
 // primitives/segmented_polynomial_indexed_linear.py:116-156,247-339):
 //
 //   linear_map  out[z, v, i] = c * sum_u W[class(z)][u, v] x[z, u, i]       forward, and with W transposed the input gradient
-//   linear_gw   gW[class][u, v] += c * sum_{z in class, i} x[z, u, i] g[z, v, i]
+//   linear_gw   gW[class][u, v] += c * sum_{z in class, i} x[z, u, i] g[z, v, i]      partial sums, added in a fixed order
 //
 // What bounds them: the rows are read once and written once, 2 * 268 MB each for 32,768 nodes of 128x(0e+1o+2e+3o);
 // 82 us at 6.5 TB/s against 46 us of three-pass TF32.  The layer used to be one GEMM launch per irrep and component
@@ -43,6 +43,8 @@ struct LParams {
   const float* x;       // linear_map: input rows; linear_gw: x rows (M side)
   const float* w;       // linear_map: weights
   float* out;           // linear_map: output rows; linear_gw: weight gradient
+  float* parts;         // linear_gw: partial sums, one slot of `slot` floats per run
+  int64_t slot;
   const float* g;       // linear_gw: cotangent rows (N side)
   int64_t ldx, ldo, w_class_stride;
   int x_mul_ir, o_mul_ir, num_paths, num_classes;
@@ -465,7 +467,8 @@ __global__ void __launch_bounds__(kGwThreads, 1) linear_gw_kernel(const __grid_c
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
       const int m = warp * 32 + lane;
       const bool good = !dead && status_clean(p.status) && m < q.K;
-      float* dst = p.out + cls * p.w_class_stride + q.w_off + (int64_t)m * q.N;
+      // runs in order: from one to the next the thread block, the (path, class) or both move on, so their sum numbers them
+      float* dst = p.parts + (int64_t)((int)blockIdx.x + (int)(&q - p.path) * p.num_classes + cls) * p.slot + (int64_t)m * q.N;
       for (int part = 0; part < q.N / 32; ++part) {
         float v[32];
         const unsigned ta = tmem_base + ((unsigned)(warp * 32) << 16) + part * 32;
@@ -478,9 +481,7 @@ __global__ void __launch_bounds__(kGwThreads, 1) linear_gw_kernel(const __grid_c
         }
         if (good) {
 #pragma unroll
-          for (int c = 0; c < 32; c += 4)
-            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"l"(dst + part * 32 + c), "f"(v[c] * q.c), "f"(v[c + 1] * q.c),
-                         "f"(v[c + 2] * q.c), "f"(v[c + 3] * q.c) : "memory");
+          for (int c = 0; c < 32; c += 4) *reinterpret_cast<float4*>(dst + part * 32 + c) = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
         }
       }
       asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -557,6 +558,31 @@ __global__ void __launch_bounds__(kGwThreads, 1) linear_gw_kernel(const __grid_c
   tmem_free_all(tmem_base, warp, 4);
 }
 
+// The runs of one (path, class) added up in their order and put into the gradient.  Before, every run was added to the
+// gradient by red.global.add, and the last bits changed from call to call.
+// start[s]: first K block of (path, class) s = path * num_classes + class; the thread block of a K block t is the largest b
+// with total * b / blocks <= t.
+struct GwStarts { int start[kMaxPaths * kMaxClasses + 1]; };
+__global__ void __launch_bounds__(128) linear_gw_sum_kernel(const __grid_constant__ LParams p, const __grid_constant__ GwStarts t, int blocks) {
+  const int s = blockIdx.y, cls = s % p.num_classes;
+  const LPath& q = p.path[s / p.num_classes];
+  const int e = (blockIdx.x * 128 + threadIdx.x) * 4;
+  if (t.start[s] == t.start[s + 1] || e >= q.K * q.N || !status_clean(p.status)) return;
+  auto block_of = [&](int64_t item) { return (int)(((item + 1) * blocks + p.total - 1) / p.total) - 1; };
+  const int b0 = block_of(t.start[s]), n = block_of(t.start[s + 1] - 1) - b0 + 1;
+  const float* src = p.parts + (int64_t)(b0 + s) * p.slot + e;
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+  for (int k = 0; k < n; ++k) {
+    const float4 a = __ldcs(reinterpret_cast<const float4*>(src + k * p.slot));
+    v.x += a.x; v.y += a.y; v.z += a.z; v.w += a.w;
+  }
+  float4* dst = reinterpret_cast<float4*>(p.out + cls * p.w_class_stride + q.w_off + e);
+  float4 o = *dst;
+  o.x += q.c * v.x; o.y += q.c * v.y; o.z += q.c * v.z; o.w += q.c * v.w;
+  *dst = o;
+}
+
 // Checks the arguments and fills the kernel parameters; `per_item` = nodes per tile or K block.  Returns the status.
 template <class PerItem>
 int make_params(const cueq_linear_args* a, PerItem per_item, bool gw, LParams* p) {
@@ -597,7 +623,28 @@ int make_params(const cueq_linear_args* a, PerItem per_item, bool gw, LParams* p
   return 0;
 }
 
+// every run ends with 64 KB of partial sums, so short inputs use fewer blocks; long ones are cut so that an accumulation
+// chain does not grow with the number of rows
+int gw_blocks(const LParams& p) {
+  int grid = (p.total + 7) / 8;
+  grid = grid < 148 ? grid : 148;
+  const int most = (p.total + kMaxRunGw - 1) / kMaxRunGw;
+  return grid < most ? most : grid;
+}
+int64_t gw_slot(const LParams& p) {
+  int64_t slot = 0;
+  for (int k = 0; k < p.num_paths; ++k) slot = (int64_t)p.path[k].K * p.path[k].N > slot ? (int64_t)p.path[k].K * p.path[k].N : slot;
+  return slot;
+}
+int64_t gw_floats(const LParams& p, int grid) { return (int64_t)(grid + p.num_paths * p.num_classes) * gw_slot(p); }
+
 }  // namespace
+
+extern "C" int64_t cueq_b200_linear_gw_floats(const cueq_linear_args* a) {
+  LParams p;
+  if (make_params(a, rows_per_block, true, &p)) return -1;
+  return p.total == 0 ? 0 : gw_floats(p, gw_blocks(p));
+}
 
 extern "C" int cueq_b200_linear_map(const cueq_linear_args* a, void* stream) {
   LParams p;
@@ -621,18 +668,31 @@ extern "C" int cueq_b200_linear_gw(const cueq_linear_args* a, void* stream) {
   p.g = (const float*)a->w;
   p.out = (float*)a->out;
   if (p.total == 0) return 0;
-  // every run ends with a 64 KB reduction into the gradient, so short inputs use fewer blocks; long ones are cut so
-  // that an accumulation chain does not grow with the number of rows
-  int grid = (p.total + 7) / 8;
-  grid = grid < 148 ? grid : 148;
-  const int most = (p.total + kMaxRunGw - 1) / kMaxRunGw;
-  if (grid < most) grid = most;
+  const int grid = gw_blocks(p);
+  const int64_t need = gw_floats(p, grid);
+  if (!a->parts || a->parts_floats < need || ((uintptr_t)a->parts & 15))
+    return cueq::fail("linear: the weight gradient needs room for %lld floats of partial sums, 16-byte aligned", (long long)need);
+  p.parts = (float*)a->parts;
+  p.slot = gw_slot(p);
+  GwStarts t;
+  int widest = 0;
+  for (int k = 0, s = 0, at = 0; k < p.num_paths; ++k) {
+    widest = p.path[k].K * p.path[k].N > widest ? p.path[k].K * p.path[k].N : widest;
+    const int n = rows_per_block(p.path[k].d);
+    for (int c = 0; c < p.num_classes; ++c, ++s) {
+      t.start[s] = at;
+      at += (p.bounds[c + 1] - p.bounds[c] + n - 1) / n;
+      t.start[s + 1] = at;
+    }
+  }
   static cueq::PerDeviceFlag configured;
   if (!configured.get()) {
     CUEQ_CUDA_OK(cudaFuncSetAttribute(linear_gw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGwSmem));
     configured.set();
   }
   linear_gw_kernel<<<grid, kGwThreads, kGwSmem, reinterpret_cast<cudaStream_t>(stream)>>>(p);
+  CUEQ_CUDA_OK(cudaGetLastError());
+  linear_gw_sum_kernel<<<dim3((widest / 4 + 127) / 128, p.num_paths * p.num_classes), 128, 0, reinterpret_cast<cudaStream_t>(stream)>>>(p, t, grid);
   CUEQ_CUDA_OK(cudaGetLastError());
   return 0;
 }

@@ -192,7 +192,13 @@ class _FusedLinear(torch.autograd.Function):
         a.w_class_stride = (w if which == "map" else out).shape[1]
         for q, (wo, u, v, xo, oo, d, c) in zip(a.paths, plan["paths"]):
             q.u, q.v, q.d, q.x_off, q.out_off, q.w_off, q.c = u, v, d, xo, oo, wo, c
-        fn = _lib.lib().cueq_b200_linear_map if which == "map" else _lib.lib().cueq_b200_linear_gw
+        L = _lib.lib()
+        fn = L.cueq_b200_linear_map if which == "map" else L.cueq_b200_linear_gw
+        parts = None
+        if which == "gw":
+            n = L.cueq_b200_linear_gw_floats(C.byref(a))
+            parts = torch.empty(max(n, 0), dtype=torch.float32, device=x.device)
+            a.parts, a.parts_floats = parts.data_ptr(), n
         name = ("linear" if len(bounds) == 2 else "indexed_linear") + "_f32x3" + ("_gx" if transposed else "" if which == "map" else "_gw")
         with torch.cuda.device(x.device), profiling.kernel(name):
             _lib.check(fn(C.byref(a), C.c_void_p(torch.cuda.current_stream(x.device).cuda_stream)))

@@ -401,7 +401,8 @@ int cueq_b200_fctp_gw(const cueq_fctp_gw_args* args, void* stream);
  * weights at w + k * w_class_stride.
  * linear_map: out[z, v, i] = c * sum_u W[u, v] x[z, u, i]; with `transposed` the input gradient: `x` holds the cotangent
  *   rows (addressed by out_off), `out` the gradient rows (addressed by x_off).
- * linear_gw:  out (the weight gradient, zeroed by the caller) [u, v] += c * sum_{z, i} x[z, u, i] g[z, v, i]; `w` = g. */
+ * linear_gw:  out (the weight gradient, zeroed by the caller) [u, v] += c * sum_{z, i} x[z, u, i] g[z, v, i]; `w` = g.  The
+ *   partial sums of its thread blocks go to `parts` (cueq_b200_linear_gw_floats(args) floats) and are added in a fixed order. */
 #define CUEQ_LINEAR_MAX_PATHS 8
 #define CUEQ_LINEAR_MAX_CLASSES 64
 typedef struct {
@@ -426,7 +427,11 @@ int cueq_b200_linear_map(const cueq_linear_args* args, void* stream);
 int cueq_b200_linear_gw(const cueq_linear_args* args, void* stream);
 
 /* ---- fully connected ("uvw") tensor product: kernels around the tensor-core GEMM -----------------
+  void* parts;          /* linear_gw: device float32, 16-byte aligned, overwritten                 */
+  int64_t parts_floats; /* its size                                                                */
  *
+/* floats that linear_gw needs in `parts` for these shapes (pointers other than null, not read); -1: invalid arguments */
+int64_t cueq_b200_linear_gw_floats(const cueq_linear_args* args);
  * For one path of uvw,iu,jv,kw+ijk (cue.descriptors.fully_connected_tensor_product,
  * cuequivariance/group_theory/descriptors/irreps_tp.py:22-91; module forward at
  * cuequivariance_torch/operations/tp_fully_connected.py:166-207) with coupling tensor cg[i][j][k]

@@ -51,3 +51,20 @@ def test_fully_connected_output_and_input_gradients(mul, lmax, batch, dtype):
         return [out.detach(), *(torch.autograd.grad(out, [x1, x2], cot) if mul != 96 else ())]   # 96: gradients folded by atomics
 
     _same(step, ("out", "gx1", "gx2"))
+
+
+@pytest.mark.parametrize("mul,lmax,rows,classes", [(128, 3, 2000, 1), (128, 3, 20011, 1), (32, 1, 300, 1), (64, 2, 1500, 10), (32, 0, 256, 64)])
+def test_linear_with_gradients(mul, lmax, rows, classes):
+    s = "+".join(f"{mul}x{ir}" for ir in LS[: lmax + 1])
+    m = cb.Linear(s, s, layout=cb.mul_ir, internal_weights=False, shared_weights=True, weight_classes=classes)
+    torch.manual_seed(0)
+    x, cot = (torch.randn(rows, m.irreps_in.dim, device=DEV) for _ in range(2))
+    w = torch.randn(classes, m.weight_numel, device=DEV, requires_grad=True)
+    x.requires_grad_(True)
+    idx = torch.sort(torch.randint(0, classes, (rows,), device=DEV)).values if classes > 1 else None
+
+    def step():
+        out = m(x, w, idx)
+        return [out.detach(), *torch.autograd.grad(out, [w, x], cot)]
+
+    _same(step, ("out", "gw", "gx"))
