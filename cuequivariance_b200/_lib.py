@@ -201,6 +201,7 @@ class FctpGwArgs(C.Structure):
         ("t", C.c_void_p), ("t_hi", C.c_void_p), ("t_lo", C.c_void_p), ("gw", C.c_void_p), ("paths", C.POINTER(FctpGwPath)),
         ("status", C.c_void_p), ("rows", C.c_int64), ("zp", C.c_int64), ("batch", C.c_int64),
         ("channels", C.c_int32), ("num_paths", C.c_int32), ("struct_bytes", C.c_int32), ("reserved", C.c_int32),
+        ("parts", C.c_void_p), ("parts_floats", C.c_int64),
     ]
 
 
@@ -221,8 +222,8 @@ class LinearArgs(C.Structure):
         ("bounds", C.POINTER(C.c_int32)), ("status", C.c_void_p),
         ("num_paths", C.c_int32), ("num_classes", C.c_int32), ("x_mul_ir", C.c_int32), ("out_mul_ir", C.c_int32),
         ("transposed", C.c_int32), ("struct_bytes", C.c_int32), ("paths", LinearPath * LINEAR_MAX_PATHS),
-    ]
         ("parts", C.c_void_p), ("parts_floats", C.c_int64),
+    ]
 
 
 class GemmF32x3TnArgs(C.Structure):
@@ -309,13 +310,15 @@ def lib() -> C.CDLL:
     L.cueq_b200_fctp_tri_transpose.argtypes = [C.c_void_p, C.c_int, C.c_int64, C.c_int32, C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p,
                                                C.c_int64, C.c_void_p]
     L.cueq_b200_fctp_gw.argtypes = [C.POINTER(FctpGwArgs), C.c_void_p]
+    L.cueq_b200_fctp_gw_floats.argtypes = [C.POINTER(FctpGwArgs)]
+    L.cueq_b200_fctp_gw_floats.restype = C.c_int64
     L.cueq_b200_linear_map.argtypes = [C.POINTER(LinearArgs), C.c_void_p]
     L.cueq_b200_linear_gw.argtypes = [C.POINTER(LinearArgs), C.c_void_p]
+    L.cueq_b200_linear_gw_floats.argtypes = [C.POINTER(LinearArgs)]
+    L.cueq_b200_linear_gw_floats.restype = C.c_int64
     L.cueq_b200_selftest_bounded_wait.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p]
     if L.cueq_b200_abi_version() != 1:
         raise CueqError("libcueq_b200.so has an unexpected ABI version; rebuild it")
-    L.cueq_b200_linear_gw_floats.argtypes = [C.POINTER(LinearArgs)]
-    L.cueq_b200_linear_gw_floats.restype = C.c_int64
     L.cueq_b200_sizeof.restype = C.c_int64
     for which, struct in enumerate((U1dDesc, Buffer, CwArgs, CwNoAllocArgs, GemmArgs, FctpArgs, FctpFusedArgs, FctpFusedTask, FctpFusedGxArgs, FctpFusedUnit, FctpFusedGwArgs, FctpFusedWUnit, GemmF32x3Args, GemmF32x3TnArgs)):
         if L.cueq_b200_sizeof(which) != C.sizeof(struct):

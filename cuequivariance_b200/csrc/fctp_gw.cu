@@ -11,8 +11,9 @@
 // arrive split by TMA.  The coupled operand used to be written to memory per path and component of the output and read back
 // by a row-reduction GEMM that transposed it: 3.5 + 8.0 ms for 32,768 samples of 64x(0e+1o+2e).
 //
-// A thread block owns one path, a range of x (all of TMEM: 512 columns of accumulators) and a range of samples, and adds its
-// result to the gradient.  hi*hi and the small terms have accumulators of their own, and the range of samples is cut so that
+// A thread block owns one path, a range of x (all of TMEM: 512 columns of accumulators) and a range of samples.  Its result is
+// added to the gradient, with more than kOrdered K blocks by red.global.add, in no fixed order; up to there through partial
+// sums that a second kernel adds in their order.  hi*hi and the small terms have accumulators of their own, and the range of samples is cut so that
 // a chain stays short (see `launch`).
 // What bounds it: shared memory.  Per tile the MMAs read 56 KB (hi of the tile against both halves of T in one instruction),
 // the builders 40 KB of S for two rows per thread and write 32 KB.  32,768 samples of 64x(0e+1o+2e): 4.3 ms.
@@ -31,11 +32,16 @@ constexpr int kMaxPaths = CUEQ_FCTP_TRI_MAX_PATHS;
 constexpr int kBuilders = 512;                         // warps 0-15
 constexpr int kThreads = kBuilders + 64;               // 16: TMA, 17: MMA issue and TMEM owner
 constexpr int kBlk = 128 * 128;                        // 128 rows x 32 float32
+// 2,048 samples.  The row-reduction GEMM before had one thread block per weight tile up to there, so that its result repeated
+// bit for bit; partial sums for all samples of a large batch would be 50 to 250 copies of the weights.
+constexpr int kOrdered = 64;
 
 // item0: first thread block of the path; chunk: K blocks (32 samples) per thread block; mask: bit 5 * e + b
-struct GwPath { int x_row, na, y_row, nb, t_row, ne, w_off, sx, sy, st, item0, chunk, mask; float coef[5][5][5]; };   // [e][a][b]
+// slot0: first partial sum of the path
+struct GwPath { int x_row, na, y_row, nb, t_row, ne, w_off, sx, sy, st, item0, chunk, mask, slot0; float coef[5][5][5]; };   // [e][a][b]
 struct GwParams {
   float* gw;
+  float* parts;             // partial sums of channels^3 floats each, or null
   int* status;
   int nblocks, num_paths;   // K blocks of all samples
   GwPath path[kMaxPaths];
@@ -237,7 +243,7 @@ __global__ void __launch_bounds__(kThreads, 1) fctp_gw_kernel(const __grid_const
     const int row = (warp & 3) * 32 + lane;                            // TMEM lane quadrant = warp % 4
     for (int m = warp >> 2; m < K::TPC; m += 4) {
       const int x = x0 + m * K::XP + row / C, yy = row % C;
-      float* dst = p.gw + t.w_off + (int64_t)x * t.sx + (int64_t)yy * t.sy;
+      float* dst = (p.parts ? p.parts + (int64_t)(t.slot0 + b0 / t.chunk) * (C * C * C) : p.gw + t.w_off) + (int64_t)x * t.sx + (int64_t)yy * t.sy;
       const unsigned col = tmem_base + ((unsigned)((warp & 3) * 32) << 16) + m * 2 * C;
       for (int c = 0; c < C; c += 8) {
         unsigned h[8], l[8];
@@ -250,7 +256,10 @@ __global__ void __launch_bounds__(kThreads, 1) fctp_gw_kernel(const __grid_const
           float v[8];
 #pragma unroll
           for (int q = 0; q < 8; ++q) v[q] = __uint_as_float(h[q]) + __uint_as_float(l[q]);
-          if (t.st == 1) {
+          if (p.parts) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) dst[(int64_t)(c + q) * t.st] = v[q];
+          } else if (t.st == 1) {
 #pragma unroll
             for (int q = 0; q < 8; q += 4)
               asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"l"(dst + c + q), "f"(v[q]), "f"(v[q + 1]), "f"(v[q + 2]), "f"(v[q + 3]) : "memory");
@@ -270,6 +279,21 @@ __global__ void __launch_bounds__(kThreads, 1) fctp_gw_kernel(const __grid_const
   }
 }
 
+// The partial sums of a path in their order, into the gradient (paths may share weights).
+__global__ void __launch_bounds__(256) fctp_gw_sum_kernel(const __grid_constant__ GwParams p, int size) {
+  const GwPath& t = p.path[blockIdx.y];
+  const int e = (blockIdx.x * 256 + threadIdx.x) * 4, n = (p.nblocks + t.chunk - 1) / t.chunk;
+  if (e >= size || !status_clean(p.status)) return;
+  const float* src = p.parts + (int64_t)t.slot0 * size + e;
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+  for (int k = 0; k < n; ++k) {
+    const float4 a = __ldcs(reinterpret_cast<const float4*>(src + (int64_t)k * size));
+    v.x += a.x; v.y += a.y; v.z += a.z; v.w += a.w;
+  }
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"l"(p.gw + t.w_off + e), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+}
+
 int make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t zp, int box_rows, bool swizzle) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return cueq::fail("fctp gw: cuTensorMapEncodeTiled is not available from the driver");
@@ -283,18 +307,25 @@ int make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t zp, int b
   return 0;
 }
 
+// K blocks per thread block: a chain has 4 additions at full magnitude per block and component.  80 keep the error below that
+// of the GEMM before (chains of up to 192), which had shorter ones where there are few samples: 12 per four blocks.
+int chunk_of(int nblocks, int ne) {
+  const int chain = nblocks * 3 < 80 ? nblocks * 3 : 80;
+  return chain / (4 * ne) > 1 ? chain / (4 * ne) : 1;
+}
+
 template <int C>
 int launch(const cueq_fctp_gw_args* a, GwParams& p, cudaStream_t st) {
   using K = Cfg<C>;
-  int64_t items = 0;
+  int64_t items = 0, slots = 0;
   for (int k = 0; k < p.num_paths; ++k) {
     GwPath& t = p.path[k];
     t.item0 = (int)items;
-    // a chain has 4 additions at full magnitude per block and component.  80 keep the error below that of the GEMM before
-    // (chains of up to 192), which had shorter ones where there are few samples: 12 per four blocks.
-    const int chain = p.nblocks * 3 < 80 ? p.nblocks * 3 : 80;
-    t.chunk = chain / (4 * t.ne) > 1 ? chain / (4 * t.ne) : 1;
-    items += (int64_t)(C / K::XR) * ((p.nblocks + t.chunk - 1) / t.chunk);
+    t.slot0 = (int)slots;
+    t.chunk = chunk_of(p.nblocks, t.ne);
+    const int64_t chunks = (p.nblocks + t.chunk - 1) / t.chunk;
+    items += (C / K::XR) * chunks;
+    slots += chunks;
   }
   if (items > 2147483647LL) return cueq::fail("fctp gw: too many samples");
   CUtensorMap mx, my, mh, ml;
@@ -309,17 +340,34 @@ int launch(const cueq_fctp_gw_args* a, GwParams& p, cudaStream_t st) {
   }
   fctp_gw_kernel<C><<<(unsigned)items, kThreads, K::smem, st>>>(mx, my, mh, ml, p);
   CUEQ_CUDA_OK(cudaGetLastError());
+  if (p.parts) {
+    fctp_gw_sum_kernel<<<dim3((C * C * C / 4 + 255) / 256, p.num_paths), 256, 0, st>>>(p, C * C * C);
+    CUEQ_CUDA_OK(cudaGetLastError());
+  }
   return 0;
 }
 
 }  // namespace
+
+extern "C" int64_t cueq_b200_fctp_gw_floats(const cueq_fctp_gw_args* a) {
+  if (!a || !a->paths || a->struct_bytes != (int)sizeof(cueq_fctp_gw_args) || a->batch < 0 || a->num_paths < 1 || a->num_paths > kMaxPaths || a->channels < 1) return -1;
+  const int64_t nblocks = (a->batch + 31) / 32;
+  if (nblocks > kOrdered || nblocks == 0) return 0;
+  int64_t slots = 0;
+  for (int k = 0; k < a->num_paths; ++k) {
+    if (a->paths[k].ne < 1) return -1;
+    const int chunk = chunk_of((int)nblocks, a->paths[k].ne);
+    slots += (nblocks + chunk - 1) / chunk;
+  }
+  return slots * a->channels * a->channels * a->channels;
+}
 
 extern "C" int cueq_b200_fctp_gw(const cueq_fctp_gw_args* a, void* stream) {
   if (!a || !a->t || !a->t_hi || !a->t_lo || !a->gw || !a->paths) return cueq::fail("fctp gw: null operand");
   if (a->struct_bytes != (int)sizeof(cueq_fctp_gw_args)) return cueq::fail("fctp gw: the binding declares another argument block");
   if (a->num_paths < 1 || a->num_paths > kMaxPaths) return cueq::fail("fctp gw: between 1 and %d paths", kMaxPaths);
   if (a->zp % 128 || a->batch < 0 || a->batch > a->zp || a->zp > 2147483647LL) return cueq::fail("fctp gw: invalid batch or pitch");
-  if (((uintptr_t)a->t | (uintptr_t)a->t_hi | (uintptr_t)a->t_lo | (uintptr_t)a->gw) & 15) return cueq::fail("fctp gw: operands must be 16-byte aligned");
+  if (((uintptr_t)a->t | (uintptr_t)a->t_hi | (uintptr_t)a->t_lo | (uintptr_t)a->gw | (uintptr_t)a->parts) & 15) return cueq::fail("fctp gw: operands must be 16-byte aligned");
   const int C = a->channels;
   if (C != 32 && C != 64 && C != 96) return cueq::fail("fctp gw: %d channels are not covered", C);
   GwParams p;
@@ -349,6 +397,9 @@ extern "C" int cueq_b200_fctp_gw(const cueq_fctp_gw_args* a, void* stream) {
         }
   }
   if (a->batch == 0) return 0;
+  const int64_t need = cueq_b200_fctp_gw_floats(a);
+  if (need > 0 && (!a->parts || a->parts_floats < need)) return cueq::fail("fctp gw: needs room for %lld floats of partial sums", (long long)need);
+  p.parts = need > 0 ? (float*)a->parts : nullptr;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   return C == 32 ? launch<32>(a, p, st) : C == 64 ? launch<64>(a, p, st) : launch<96>(a, p, st);
 }

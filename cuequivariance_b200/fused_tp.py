@@ -473,6 +473,9 @@ class DenseUVW:
                                                                   t[1, r].data_ptr(), t[2, r].data_ptr(), zp, stream))
                 a = _lib.FctpGwArgs()
                 a.t, a.t_hi, a.t_lo, a.gw = t[0].data_ptr(), t[1].data_ptr(), t[2].data_ptr(), gw.data_ptr()
+                room = L.cueq_b200_fctp_gw_floats(C.byref(a))
+                parts = torch.empty(max(room, 0), dtype=torch.float32, device=dev)
+                a.parts, a.parts_floats = parts.data_ptr(), room
                 a.paths = C.cast(paths, C.POINTER(_lib.FctpGwPath))
                 a.status = _lib.status_word(dev).data_ptr()
                 a.rows, a.zp, a.batch = rows, zp, nb

@@ -373,7 +373,8 @@ int cueq_b200_fctp_tri_transpose(const void* x, int dtype, int64_t batch, int32_
 /* The weight gradient of the same product, float32: gw[x, y, t] += sum over samples, a, b, e of
  *   coef[e][a][b] X[z, a, x] Y[z, b, y] T[z, e, t],   x, y, t = the axes u, v, w in the order given per path.
  * All operands transposed and stacked: row = column of x1, x2 or the cotangent; sums run over K blocks of 32 samples, so the
- * columns batch..zp of `t`, `t_hi`, `t_lo` hold zeros.  gw is zeroed by the caller. */
+ * columns batch..zp of `t`, `t_hi`, `t_lo` hold zeros.  gw is zeroed by the caller.  For small batches (up to 2,048 samples)
+ * partial sums go to `parts` and are added in a fixed order; beyond, the order is left to the thread blocks. */
 typedef struct {
   int32_t x_row, na, y_row, nb, t_row, ne;   /* first stacked row and components of X, Y, T        */
   int32_t w_off;              /* first weight of the path                                          */
@@ -391,7 +392,11 @@ typedef struct {
   int32_t channels, num_paths;
   int32_t struct_bytes; /* sizeof(cueq_fctp_gw_args) as the caller declares it                     */
   int32_t reserved;
+  void* parts;          /* device float32, 16-byte aligned, overwritten; null where no room is needed */
+  int64_t parts_floats; /* its size                                                                */
 } cueq_fctp_gw_args;
+/* floats that fctp_gw needs in `parts` for this batch (pointers other than `paths` are not read); -1: invalid arguments */
+int64_t cueq_b200_fctp_gw_floats(const cueq_fctp_gw_args* args);
 int cueq_b200_fctp_gw(const cueq_fctp_gw_args* args, void* stream);
 
 /* Equivariant linear layer, all irreps and weight classes in one launch, in the accuracy of the GEMMs above
@@ -422,16 +427,16 @@ typedef struct {
   int32_t transposed;
   int32_t struct_bytes; /* sizeof(cueq_linear_args) as the caller declares it                      */
   cueq_linear_path paths[CUEQ_LINEAR_MAX_PATHS];
+  void* parts;          /* linear_gw: device float32, 16-byte aligned, overwritten                 */
+  int64_t parts_floats; /* its size                                                                */
 } cueq_linear_args;
+/* floats that linear_gw needs in `parts` for these shapes (pointers other than null, not read); -1: invalid arguments */
+int64_t cueq_b200_linear_gw_floats(const cueq_linear_args* args);
 int cueq_b200_linear_map(const cueq_linear_args* args, void* stream);
 int cueq_b200_linear_gw(const cueq_linear_args* args, void* stream);
 
 /* ---- fully connected ("uvw") tensor product: kernels around the tensor-core GEMM -----------------
-  void* parts;          /* linear_gw: device float32, 16-byte aligned, overwritten                 */
-  int64_t parts_floats; /* its size                                                                */
  *
-/* floats that linear_gw needs in `parts` for these shapes (pointers other than null, not read); -1: invalid arguments */
-int64_t cueq_b200_linear_gw_floats(const cueq_linear_args* args);
  * For one path of uvw,iu,jv,kw+ijk (cue.descriptors.fully_connected_tensor_product,
  * cuequivariance/group_theory/descriptors/irreps_tp.py:22-91; module forward at
  * cuequivariance_torch/operations/tp_fully_connected.py:166-207) with coupling tensor cg[i][j][k]

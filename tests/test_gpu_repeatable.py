@@ -68,3 +68,14 @@ def test_linear_with_gradients(mul, lmax, rows, classes):
         return [out.detach(), *torch.autograd.grad(out, [w, x], cot)]
 
     _same(step, ("out", "gw", "gx"))
+
+
+@pytest.mark.parametrize("mul,lmax,batch", [(32, 2, 200), (32, 2, 2048), (64, 2, 300), (64, 1, 2047), (96, 1, 500)])
+def test_fully_connected_weight_gradient_of_small_batches(mul, lmax, batch):
+    s = "+".join(f"{mul}x{ir}" for ir in LS[: lmax + 1])
+    m = cb.FullyConnectedTensorProduct(s, s, s, layout=cb.ir_mul, internal_weights=False, shared_weights=True)
+    torch.manual_seed(0)
+    x1, x2, cot = (torch.randn(batch, m.irreps_in1.dim, device=DEV) for _ in range(3))
+    w = torch.randn(1, m.weight_numel, device=DEV, requires_grad=True)
+    out = m(x1, x2, w)
+    _same(lambda: torch.autograd.grad(out, [w], cot, retain_graph=True), ("gw",))
