@@ -154,9 +154,10 @@ class _TensorCoreUVW(torch.autograd.Function):
             ctx.save_for_backward(w, x1, x2)
             return out.to(x1.dtype)
         if FUSED and owner._fused_tasks() is not None:
-            out = owner._fused_forward(w, x1, x2, status)
+            w16 = owner._weights_bf16(w, False)
+            out = owner._fused_forward(w16, x1, x2, status)
             ctx.owner, ctx.status = owner, status
-            ctx.save_for_backward(w, x1, x2)
+            ctx.save_for_backward(w, x1, x2, w16)
             return out.to(x1.dtype)
         x1c, x2c = owner._as_kernel_input(x1), owner._as_kernel_input(x2)
         out = torch.zeros((B, owner.out_size), dtype=torch.float32, device=dev)
@@ -185,7 +186,7 @@ class _TensorCoreUVW(torch.autograd.Function):
         from . import profiling
 
         owner = ctx.owner
-        w, x1, x2 = ctx.saved_tensors
+        w, x1, x2, *w16 = ctx.saved_tensors
         d, off = owner.d, owner.offsets
         B, dev = x1.shape[0], x1.device
         need_w, need_x1, need_x2 = ctx.needs_input_grad[1], ctx.needs_input_grad[2], ctx.needs_input_grad[3]
@@ -206,9 +207,10 @@ class _TensorCoreUVW(torch.autograd.Function):
                 gwf = owner._fused_gw(w, x1b, x2b, gout16, status)
                 need_w = False
             if need_x1:
-                gx1f = owner._fused_gx(1, owner._weights_bf16(w, False), x2b, gout16, status)
+                gx1f = owner._fused_gx(1, w16, x2b, gout16, status)
+            w16 = w16[0] if w16 else owner._weights_bf16(w, False)
             if need_x2:
-                gx2f = owner._fused_gx(2, owner._weights_bf16(w, True), x1b, gout16, status)
+                gx2f = owner._fused_gx(2, owner._weights_bf16(w16, True), x1b, gout16, status)
             need_x1 = need_x2 = False
         x1c, x2c = owner._as_kernel_input(x1), owner._as_kernel_input(x2)
         gw = torch.zeros((1, w.shape[1]), dtype=torch.float32, device=dev) if need_w else None
@@ -266,23 +268,15 @@ class DenseUVW:
         self.offsets = [op.offsets() for op in d.operands]
         self.out_size = d.operands[3].size
         self._flat = {}
-        self._wcache = {}
         self._tri_mul = None
 
-    def _weights_bf16(self, w: torch.Tensor, transposed: bool) -> torch.Tensor:
-        """The shared weights as bf16 rows of 64, in ``[u][v][w]`` order or (``transposed``) ``[v][u][w]``.  The same
-        weight tensor is used by every call of a step and changes only when the optimizer updates it, so the
-        converted copies are kept until the tensor's version counter moves (or another tensor is passed)."""
-        key = (w.data_ptr(), w._version, tuple(w.shape), w.dtype, transposed)
-        hit = self._wcache.get(transposed)
-        if hit is not None and hit[0] == key:
-            return hit[1]
-        if transposed:
-            t = w.detach().reshape(-1, 64, 64, 64).transpose(1, 2).reshape(-1, 64).to(torch.bfloat16).contiguous()
-        else:
-            t = w.detach().reshape(-1, 64).to(torch.bfloat16).contiguous()
-        self._wcache[transposed] = (key, t)
-        return t
+    @staticmethod
+    def _weights_bf16(w: torch.Tensor, transposed: bool) -> torch.Tensor:
+        """The shared weights as bf16 rows of 64, in ``[u][v][w]`` order or (``transposed``) ``[v][u][w]``.  Made once per pass
+        (the backward pass gets the forward's copy): neither an address nor a version counter tells that the values are
+        still those of an earlier call."""
+        t = w.detach().to(torch.bfloat16).reshape(-1, 64, 64, 64)
+        return (t.transpose(1, 2) if transposed else t).reshape(-1, 64).contiguous()
 
     # -- tensor-core route ---------------------------------------------------------------------
     def _tc_applicable(self, w, x1, x2) -> bool:
@@ -609,7 +603,7 @@ class DenseUVW:
             _lib.check(_lib.lib().cueq_b200_fctp_fused_gw(C.byref(a), C.c_void_p(torch.cuda.current_stream().cuda_stream)))
         return gw.reshape(1, -1)
 
-    def _fused_forward(self, w, x1, x2, status):
+    def _fused_forward(self, w16, x1, x2, status):
         import ctypes as C
 
         from . import profiling
@@ -617,7 +611,6 @@ class DenseUVW:
         tasks = self._fused_tasks()
         B = x1.shape[0]
         x1c, x2c = x1.to(torch.bfloat16).contiguous(), x2.to(torch.bfloat16).contiguous()
-        w16 = self._weights_bf16(w, False)
         out = torch.empty((B, self.out_size), dtype=torch.float32, device=x1.device)
         a = _lib.FctpFusedArgs()
         a.x1, a.x2, a.w, a.out = x1c.data_ptr(), x2c.data_ptr(), w16.data_ptr(), out.data_ptr()
