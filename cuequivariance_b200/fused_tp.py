@@ -206,9 +206,9 @@ class _TensorCoreUVW(torch.autograd.Function):
             if need_w and FUSED_GW:
                 gwf = owner._fused_gw(w, x1b, x2b, gout16, status)
                 need_w = False
+            w16 = w16[0] if w16 else owner._weights_bf16(w, False)
             if need_x1:
                 gx1f = owner._fused_gx(1, w16, x2b, gout16, status)
-            w16 = w16[0] if w16 else owner._weights_bf16(w, False)
             if need_x2:
                 gx2f = owner._fused_gx(2, owner._weights_bf16(w16, True), x1b, gout16, status)
             need_x1 = need_x2 = False
@@ -411,11 +411,11 @@ class DenseUVW:
                             _lib.check(L.cueq_b200_fctp_tri_transpose(xb.data_ptr(), dtype_code(dt), nb, x.shape[1], x.shape[1], t.data_ptr(), None, None,
                                                                       zp, stream))
                         a.qt[s] = t.data_ptr()
-                a.parts = None if parts is None else parts.data_ptr()
                         keep.append(t)
                 a.b_hi, a.b_lo, a.b_rows = hi.data_ptr(), None if lo is None else lo.data_ptr(), hi.shape[0]
                 a.status = _lib.status_word(dev).data_ptr()
                 a.out, a.ldo, a.zp, a.batch = out[b0].data_ptr(), size, zp, nb
+                a.parts = None if parts is None else parts.data_ptr()
                 a.dtype, a.channels, a.splits, a.struct_bytes = dtype_code(dt), c, splits, C.sizeof(a)
                 for o, nc, paths, np_ in launches:
                     a.out_off, a.nc, a.num_paths = o, nc, np_
@@ -467,13 +467,13 @@ class DenseUVW:
                                                                   t[1, r].data_ptr(), t[2, r].data_ptr(), zp, stream))
                 a = _lib.FctpGwArgs()
                 a.t, a.t_hi, a.t_lo, a.gw = t[0].data_ptr(), t[1].data_ptr(), t[2].data_ptr(), gw.data_ptr()
-                room = L.cueq_b200_fctp_gw_floats(C.byref(a))
-                parts = torch.empty(max(room, 0), dtype=torch.float32, device=dev)
-                a.parts, a.parts_floats = parts.data_ptr(), room
                 a.paths = C.cast(paths, C.POINTER(_lib.FctpGwPath))
                 a.status = _lib.status_word(dev).data_ptr()
                 a.rows, a.zp, a.batch = rows, zp, nb
                 a.channels, a.num_paths, a.struct_bytes = self._gw_channels(), len(self.d.paths), C.sizeof(a)
+                room = L.cueq_b200_fctp_gw_floats(C.byref(a))
+                parts = torch.empty(max(room, 0), dtype=torch.float32, device=dev)
+                a.parts, a.parts_floats = parts.data_ptr(), room
                 with profiling.kernel(name):
                     _lib.check(L.cueq_b200_fctp_gw(C.byref(a), stream))
         return gw
