@@ -795,19 +795,21 @@ class DenseUVW:
             gw[0, off[0][sw] : off[0][sw] + U * V * Wd] = acc[: U * V, :Wd].reshape(-1)
         return gw
 
-    def map_x(self, w, x1, x2, g):
-        """(dPhi/dx1, dPhi/dx2): per path gZ = g W^T by one GEMM per component, folded against the other operand."""
+    def map_x(self, w, x1, x2, g, need=(True, True)):
+        """(dPhi/dx1, dPhi/dx2), None for one that is not needed: per path gZ = g W^T by one GEMM per component, folded
+        against the other operand."""
         import ctypes as C
 
         from . import profiling
         from .dense import gemm_f32x3, split_tf32
 
         if self._tri_channels(torch.float32) and x1.shape[0]:
-            return self.tri_map(0, w, (x2, g), "fctp_f32_gx"), self.tri_map(1, w, (x1, g), "fctp_f32_gx")
+            return (self.tri_map(0, w, (x2, g), "fctp_f32_gx") if need[0] else None,
+                    self.tri_map(1, w, (x1, g), "fctp_f32_gx") if need[1] else None)
         d, off = self.d, self.offsets
         B, dev = x1.shape[0], x1.device
-        gx1 = torch.zeros(x1.shape, dtype=torch.float32, device=dev)
-        gx2 = torch.zeros(x2.shape, dtype=torch.float32, device=dev)
+        gx1 = torch.zeros(x1.shape, dtype=torch.float32, device=dev) if need[0] else None
+        gx2 = torch.zeros(x2.shape, dtype=torch.float32, device=dev) if need[1] else None
         for k, p in enumerate(d.paths):
             sw, _, _, so = p.indices
             U, V, Wd = d.operands[0].segments[sw]
@@ -832,7 +834,7 @@ class DenseUVW:
                     gemm_f32x3(gk, Wk, name="fctp_f32_gx", out=gZ3[:, kk, :], b_split=Wk_split)
                 a = self._fctp_args(k, x1[b0:b1], x2[b0:b1], b1 - b0)
                 a.z, a.z_dtype, a.ldz = gZ.data_ptr(), _lib.F32, N
-                a.gx1, a.gx2 = gx1[b0:b1].data_ptr(), gx2[b0:b1].data_ptr()
+                a.gx1, a.gx2 = (t[b0:b1].data_ptr() if t is not None else None for t in (gx1, gx2))
                 with profiling.kernel("fctp_consume_gz"):
                     _lib.check(_lib.lib().cueq_b200_fctp_consume_gz(C.byref(a), C.c_void_p(torch.cuda.current_stream().cuda_stream)))
                 del gZ, gZ3
@@ -856,9 +858,10 @@ class _DenseOut(torch.autograd.Function):
         g = g.contiguous()
         gw = _DenseGw.apply(ctx.owner, x1, x2, g) if ctx.needs_input_grad[1] else None
         gx1 = gx2 = None
-        if ctx.needs_input_grad[2] or ctx.needs_input_grad[3]:
-            gx1, gx2 = _DenseGx.apply(ctx.owner, w, x1, x2, g)
-        return None, gw, gx1 if ctx.needs_input_grad[2] else None, gx2 if ctx.needs_input_grad[3] else None
+        need = tuple(ctx.needs_input_grad[2:4])
+        if any(need):
+            gx1, gx2 = _DenseGx.apply(ctx.owner, need, w, x1, x2, g)
+        return None, gw, gx1, gx2
 
 
 class _DenseGw(torch.autograd.Function):
@@ -873,26 +876,27 @@ class _DenseGw(torch.autograd.Function):
         x1, x2, g = ctx.saved_tensors
         tw = tw.contiguous()
         gx1 = gx2 = gg = None
-        if ctx.needs_input_grad[1] or ctx.needs_input_grad[2]:
-            gx1, gx2 = _DenseGx.apply(ctx.owner, tw, x1, x2, g)
+        need = tuple(ctx.needs_input_grad[1:3])
+        if any(need):
+            gx1, gx2 = _DenseGx.apply(ctx.owner, need, tw, x1, x2, g)
         if ctx.needs_input_grad[3]:
             gg = _DenseOut.apply(ctx.owner, tw, x1, x2)
-        return None, gx1 if ctx.needs_input_grad[1] else None, gx2 if ctx.needs_input_grad[2] else None, gg
+        return None, gx1, gx2, gg
 
 
 class _DenseGx(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, owner, w, x1, x2, g):
+    def forward(ctx, owner, need, w, x1, x2, g):
         ctx.owner = owner
         ctx.set_materialize_grads(False)
         ctx.save_for_backward(w, x1, x2, g)
-        return owner.map_x(w.detach(), x1.detach(), x2.detach(), g.detach())
+        return owner.map_x(w.detach(), x1.detach(), x2.detach(), g.detach(), need)
 
     @staticmethod
     def backward(ctx, t1, t2):
         w, x1, x2, g = ctx.saved_tensors
         owner = ctx.owner
-        need_w, need_1, need_2, need_g = ctx.needs_input_grad[1:5]
+        need_w, need_1, need_2, need_g = ctx.needs_input_grad[2:6]
         gw = g1 = g2 = gg = None
 
         def add(a, b):
@@ -903,7 +907,7 @@ class _DenseGx(torch.autograd.Function):
             if need_w:
                 gw = add(gw, _DenseGw.apply(owner, t1, x2, g))
             if need_2:
-                g2 = add(g2, _DenseGx.apply(owner, w, t1, x2, g)[1])
+                g2 = add(g2, _DenseGx.apply(owner, (False, True), w, t1, x2, g)[1])
             if need_g:
                 gg = add(gg, _DenseOut.apply(owner, w, t1, x2))
         if t2 is not None:          # <t2, dPhi/dx2(w, x1, g)> = Phi(w, x1, t2, g)
@@ -911,7 +915,7 @@ class _DenseGx(torch.autograd.Function):
             if need_w:
                 gw = add(gw, _DenseGw.apply(owner, x1, t2, g))
             if need_1:
-                g1 = add(g1, _DenseGx.apply(owner, w, x1, t2, g)[0])
+                g1 = add(g1, _DenseGx.apply(owner, (True, False), w, x1, t2, g)[0])
             if need_g:
                 gg = add(gg, _DenseOut.apply(owner, w, x1, t2))
-        return None, gw, g1, g2, gg
+        return None, None, gw, g1, g2, gg

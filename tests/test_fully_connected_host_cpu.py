@@ -25,3 +25,50 @@ def test_bf16_weights_follow_the_values():
         version = w._version
         w.data.mul_(-0.5)
         assert w._version == version
+
+
+class _Owner:
+    """out[z] = w x1[z] x2[z], elementwise, with the interface of the float32 route."""
+
+    def __init__(self):
+        self.asked = []
+
+    def map_out(self, w, x1, x2):
+        return w * x1 * x2
+
+    def map_w(self, x1, x2, g):
+        return (x1 * x2 * g).sum(0, keepdim=True)
+
+    def map_x(self, w, x1, x2, g, need=(True, True)):
+        self.asked.append(need)
+        return (w * x2 * g if need[0] else None), (w * x1 * g if need[1] else None)
+
+
+@pytest.mark.parametrize("need", [(True, False), (False, True), (True, True)])
+def test_only_the_gradients_asked_for(need):
+    torch.manual_seed(0)
+    owner = _Owner()
+    w, x1, x2, g = (torch.randn(n, 4, dtype=torch.float64) for n in (1, 5, 5, 5))
+    xs = [t.requires_grad_(n) for t, n in zip((x1, x2), need)]
+    out = fused_tp._DenseOut.apply(owner, w, *xs)
+    wanted = [t for t in xs if t.requires_grad]
+    grads = torch.autograd.grad(out, wanted, g)
+    assert owner.asked == [need]
+    ref = torch.autograd.grad(w * xs[0] * xs[1], wanted, g)
+    assert all(torch.allclose(a, b, rtol=1e-14) for a, b in zip(grads, ref))
+
+
+def test_derivatives_to_third_order():
+    torch.manual_seed(0)
+    owner = _Owner()
+    xs = [torch.randn(n, 3, dtype=torch.float64, requires_grad=True) for n in (1, 4, 4)]
+    f = lambda *a: fused_tp._DenseOut.apply(owner, *a)  # noqa: E731
+    assert torch.autograd.gradcheck(f, xs) and torch.autograd.gradgradcheck(f, xs)
+
+    def third(fn):
+        a = torch.autograd.grad(fn(*xs).pow(2).sum(), xs, create_graph=True)
+        b = torch.autograd.grad(sum(t.pow(2).sum() for t in a), xs, create_graph=True)
+        return torch.autograd.grad(sum(t.pow(2).sum() for t in b), xs)
+
+    for a, b in zip(third(f), third(lambda w, a, b: w * a * b)):
+        assert torch.allclose(a, b, rtol=1e-10)
