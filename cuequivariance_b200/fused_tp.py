@@ -43,6 +43,8 @@ from .polynomial import Polynomial
 FLATTEN_LIMIT = 20000  # flattened paths above which the composite route is taken
 FUSED_GW = True
 FUSED = True  # fully connected tensor-core route: build the coupled operand on chip when the shape allows
+TRI_CHUNK = 2**30  # float32 values of the widest transposed operand per pass of the output and input gradients (4 GB)
+GW_CHUNK = 2**28   # ... and of each of the weight gradient's three transposed arrays (1 GB)
 
 
 def _flatten_all_but_inner(poly: Polynomial) -> Polynomial:
@@ -386,7 +388,7 @@ class DenseUVW:
             w = w.to(torch.bfloat16 if bf16 else torch.float32)
         hi = torch.empty((n * c * c, c), dtype=dt, device=dev)
         lo = None if bf16 else torch.empty_like(hi)
-        step = min(B, max(128, 2**30 // max(x.shape[1] for x in xs) // 128 * 128))   # transposed operands of 4 GB at most
+        step = min(B, max(128, TRI_CHUNK // max(x.shape[1] for x in xs) // 128 * 128))
         rt = c if c <= 64 else c // 2
         with torch.cuda.device(dev):
             stream = C.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
@@ -454,7 +456,7 @@ class DenseUVW:
         xs = [x.contiguous() for x in operands]
         dev, B, rows = xs[0].device, xs[0].shape[0], row0[-1]
         gw = torch.zeros((1, self.d.operands[0].size), dtype=torch.float32, device=dev)
-        step = min(B, max(128, 2**28 // rows // 128 * 128))          # 1 GB for each of the three transposed arrays
+        step = min(B, max(128, GW_CHUNK // rows // 128 * 128))
         with torch.cuda.device(dev):
             stream = C.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
             for b0 in range(0, B, step):

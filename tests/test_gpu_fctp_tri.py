@@ -64,9 +64,12 @@ def test_against_float64_sums(mul, lmax, batch, dtype):
         assert bool((err <= bound).all()), (name, (err / bound).max().item())
         # ... and the typical error is that of float32 sums, not the worst case
         rel = (err.norm() / b.norm()).item()
+        typical = 2.0 ** -8 if dt == torch.bfloat16 else 2.0 ** -19
         if mul == 96 and name == "out":
-            continue                             # long chains on the memory route
-        assert rel <= (2.0 ** -8 if dt == torch.bfloat16 else 2.0 ** -19), (name, rel)
+            # the memory route: up to six paths' (u, v) in one sum, eight per instruction on four accumulators that cut up to
+            # 2^-23 of the sum, 2^-24 on average, with each addition
+            typical = 6 * mul * mul / (8 * 4) * 2.0 ** -24
+        assert rel <= typical, (name, rel)
 
 
 def test_missing_paths_passes_and_second_order():
