@@ -41,7 +41,7 @@ class Buffer(C.Structure):
         ("dtype", C.c_int32),
         ("index", C.c_void_p),
         ("index_is_64", C.c_int32),
-        ("layout", C.c_int32),
+        ("reserved", C.c_int32),
     ]
 
 
@@ -58,7 +58,13 @@ class CwArgs(C.Structure):
         ("w_offset", C.c_int32 * 8), ("out_offset", C.c_int32 * 8),
         ("x1_mul_ir", C.c_int32), ("out_mul_ir", C.c_int32), ("channels_per_lane", C.c_int32), ("staging", C.c_int32),
         ("status", C.c_void_p), ("recv_mod", C.c_int32), ("variant", C.c_int32),
-        ("path_mask", C.c_int32), ("x2_width", C.c_int32), ("dtype", C.c_int32), ("mean_degree", C.c_int32),
+    ]
+
+
+class CwOptions(C.Structure):
+    _fields_ = [
+        ("struct_bytes", C.c_int32), ("path_mask", C.c_int32), ("x2_width", C.c_int32), ("dtype", C.c_int32), ("mean_degree", C.c_int32),
+        ("reserved", C.c_int32),
     ]
 
 
@@ -71,7 +77,7 @@ class CwNoAllocArgs(C.Structure):
         ("num_edges", C.c_int64), ("num_receivers", C.c_int64),
         ("extent", C.c_int32), ("x1_offset", C.c_int32), ("num_paths", C.c_int32), ("num_terms", C.c_int32),
         ("w_offset", C.c_int32 * 8), ("out_offset", C.c_int32 * 8),
-        ("mul_ir", C.c_int32), ("path_mask", C.c_int32),
+        ("mul_ir", C.c_int32), ("reserved", C.c_int32),
     ]
 
 
@@ -286,7 +292,9 @@ def lib() -> C.CDLL:
     L.cueq_b200_cw_backward.argtypes = [C.c_int, C.POINTER(CwArgs), C.c_void_p]
     L.cueq_b200_csr_rowptr.argtypes = [C.c_void_p, C.c_int, C.c_int64, C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p]
     L.cueq_b200_csr_small.argtypes = [C.c_void_p, C.c_int, C.c_int64, C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p]
-    L.cueq_b200_cw_run.argtypes = [C.c_int, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]
+    L.cueq_b200_cw_forward_opt.argtypes = [C.c_int, C.POINTER(CwArgs), C.POINTER(CwOptions), C.c_void_p]
+    L.cueq_b200_cw_backward_opt.argtypes = [C.c_int, C.POINTER(CwArgs), C.POINTER(CwOptions), C.c_void_p]
+    L.cueq_b200_cw_run.argtypes = [C.c_int, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int32, C.c_void_p]
     L.cueq_b200_cw_forward_noalloc.argtypes = [C.c_int, C.POINTER(CwNoAllocArgs), C.c_void_p]
     L.cueq_b200_u1d_static_find.argtypes = [C.c_char_p]
     L.cueq_b200_u1d_static_find.restype = C.c_int
@@ -294,6 +302,8 @@ def lib() -> C.CDLL:
     L.cueq_b200_u1d_static_name.restype = C.c_char_p
     L.cueq_b200_u1d_static_launch.argtypes = [C.c_int, C.c_int64, C.c_int32, C.POINTER(Buffer), C.POINTER(C.c_int32),
                                               C.POINTER(C.c_int32), C.c_int32, C.c_void_p]
+    L.cueq_b200_u1d_static_launch_layouts.argtypes = [C.c_int, C.c_int64, C.c_int32, C.POINTER(Buffer), C.POINTER(C.c_int32),
+                                              C.POINTER(C.c_int32), C.c_int32, C.POINTER(C.c_int32), C.c_void_p]
     L.cueq_b200_gemm_bf16_tn.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_int64, C.c_int64,
                                          C.c_int64, C.c_int64, C.c_int32, C.c_void_p, C.c_void_p]
     L.cueq_b200_gemm_bf16.argtypes = [C.POINTER(GemmArgs), C.c_void_p]

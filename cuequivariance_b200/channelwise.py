@@ -419,13 +419,14 @@ class _ChannelwiseBase:
                 t.out_offset[q] = g["out_off"][q]
             keep = None
             # x2 holds l = 0, 1, 2, ... in order and no path of a group reads beyond l = 3: the first 16 components of a wider row
-            t.path_mask, t.x2_width, t.dtype = g["mask"], min(plan.row_sizes[2], 16), _lib.F64 if f64 else _lib.F32
+            o = _lib.CwOptions()
+            o.struct_bytes, o.path_mask, o.x2_width, o.dtype = C.sizeof(o), g["mask"], min(plan.row_sizes[2], 16), _lib.F64 if f64 else _lib.F32
             if which == "bwd_tab":
                 keep = ((C.c_double if f64 else C.c_float) * g["nterm"])(*g["bwd_tab"][2])
                 t.bwd_coef = C.cast(keep, C.c_void_p)
-            tmpl = (bytes(t), keep)
+            tmpl = (bytes(t), keep, bytes(o))
             cache[(which, f64)] = tmpl
-        a = _lib.CwArgs.from_buffer_copy(tmpl[0])
+        a, o = _lib.CwArgs.from_buffer_copy(tmpl[0]), _lib.CwOptions.from_buffer_copy(tmpl[2])
         for k, t in tensors.items():
             if t is not None and t.numel():
                 setattr(a, k, t.data_ptr())
@@ -437,7 +438,7 @@ class _ChannelwiseBase:
         ts, tj, tc = tabs[which]
         a.tab_start, a.tab_j, a.tab_c = ts.data_ptr(), tj.data_ptr(), tc.data_ptr()
         a.num_receivers = nrecv
-        a.mean_degree = tensors["w"].shape[0] // max(nrecv, 1)
+        o.mean_degree = tensors["w"].shape[0] // max(nrecv, 1)
         if x1_is_block:
             # may be a column slice of a wider tensor (several irrep blocks gathered together); a
             # gradient block, if any, must then be the matching slice of an equally wide tensor
@@ -455,7 +456,7 @@ class _ChannelwiseBase:
         a.variant = BWD_VARIANT if which == "bwd_tab" else 0
         if a.staging:
             a.status = _lib.status_word(tensors["w"].device).data_ptr()
-        return a, tmpl[1]
+        return a, o, tmpl[1]
 
     def _run_groups(self, which, common, csr_rows, mul_ir, recv_mod, **tensors) -> bool:
         """All groups by one library call, or False when they have to be launched one by one: to be timed, or with
@@ -476,13 +477,13 @@ class _ChannelwiseBase:
         kept = plan._templates.get(key)
         if kept is None:
             n = len(plan.groups)
-            arr, keep = (_lib.CwArgs * n)(), []
+            arr, opts, keep = (_lib.CwArgs * n)(), (_lib.CwOptions * n)(), []
             for i, (g, t) in enumerate(zip(plan.groups, plan.tables_on(dev, w.dtype))):
-                arr[i], k = self._args(g, t, which, dict(senders=None, x1_mul_ir=False), None, t[which][0], 0, False, dict(w=w))
+                arr[i], opts[i], k = self._args(g, t, which, dict(senders=None, x1_mul_ir=False), None, t[which][0], 0, False, dict(w=w))
                 keep.append((k, t))
-            kept = (n, (C.c_int32 * n)(*[g["id"] for g in plan.groups]), arr, keep)
+            kept = (n, (C.c_int32 * n)(*[g["id"] for g in plan.groups]), arr, opts, keep)
             plan._templates[key] = kept
-        n, groups, arr, _ = kept
+        n, groups, arr, opts, _ = kept
         a = _lib.CwArgs()
         for name, t in tensors.items():
             if t is not None:
@@ -492,10 +493,10 @@ class _ChannelwiseBase:
         if order is not None:
             a.order = order.data_ptr()
         a.rowptr, a.num_receivers, a.recv_mod = rowptr.data_ptr(), nrecv, recv_mod
-        a.mean_degree = w.shape[0] // max(nrecv, 1)
         a.x1_mul_ir, a.out_mul_ir = int(common["x1_mul_ir"]), int(mul_ir)
         with _lib.on_device(dev):
-            _lib.check(_lib.lib().cueq_b200_cw_run(int(which == "bwd_tab"), n, groups, arr, C.byref(a), torch.cuda.current_stream(dev).cuda_stream))
+            _lib.check(_lib.lib().cueq_b200_cw_run(int(which == "bwd_tab"), n, groups, arr, opts, C.byref(a), w.shape[0] // max(nrecv, 1),
+                                                    torch.cuda.current_stream(dev).cuda_stream))
         profiling.launch_count += n
         return True
 
@@ -513,9 +514,9 @@ class _ChannelwiseBase:
         g, t = self.plan.groups[gi], self.plan.tables_on(w.device, w.dtype)[gi]
         stream = C.c_void_p(torch.cuda.current_stream(w.device).cuda_stream)
         with torch.cuda.device(w.device):
-            a, _ = self._args(g, t, "fwd_tab", common, order, rowptr, nrecv, mul_ir, dict(w=w, x1=x1_block, x2=x2, out=out), x1_is_block=True)
+            a, o, _ = self._args(g, t, "fwd_tab", common, order, rowptr, nrecv, mul_ir, dict(w=w, x1=x1_block, x2=x2, out=out), x1_is_block=True)
             with profiling.kernel(f"cw_fwd[{g['id']}]", stream):
-                _lib.check(_lib.lib().cueq_b200_cw_forward(g["id"], C.byref(a), stream))
+                _lib.check(_lib.lib().cueq_b200_cw_forward_opt(g["id"], C.byref(a), C.byref(o), stream))
 
     def launch_backward_group(self, gi, common, csr, mul_ir, w, x1_block, x2, gout, gw, gx1_block, gx2):
         import ctypes as C
@@ -528,10 +529,10 @@ class _ChannelwiseBase:
         g, t = self.plan.groups[gi], self.plan.tables_on(w.device, w.dtype)[gi]
         stream = C.c_void_p(torch.cuda.current_stream(w.device).cuda_stream)
         with torch.cuda.device(w.device):
-            a, keep = self._args(g, t, "bwd_tab", common, order, rowptr, nrecv, mul_ir,
+            a, o, keep = self._args(g, t, "bwd_tab", common, order, rowptr, nrecv, mul_ir,
                                  dict(w=w, x1=x1_block, x2=x2, gout=gout, gw=gw, gx1=gx1_block, gx2=gx2), x1_is_block=True)
             with profiling.kernel(f"cw_bwd[{g['id']}]", stream):
-                _lib.check(_lib.lib().cueq_b200_cw_backward(g["id"], C.byref(a), stream))
+                _lib.check(_lib.lib().cueq_b200_cw_backward_opt(g["id"], C.byref(a), C.byref(o), stream))
             del keep
 
     def _launch_forward(self, common, csr, mul_ir, w, x1, x2):
@@ -550,9 +551,9 @@ class _ChannelwiseBase:
         stream = C.c_void_p(torch.cuda.current_stream(w.device).cuda_stream)
         with torch.cuda.device(w.device):
             for g, t in zip(plan.groups, tabs):
-                a, _ = self._args(g, t, "fwd_tab", common, order, rowptr, nrecv, mul_ir, dict(w=w, x1=x1, x2=x2, out=out))
+                a, o, _ = self._args(g, t, "fwd_tab", common, order, rowptr, nrecv, mul_ir, dict(w=w, x1=x1, x2=x2, out=out))
                 with profiling.kernel(f"cw_fwd[{g['id']}]", stream):
-                    _lib.check(_lib.lib().cueq_b200_cw_forward(g["id"], C.byref(a), stream))
+                    _lib.check(_lib.lib().cueq_b200_cw_forward_opt(g["id"], C.byref(a), C.byref(o), stream))
         return out
 
     def _launch_backward(self, common, csr, mul_ir, w, x1, x2, gout, needs):
@@ -579,11 +580,11 @@ class _ChannelwiseBase:
         stream = C.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
         with torch.cuda.device(dev):
             for g, t in zip(plan.groups, tabs):
-                a, keep = self._args(g, t, "bwd_tab", common, order, rowptr, nrecv, mul_ir,
+                a, o, keep = self._args(g, t, "bwd_tab", common, order, rowptr, nrecv, mul_ir,
                                      dict(w=w, x1=x1, x2=x2, gout=gout, gw=gw, gx1=gx1, gx2=gx2))
                 a.recv_mod = recv_mod
                 with profiling.kernel(f"cw_bwd[{g['id']}]", stream):
-                    _lib.check(_lib.lib().cueq_b200_cw_backward(g["id"], C.byref(a), stream))
+                    _lib.check(_lib.lib().cueq_b200_cw_backward_opt(g["id"], C.byref(a), C.byref(o), stream))
                 del keep
         return gw, gx1, gx2
 

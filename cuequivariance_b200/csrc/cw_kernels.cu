@@ -25,7 +25,7 @@ template <class T>
 bool is_masked(const CwParamsT<T>& p, const GroupEntry& g) { return p.path_mask != (1u << g.npath) - 1u || p.nx2 != g.nx2 || (p.x2_stride & 3); }
 
 template <class T>
-int fill_params(const cueq_cw_args* a, const GroupEntry& g, CwParamsT<T>& p, int expected_terms) {
+int fill_params(const cueq_cw_args* a, const cueq_cw_options& o, const GroupEntry& g, CwParamsT<T>& p, int expected_terms) {
   constexpr int V = 16 / (int)sizeof(T);   // elements per 16-byte access
   if (!a) return cueq::fail("channelwise: null arguments");
   if (a->extent < V || a->extent % V) return cueq::fail("channelwise: extent %d must be a positive multiple of %d", a->extent, V);
@@ -53,8 +53,8 @@ int fill_params(const cueq_cw_args* a, const GroupEntry& g, CwParamsT<T>& p, int
   if ((p.w_stride | p.x1_stride | p.out_stride) & (V - 1)) return cueq::fail("channelwise: row strides must be multiples of %d elements", V);
   const uintptr_t ptrs = (uintptr_t)a->w | (uintptr_t)a->x1 | (uintptr_t)a->x2 | (uintptr_t)a->out | (uintptr_t)a->gout | (uintptr_t)a->gw | (uintptr_t)a->gx1;
   const unsigned all = (1u << g.npath) - 1u;
-  p.path_mask = a->path_mask ? (unsigned)a->path_mask : all;
-  p.nx2 = a->x2_width ? a->x2_width : g.nx2;
+  p.path_mask = o.path_mask ? (unsigned)o.path_mask : all;
+  p.nx2 = o.x2_width ? o.x2_width : g.nx2;
   if ((p.path_mask & ~all) || p.nx2 < 1 || p.nx2 > g.nx2) return cueq::fail("channelwise: path mask or x2 width outside the group");
   if (ptrs & 15) return cueq::fail("channelwise: tensors must be 16-byte aligned");
   p.need_gw = a->gw != nullptr; p.need_gx1 = a->gx1 != nullptr; p.need_gx2 = a->gx2 != nullptr;
@@ -78,18 +78,26 @@ extern "C" int cueq_b200_cw_group_info(int g, int32_t* d1, int32_t* npath, int32
 
 namespace {
 
-int run_forward(int g, const cueq_cw_args* a, int overlap, void* stream) {
+int take_options(const cueq_cw_options* options, cueq_cw_options& o) {
+  std::memset(&o, 0, sizeof(o));
+  if (!options) return 0;
+  if (options->struct_bytes != (int)sizeof(o)) return cueq::fail("channelwise: the binding declares another options block");
+  o = *options;
+  return 0;
+}
+
+int run_forward(int g, const cueq_cw_args* a, const cueq_cw_options& o, int overlap, void* stream) {
   if (g < 0 || g >= kNumGroups) return cueq::fail("channelwise: group %d out of range", g);
-  if (a && a->dtype == CUEQ_F64) {
+  if (o.dtype == CUEQ_F64) {
     CwParamsT<double> p;
-    if (int rc = fill_params(a, *kGroups[g], p, kGroups[g]->nterm_fwd)) return rc;
+    if (int rc = fill_params(a, o, *kGroups[g], p, kGroups[g]->nterm_fwd)) return rc;
     p.overlap = overlap;
     if (!p.w || !p.x1 || !p.x2 || !p.out) return cueq::fail("channelwise forward: null tensor");
     return p.num_receivers == 0 ? 0 : kGroups64[g]->fwd(p, a->x1_mul_ir, reinterpret_cast<cudaStream_t>(stream));
   }
-  if (a && a->dtype != CUEQ_F32) return cueq::fail("channelwise: float32 or float64 operands");
+  if (o.dtype != CUEQ_F32) return cueq::fail("channelwise: float32 or float64 operands");
   CwParams p;
-  if (int rc = fill_params(a, *kGroups[g], p, kGroups[g]->nterm_fwd)) return rc;
+  if (int rc = fill_params(a, o, *kGroups[g], p, kGroups[g]->nterm_fwd)) return rc;
   p.overlap = overlap;
   if (!p.w || !p.x1 || !p.x2 || !p.out) return cueq::fail("channelwise forward: null tensor");
   if (p.num_receivers == 0) return 0;
@@ -100,11 +108,11 @@ int run_forward(int g, const cueq_cw_args* a, int overlap, void* stream) {
   return kGroups[g]->fwd(p, a->x1_mul_ir, pick_cpl(a), masked, reinterpret_cast<cudaStream_t>(stream));
 }
 
-int run_backward(int g, const cueq_cw_args* a, int overlap, void* stream) {
+int run_backward(int g, const cueq_cw_args* a, const cueq_cw_options& o, int overlap, void* stream) {
   if (g < 0 || g >= kNumGroups) return cueq::fail("channelwise: group %d out of range", g);
-  if (a && a->dtype == CUEQ_F64) {
+  if (o.dtype == CUEQ_F64) {
     CwParamsT<double> p;
-    if (int rc = fill_params(a, *kGroups[g], p, kGroups[g]->nterm)) return rc;
+    if (int rc = fill_params(a, o, *kGroups[g], p, kGroups[g]->nterm)) return rc;
     p.overlap = overlap;
     if (!p.w || !p.x1 || !p.x2 || !p.gout) return cueq::fail("channelwise backward: null tensor");
     if (!a->bwd_coef) return cueq::fail("channelwise backward: null coefficient table");
@@ -113,9 +121,9 @@ int run_backward(int g, const cueq_cw_args* a, int overlap, void* stream) {
     for (int t = 0; t < kGroups[g]->nterm; ++t) coef.c[t] = static_cast<const double*>(a->bwd_coef)[t];
     return p.num_receivers == 0 ? 0 : kGroups64[g]->bwd(p, coef, a->x1_mul_ir, reinterpret_cast<cudaStream_t>(stream));
   }
-  if (a && a->dtype != CUEQ_F32) return cueq::fail("channelwise: float32 or float64 operands");
+  if (o.dtype != CUEQ_F32) return cueq::fail("channelwise: float32 or float64 operands");
   CwParams p;
-  if (int rc = fill_params(a, *kGroups[g], p, kGroups[g]->nterm)) return rc;
+  if (int rc = fill_params(a, o, *kGroups[g], p, kGroups[g]->nterm)) return rc;
   p.overlap = overlap;
   if (!p.w || !p.x1 || !p.x2 || !p.gout) return cueq::fail("channelwise backward: null tensor");
   if (!a->bwd_coef) return cueq::fail("channelwise backward: null coefficient table");
@@ -129,7 +137,7 @@ int run_backward(int g, const cueq_cw_args* a, int overlap, void* stream) {
   // and few edges per receiver the cotangent row is staged by a block for too little work; 100,000 edges, lmax 3, one warp
   // against one block per receiver: 64 channels, 20 edges 680 / 536 us, 5 edges 720 / 757 us; 32 channels, 5 edges
   // 1371 / 687 us; 2,000 edges on 100 receivers, 64 channels: 153 / 51 us.
-  const bool few = a->mean_degree > 0 && a->mean_degree < 8 && a->extent > 32 && a->extent % 128;
+  const bool few = o.mean_degree > 0 && o.mean_degree < 8 && a->extent > 32 && a->extent % 128;
   const bool masked = is_masked(p, *kGroups[g]);
   const bool block_per_receiver = a->variant >= 2 || (a->variant == 0 && a->channels_per_lane != 2 && !few);
   if (a->variant == 3 && a->extent % 128) return cueq::fail("channelwise backward: variant 3 needs a multiple of 128 channels");
@@ -143,28 +151,40 @@ int run_backward(int g, const cueq_cw_args* a, int overlap, void* stream) {
 
 }  // namespace
 
-extern "C" int cueq_b200_cw_forward(int g, const cueq_cw_args* a, void* stream) { return run_forward(g, a, 0, stream); }
-
-extern "C" int cueq_b200_cw_backward(int g, const cueq_cw_args* a, void* stream) { return run_backward(g, a, 0, stream); }
+extern "C" int cueq_b200_cw_forward_opt(int g, const cueq_cw_args* a, const cueq_cw_options* options, void* stream) {
+  cueq_cw_options o;
+  if (int rc = take_options(options, o)) return rc;
+  return run_forward(g, a, o, 0, stream);
+}
+extern "C" int cueq_b200_cw_backward_opt(int g, const cueq_cw_args* a, const cueq_cw_options* options, void* stream) {
+  cueq_cw_options o;
+  if (int rc = take_options(options, o)) return rc;
+  return run_backward(g, a, o, 0, stream);
+}
+extern "C" int cueq_b200_cw_forward(int g, const cueq_cw_args* a, void* stream) { return cueq_b200_cw_forward_opt(g, a, nullptr, stream); }
+extern "C" int cueq_b200_cw_backward(int g, const cueq_cw_args* a, void* stream) { return cueq_b200_cw_backward_opt(g, a, nullptr, stream); }
 
 // All groups of a polynomial by one call: the constant part of each group's arguments comes from `templates`, which the
 // caller keeps, tensors and sizes from `call`.  Every group but the first may start before the one in front of it has
 // ended (cw_kernels.cuh, launch_kernel), unless that would leave the x2 gradient's sum in no fixed order: where one block of
 // channels holds them all, a group adds one value to a component, the first two in either order (0 + a + b), the others
 // each after the groups before.  Several blocks of channels add in no fixed order anyway.
-extern "C" int cueq_b200_cw_run(int backward, int num_groups, const int32_t* groups, const cueq_cw_args* templates, const cueq_cw_args* call,
-                                void* stream) {
-  if (num_groups < 0 || (num_groups && (!groups || !templates || !call))) return cueq::fail("channelwise: null argument");
+extern "C" int cueq_b200_cw_run(int backward, int num_groups, const int32_t* groups, const cueq_cw_args* templates, const cueq_cw_options* options,
+                                const cueq_cw_args* call, int32_t mean_degree, void* stream) {
+  if (num_groups < 0 || (num_groups && (!groups || !templates || !options || !call))) return cueq::fail("channelwise: null argument");
   for (int i = 0; i < num_groups; ++i) {
     cueq_cw_args a = templates[i];
+    cueq_cw_options o;
+    if (int rc = take_options(options + i, o)) return rc;
+    o.mean_degree = mean_degree;
     a.w = call->w; a.x1 = call->x1; a.x2 = call->x2; a.out = call->out;
     a.gout = call->gout; a.gw = call->gw; a.gx1 = call->gx1; a.gx2 = call->gx2;
     a.senders = call->senders; a.order = call->order; a.rowptr = call->rowptr;
-    a.num_receivers = call->num_receivers; a.recv_mod = call->recv_mod; a.mean_degree = call->mean_degree;
+    a.num_receivers = call->num_receivers; a.recv_mod = call->recv_mod;
     a.x1_mul_ir = call->x1_mul_ir; a.out_mul_ir = call->out_mul_ir;
-    const bool one_block = a.extent <= (a.dtype == CUEQ_F32 && a.extent % 128 == 0 ? 128 : 64);
+    const bool one_block = a.extent <= (o.dtype == CUEQ_F32 && a.extent % 128 == 0 ? 128 : 64);
     const int overlap = i > 0 && !(backward && a.gx2 && one_block && i > 1);
-    if (int rc = backward ? run_backward(groups[i], &a, overlap, stream) : run_forward(groups[i], &a, overlap, stream)) return rc;
+    if (int rc = backward ? run_backward(groups[i], &a, o, overlap, stream) : run_forward(groups[i], &a, o, overlap, stream)) return rc;
   }
   return 0;
 }
@@ -262,9 +282,9 @@ extern "C" int cueq_b200_cw_forward_noalloc(int g, const cueq_cw_noalloc_args* a
   full.num_paths = a->num_paths; full.num_terms = a->num_terms;
   for (int q = 0; q < 8; ++q) { full.w_offset[q] = a->w_offset[q]; full.out_offset[q] = a->out_offset[q]; }
   full.x1_mul_ir = a->mul_ir; full.out_mul_ir = a->mul_ir; full.channels_per_lane = 0;
-  full.path_mask = a->path_mask;
+  const cueq_cw_options whole = {};
   CwParams p;
-  if (int rc = fill_params(&full, ge, p, ge.nterm_fwd)) return rc;
+  if (int rc = fill_params(&full, whole, ge, p, ge.nterm_fwd)) return rc;
   if (!p.w || !p.x1 || !p.x2 || !p.out) return cueq::fail("channelwise (no-alloc): null tensor");
   if (p.num_receivers == 0) return 0;
 

@@ -130,11 +130,18 @@ extern "C" const char* cueq_b200_u1d_static_name(int id) { return (id >= 0 && id
 extern "C" int cueq_b200_u1d_static_launch(int id, int64_t batch, int32_t extent, const cueq_buffer* buffers,
                                            const int32_t* buffer_dim, const int32_t* buffer_num_segments, int32_t num_buffers,
                                            void* stream) {
+  const int32_t layouts[kMaxBuf] = {};
+  return cueq_b200_u1d_static_launch_layouts(id, batch, extent, buffers, buffer_dim, buffer_num_segments, num_buffers, layouts, stream);
+}
+
+extern "C" int cueq_b200_u1d_static_launch_layouts(int id, int64_t batch, int32_t extent, const cueq_buffer* buffers,
+                                                   const int32_t* buffer_dim, const int32_t* buffer_num_segments, int32_t num_buffers,
+                                                   const int32_t* layouts, void* stream) {
   if (id < 0 || id >= kNumStatic) return cueq::fail("u1d_static: kernel id %d out of range", id);
   const StaticEntry& e = kStatic[id];
   if (num_buffers != e.num_inputs + e.num_outputs) return cueq::fail("u1d_static: %s takes %d buffers, got %d", e.name, e.num_inputs + e.num_outputs, num_buffers);
   if (num_buffers > kMaxBuf) return cueq::fail("u1d_static: too many buffers");
-  if (!buffers || !buffer_dim || !buffer_num_segments) return cueq::fail("u1d_static: null argument");
+  if (!buffers || !buffer_dim || !buffer_num_segments || !layouts) return cueq::fail("u1d_static: null argument");
   if (batch < 0 || extent < 1) return cueq::fail("u1d_static: invalid batch or extent");
   StaticParams P;
   std::memset(&P, 0, sizeof(P));
@@ -147,9 +154,9 @@ extern "C" int cueq_b200_u1d_static_launch(int id, int64_t batch, int32_t extent
     if (s.mode == CUEQ_INDEXED && !s.index && batch > 0) return cueq::fail("u1d_static: indexed buffer %d has no index", b);
     P.buf[b].ptr = s.ptr; P.buf[b].index = s.index; P.buf[b].mode = s.mode; P.buf[b].index_is_64 = s.index_is_64;
     P.buf[b].vec = buffer_dim[b];
-    if (s.layout != 0 && s.layout != 1) return cueq::fail("u1d_static: buffer %d has invalid layout", b);
-    P.buf[b].mul_ir = s.layout;
-    if (s.layout) {
+    if (layouts[b] != 0 && layouts[b] != 1) return cueq::fail("u1d_static: buffer %d has invalid layout", b);
+    P.buf[b].mul_ir = layouts[b];
+    if (layouts[b]) {
       const int n = buffer_num_segments[b];
       if (!buffer_dim[b] || (n != 1 && n != 4 && n != 9 && n != 16))
         return cueq::fail("u1d_static: buffer %d cannot be channel-major (%d segments, channel axis %d)", b, n, buffer_dim[b]);

@@ -294,25 +294,25 @@ class StaticKernel:
             in_place = [cfg.layout(b) is not None and self._in_place(program, cfg, b) for b in range(len(specs))]
             zeroed = [s.mode != _lib.BATCHED or program.buffer_dim[n_in + j] == 0 for j, s in enumerate(cfg.outputs)]
             kept = (in_place, [cfg.layout(b) is not None and not f for b, f in enumerate(in_place)], zeroed,
-                    _lib.int32_array(program.buffer_dim), _lib.int32_array(program.buffer_num_segments))
+                    _lib.int32_array(program.buffer_dim), _lib.int32_array(program.buffer_num_segments), _lib.int32_array(map(int, in_place)))
             self._kept[key] = kept
-        in_place, transposed, zeroed, dims, segments = kept
+        _, transposed, zeroed, dims, segments, layouts = kept
         xs = [transpose_blocks(x, cfg.layout(i), to_ir_mul=True) if transposed[i] else x for i, x in enumerate(xs)]
         outs = [(torch.zeros if z else torch.empty)((spec.rows, program.row_sizes[n_in + j]), dtype=torch.float32, device=device)
                 for j, (spec, z) in enumerate(zip(cfg.outputs, zeroed))]
         nb = len(specs)
         bufs = (_lib.Buffer * nb)()
         keep = []
-        for buf, t, spec, placed in zip(bufs, xs + outs, specs, in_place):
-            buf.ptr, buf.rows, buf.mode, buf.dtype, buf.layout = t.data_ptr(), spec.rows, spec.mode, _lib.F32, placed
+        for buf, t, spec in zip(bufs, xs + outs, specs):
+            buf.ptr, buf.rows, buf.mode, buf.dtype = t.data_ptr(), spec.rows, spec.mode, _lib.F32
             if spec.mode == _lib.INDEXED:
                 idx = spec.index.contiguous()
                 keep.append(idx)
                 buf.index = idx.data_ptr()
                 buf.index_is_64 = idx.dtype == torch.int64
         with _lib.on_device(device), profiling.kernel(f"u1d_static[{self.name}]"):
-            _lib.check(_lib.lib().cueq_b200_u1d_static_launch(self.kernel_id, cfg.batch, program.extent, bufs, dims, segments, nb,
-                                                              torch.cuda.current_stream(device).cuda_stream))
+            _lib.check(_lib.lib().cueq_b200_u1d_static_launch_layouts(self.kernel_id, cfg.batch, program.extent, bufs, dims, segments, nb, layouts,
+                                                                      torch.cuda.current_stream(device).cuda_stream))
         for j in range(program.num_outputs):
             b = program.num_inputs + j
             if transposed[b]:

@@ -67,8 +67,7 @@ typedef struct {
   int32_t dtype;      /* CUEQ_F32 / F64 / BF16 / F16                                              */
   const void* index;  /* device pointer [batch] when mode == CUEQ_INDEXED, else NULL               */
   int32_t index_is_64; /* 1: int64 indices, 0: int32                                              */
-  int32_t layout;     /* 0: segment after segment (ir_mul).  1: channel-major (mul_ir) blocks of 1, 3, 5, ...
-                         segments, [channel][component] each - cueq_b200_u1d_static_launch only           */
+  int32_t reserved;
 } cueq_buffer;
 
 int cueq_b200_abi_version(void);
@@ -206,7 +205,7 @@ typedef struct {
   const int32_t* rowptr;
   const int32_t* tab_start;
   const int32_t* tab_j;
-  const void* tab_c;    /* float or double, by dtype                                            */
+  const void* tab_c;    /* float, or double with dtype CUEQ_F64 (cueq_cw_options)               */
   const void* bwd_coef;
   int64_t w_stride, x1_stride, x2_stride, out_stride; /* row strides in elements               */
   int64_t num_receivers;
@@ -224,18 +223,24 @@ typedef struct {
                            receiver r % recv_mod), used to visit the edges in sender-range passes        */
   int32_t variant;      /* backward only: 0 = the library chooses (multiples of 128 channels: 3 for x1 degrees >= 1, 2 for
                            the scalar block; other channel counts: the same with two channels per thread, or 1
-                           where receivers have few edges, see mean_degree); 1 = one warp per receiver (2 or 4 channels
+                           where receivers have few edges, see cueq_cw_options); 1 = one warp per receiver (2 or 4 channels
                            per thread); 2 = one thread block per receiver: its warps share the staged
                            cotangent row and split the receiver's edges, four channels per thread;
                            3 = as 2, with the x1 gradient of an edge leaving as one bulk reduction
                            (cp.reduce.async.bulk) per warp instead of vector reductions per lane (mul_ir
                            rows, 128 | extent; falls back to 2 where the rows are not 16-byte aligned)        */
+} cueq_cw_args;
+
+/* What a polynomial is beyond a whole group in float32; null or zeros: nothing. */
+typedef struct {
+  int32_t struct_bytes; /* sizeof(cueq_cw_options) as the caller declares it                       */
   int32_t path_mask;    /* bit q: path q of the group is part of the polynomial (0: all are); tables and offsets
                            keep the full group's numbering, entries of absent paths have no terms           */
   int32_t x2_width;     /* components of an x2 row that the paths read: 1, 4, 9 or 16 (0: 16)            */
   int32_t dtype;        /* CUEQ_F32, or CUEQ_F64: two channels per thread, staging / variant ignored    */
-  int32_t mean_degree;    /* backward: edges per receiver, rounded down (0: unknown); picks the division of the work */
-} cueq_cw_args;
+  int32_t mean_degree;  /* backward: edges per receiver, rounded down (0: unknown); picks the division of the work */
+  int32_t reserved;
+} cueq_cw_options;
 
 /* Row pointers [rows + 1] of an ascending receiver index [n]: rowptr[r] = first position with index >= r.  *descends (zeroed
  * by the caller) becomes 1 if the index does not ascend; the row pointers are then of no use. */
@@ -248,11 +253,14 @@ const char* cueq_b200_cw_group_signature(int group);
 int cueq_b200_cw_group_info(int group, int32_t* d1, int32_t* num_paths, int32_t* num_pairs, int32_t* num_terms);
 int cueq_b200_cw_forward(int group, const cueq_cw_args* args, void* stream);
 int cueq_b200_cw_backward(int group, const cueq_cw_args* args, void* stream);
-/* num_groups forward (backward = 0) or backward launches: group i runs with templates[i], except for the tensors (w, x1, x2,
- * out, gout, gw, gx1, gx2), senders, order, rowptr, num_receivers, recv_mod, mean_degree and the two layouts, which come from
- * `call`. */
-int cueq_b200_cw_run(int backward, int num_groups, const int32_t* groups, const cueq_cw_args* templates, const cueq_cw_args* call,
-                     void* stream);
+/* The same with options (nullable). */
+int cueq_b200_cw_forward_opt(int group, const cueq_cw_args* args, const cueq_cw_options* options, void* stream);
+int cueq_b200_cw_backward_opt(int group, const cueq_cw_args* args, const cueq_cw_options* options, void* stream);
+/* num_groups forward (backward = 0) or backward launches: group i runs with templates[i] and options[i], except for the tensors
+ * (w, x1, x2, out, gout, gw, gx1, gx2), senders, order, rowptr, num_receivers, recv_mod and the two layouts, which come from
+ * `call`, and mean_degree. */
+int cueq_b200_cw_run(int backward, int num_groups, const int32_t* groups, const cueq_cw_args* templates, const cueq_cw_options* options,
+                     const cueq_cw_args* call, int32_t mean_degree, void* stream);
 
 /* ---- kernels written out at build time for known polynomials ---------------------------------
  *
@@ -261,13 +269,17 @@ int cueq_b200_cw_run(int backward, int num_groups, const int32_t* groups, const 
  * generated when the library was built - the counterpart of the per-polynomial NVRTC kernels of
  * the reference's closed op (CHANGELOG.md:38,49).  `digest` identifies the polynomial
  * (cuequivariance_b200/static_poly.py); _find returns a kernel id or -1.
- * A buffer may be channel-major (cueq_buffer.layout = 1) when it has a channel axis and 1, 4, 9 or 16 segments;
- * an output then has to be batched and the extent a multiple of 32. */
+ * _launch_layouts: layouts[b] = 1 where buffer b is channel-major (mul_ir): blocks of 1, 3, 5, ... segments, [channel][component]
+ * each, instead of segment after segment (0).  It then has a channel axis and 1, 4, 9 or 16 segments; an output has to be
+ * batched and the extent a multiple of 32. */
 int cueq_b200_u1d_static_find(const char* digest);
 const char* cueq_b200_u1d_static_name(int id);
 int cueq_b200_u1d_static_launch(int id, int64_t batch, int32_t extent, const cueq_buffer* buffers,
                                 const int32_t* buffer_dim, const int32_t* buffer_num_segments,
                                 int32_t num_buffers, void* stream);
+int cueq_b200_u1d_static_launch_layouts(int id, int64_t batch, int32_t extent, const cueq_buffer* buffers,
+                                const int32_t* buffer_dim, const int32_t* buffer_num_segments,
+                                int32_t num_buffers, const int32_t* layouts, void* stream);
 
 /* ---- tensor-core GEMM for the dense (uvw) contractions --------------------------------------
  *
@@ -604,7 +616,7 @@ typedef struct {
   int32_t w_offset[8];
   int32_t out_offset[8];
   int32_t mul_ir;                /* layout of x1 and out, as in cueq_cw_args                         */
-  int32_t path_mask;            /* as in cueq_cw_args; x2 rows have 16 components                     */
+  int32_t reserved;
 } cueq_cw_noalloc_args;
 
 int cueq_b200_cw_forward_noalloc(int group, const cueq_cw_noalloc_args* args, void* stream);

@@ -22,12 +22,12 @@ def test_matched_plans_pass_the_library_checks(l_in, l_sh, l_out):
         return
     L = _lib.lib()
     for g in plan.groups:
-        for which, fn in (("fwd_tab", L.cueq_b200_cw_forward), ("bwd_tab", L.cueq_b200_cw_backward)):
+        for which, fn in (("fwd_tab", L.cueq_b200_cw_forward_opt), ("bwd_tab", L.cueq_b200_cw_backward_opt)):
             w = torch.zeros(4, plan.row_sizes[0])
             tabs = plan.tables_on(torch.device("cpu"))[plan.groups.index(g)]
             x = torch.zeros(4, max(plan.row_sizes[1:]))
             rp = torch.zeros(1, dtype=torch.int32)
             # no receiver: the checks run, nothing is launched
-            a, keep = cw.ChannelwiseForward(plan)._args(g, tabs, which, dict(senders=None, x1_mul_ir=False), None, rp, 0, False,
+            a, o, keep = cw.ChannelwiseForward(plan)._args(g, tabs, which, dict(senders=None, x1_mul_ir=False), None, rp, 0, False,
                                                         dict(w=w, x1=x, x2=x, **({"out": x} if which == "fwd_tab" else {"gout": x})))
-            assert fn(g["id"], C.byref(a), None) == 0, L.cueq_b200_last_error()
+            assert fn(g["id"], C.byref(a), C.byref(o), None) == 0, L.cueq_b200_last_error()
