@@ -37,7 +37,8 @@ constexpr int kThreads = kConsumers + 128;             // 16: TMA, 17: MMA issue
 constexpr int kBlk = 128 * 128;                        // 128 rows x 128 bytes
 // Registers: 20 warps leave 96 per thread at launch; the consumers' components of R alone are up to 80.  The producers'
 // warpgroup gives its surplus to the four consumer warpgroups: 640 * 96 = 61440 = 512 * 112 + 128 * 32.  Every kernel of
-// this file is compiled to exactly 96 (__launch_bounds__ allows no more, the host checks that it is no less).
+// this file is compiled to exactly 96 (__launch_bounds__ allows no more, the host checks that it is no less; a build by another
+// compiler where it is not says so in cueq_b200_fctp_tri_ready and keeps the routes for other shapes).
 constexpr int kLaunchRegs = 96;
 #define CONSUMER_REGS() asm volatile("setmaxnreg.inc.sync.aligned.u32 112;\n")
 #define PRODUCER_REGS() asm volatile("setmaxnreg.dec.sync.aligned.u32 32;\n")
@@ -424,15 +425,32 @@ int make_map(CUtensorMap* map, bool bf16, const void* base, int64_t rows, int C,
   return 0;
 }
 
+// setmaxnreg.inc would wait for registers that the block was not launched with
+template <bool BF16, int C, int NC>
+cudaError_t launch_regs(int* regs) {
+  cudaFuncAttributes attr;
+  const cudaError_t e = cudaFuncGetAttributes(&attr, fctp_tri_kernel<BF16, C, NC>);
+  *regs = e == cudaSuccess ? attr.numRegs : 0;
+  return e;
+}
+template <bool BF16, int C>
+int compiled_as_needed() {
+  int a = 0, b = 0, c = 0;
+  if (launch_regs<BF16, C, 1>(&a) != cudaSuccess || launch_regs<BF16, C, 3>(&b) != cudaSuccess || launch_regs<BF16, C, 5>(&c) != cudaSuccess) {
+    cudaGetLastError();
+    return -1;
+  }
+  return a == kLaunchRegs && b == kLaunchRegs && c == kLaunchRegs;
+}
+
 template <bool BF16, int C, int NC>
 int launch_c(const CUtensorMap& hi, const CUtensorMap& lo, const TriParams& p, cudaStream_t st) {
   using K = Cfg<BF16, C>;
   static cueq::PerDeviceFlag configured;
   if (!configured.get()) {
-    cudaFuncAttributes attr;
-    CUEQ_CUDA_OK(cudaFuncGetAttributes(&attr, fctp_tri_kernel<BF16, C, NC>));
-    if (attr.numRegs != kLaunchRegs)   // setmaxnreg.inc would wait for registers that the block was not launched with
-      return cueq::fail("fctp tri: compiled to %d registers per thread, the warpgroups divide %d", attr.numRegs, kLaunchRegs);
+    int regs = 0;
+    CUEQ_CUDA_OK((launch_regs<BF16, C, NC>(&regs)));
+    if (regs != kLaunchRegs) return cueq::fail("fctp tri: compiled to %d registers per thread, the warpgroups divide %d", regs, kLaunchRegs);
     CUEQ_CUDA_OK(cudaFuncSetAttribute(fctp_tri_kernel<BF16, C, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)K::smem));
     configured.set();
   }
@@ -472,6 +490,12 @@ int launch(const cueq_fctp_tri_args* a, TriParams& p, cudaStream_t st) {
 }
 
 }  // namespace
+
+extern "C" int cueq_b200_fctp_tri_ready(int dtype, int channels) {
+  if (dtype == CUEQ_BF16) return channels == 128 ? compiled_as_needed<true, 128>() : 0;
+  if (dtype == CUEQ_F32) return channels == 32 ? compiled_as_needed<false, 32>() : channels == 64 ? compiled_as_needed<false, 64>() : 0;
+  return 0;
+}
 
 extern "C" int cueq_b200_fctp_tri(const cueq_fctp_tri_args* a, void* stream) {
   if (!a || !a->out || !a->b_hi || !a->paths) return cueq::fail("fctp tri: null operand");

@@ -271,6 +271,7 @@ class DenseUVW:
         self.out_size = d.operands[3].size
         self._flat = {}
         self._tri_mul = None
+        self._tri_ready = {}
 
     @staticmethod
     def _weights_bf16(w: torch.Tensor, transposed: bool) -> torch.Tensor:
@@ -300,7 +301,11 @@ class DenseUVW:
         # and both input gradients of 32,768 samples of 64x(0e+1o+2e).  Other shapes used to write the coupled operand to
         # memory: the same sums in float32 took 23 ms, 10 ms here.  float32 with 96 channels stays there: chains of twelve
         # additions in the tensor core, input gradients 3.8e-7 off where the memory route is 2.5e-7 off.
-        return c if c in ((128,) if dtype == torch.bfloat16 else (32, 64)) else 0
+        if c not in ((128,) if dtype == torch.bfloat16 else (32, 64)):
+            return 0
+        if dtype not in self._tri_ready:     # 0: a build whose kernels did not come out as they have to
+            self._tri_ready[dtype] = _lib.lib().cueq_b200_fctp_tri_ready(_lib.BF16 if dtype == torch.bfloat16 else _lib.F32, c) != 0
+        return c if self._tri_ready[dtype] else 0
 
     def _gw_channels(self) -> int:
         """Likewise for ``cueq_b200_fctp_gw`` (float32)."""

@@ -375,6 +375,9 @@ typedef struct {
   int32_t reserved;
 } cueq_fctp_tri_args;
 int cueq_b200_fctp_tri(const cueq_fctp_tri_args* args, void* stream);
+/* 1: the kernels for this type and multiplicity are there and were compiled to the registers that their division among the
+ * warps counts on; 0: not (cueq_b200_fctp_tri refuses the call); -1: cannot be told without a device */
+int cueq_b200_fctp_tri_ready(int dtype, int channels);
 /* order[k] = 100 * (axis of p) + 10 * (axis of q) + (axis of r), axes of W[u][v][w]: 0, 1, 2; w_off in elements */
 int cueq_b200_fctp_tri_weights(const void* w, int w_dtype, int dtype, int channels, int num_paths, const int32_t* w_off,
                                const int32_t* order, void* hi, void* lo, void* stream);

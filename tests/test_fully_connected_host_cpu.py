@@ -72,3 +72,28 @@ def test_derivatives_to_third_order():
 
     for a, b in zip(third(f), third(lambda w, a, b: w * a * b)):
         assert torch.allclose(a, b, rtol=1e-10)
+
+
+def test_a_build_without_usable_kernels_keeps_the_memory_route(monkeypatch):
+    """The tri-linear kernels divide a fixed number of registers; a library whose compiler gave them another number says so."""
+    prog, bf16 = _product(64), _product(128)
+    assert prog._tri_channels(torch.float32) == 64 and bf16._tri_channels(torch.bfloat16) == 128
+    asked = []
+
+    class _Lib:
+        def cueq_b200_fctp_tri_ready(self, dtype, channels):
+            asked.append((dtype, channels))
+            return 0
+
+    monkeypatch.setattr(_lib, "lib", _Lib)
+    for p, dt in ((_product_again(prog), torch.float32), (_product_again(bf16), torch.bfloat16)):
+        assert p._tri_channels(dt) == 0 and p._tri_channels(dt) == 0
+    assert asked == [(_lib.F32, 64), (_lib.BF16, 128)]
+    assert _product_again(prog)._gw_channels() == 64
+
+
+def _product_again(prog):
+    """The same product with nothing decided yet."""
+    new = object.__new__(type(prog))
+    new.__dict__.update(prog.__dict__, _tri_mul=None, _tri_ready={})
+    return new
