@@ -66,8 +66,9 @@ def digest(poly: Polynomial) -> str:
 
 def registered_polynomials() -> List[Tuple[str, Polynomial]]:
     """(name, flattened polynomial) of everything that gets a static kernel: the MACE symmetric contractions
-    0e+1o[+2e[+3o]] -> 0e[+1o] of degree 2 and 3 - the shapes whose path tables ship with the package, so that the
-    digest cannot depend on the host that evaluates it - and their first derivatives, each alone and both together."""
+    0e+1o[+2e[+3o]] -> 0e[+1o] of degree 2 and 3 and their first derivatives, each alone and both together.  The path
+    tables of these shapes ship with the package, so that the digest cannot depend on the host that evaluates it (tables
+    ship for 0e -> 0e, for outputs 0e+1o+2e and for degree 1 too; those run on the table-driven kernel)."""
     from . import descriptors
 
     out = []
