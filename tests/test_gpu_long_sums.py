@@ -48,17 +48,18 @@ def test_linear_weight_gradient_beyond_the_usual_grid(rows, classes):
     out = m(x.to(DEV), wd, None if idx is None else idx.to(DEV))
     (gw,) = torch.autograd.grad(out, [wd], cot.to(DEV))
     ref, mag = (_reference(m._fused_plan, m, bounds, f(w.double()), f(x.double()), f(cot.double()), cb.mul_ir, cb.mul_ir)[1] for f in (lambda t: t, torch.abs))
-    # the bound of test_gpu_linear_fused.py: 4 * 128 / 3 additions per accumulator, four accumulators, one per thread block
+    # the bound of test_gpu_linear_fused.py: 4 * 128 / 3 additions per accumulator, four accumulators, one per thread block;
+    # the tensor core cuts up to 2^-23 of the sum with each addition, 2^-24 on average
     err = (gw.cpu().double() - ref).abs()
     assert bool((err <= (2.0 ** -21 + (200 + rows // 64) * 2.0 ** -23) * mag).all())
-    assert float(err.norm() / ref.norm()) <= 2.0 ** -19
+    assert float(err.norm() / ref.norm()) <= 4 * 128 / 3 * 2.0 ** -24
 
 
-@pytest.mark.parametrize("mul,batch", [(32, 200), (64, 130)])
-def test_second_derivatives_by_value(mul, batch):
+@pytest.mark.parametrize("mul,lmax,batch", [(32, 2, 100), (64, 1, 130)])
+def test_second_derivatives_by_value(mul, lmax, batch):
     """Gradients of a sum of squares of all first gradients, against the same in float64 by plain sums: three contractions one
     after the other, each within 2^-19 of its result, and the factor of the square."""
-    s = f"{mul}x0e+{mul}x1o"
+    s = "+".join(f"{mul}x{l}{'eo'[l % 2]}" for l in range(lmax + 1))  # noqa: E741
     m = cb.FullyConnectedTensorProduct(s, s, s, layout=cb.ir_mul, internal_weights=False, shared_weights=True)
     prog = m.f._program(torch.float32)
     assert prog._tri_channels(torch.float32) == mul
