@@ -83,8 +83,10 @@ template <typename T>
 int launch(const void* x, void* y, int64_t rows, int64_t dim, const int32_t* info, int nb, cudaStream_t st) {
   const size_t smem = (size_t)dim * sizeof(T);
   if (smem > 200 * 1024) return cueq::fail("segmented_transpose: row of %lld elements does not fit shared memory", (long long)dim);
-  // rows in whole groups of four elements, at the alignment of a group
-  if (dim % 4 == 0 && (((uintptr_t)x | (uintptr_t)y) % (4 * sizeof(T))) == 0 && smem <= 24 * 1024) {
+  // Rows in whole groups of four elements, at the alignment of a group.  float64 only up to 6 KB: beyond, the gather of four
+  // doubles per thread conflicts in shared memory and few warps hold their rows; 16 M elements in rows of 576 / 1,152 / 2,304:
+  // 77 / 64 / 61 us by the kernel with a block per row, 63 / 73 / 75 us by this one (float32 72 / 58 / 52 and 28 / 32 / 37 us).
+  if (dim % 4 == 0 && (((uintptr_t)x | (uintptr_t)y) % (4 * sizeof(T))) == 0 && smem <= (sizeof(T) == 8 ? 6 : 24) * 1024) {
     int warps = 8;
     while (warps > 1 && warps * smem > 48 * 1024) warps /= 2;
     const unsigned grid = (unsigned)std::min<int64_t>((rows + warps - 1) / warps, 148 * 32);
