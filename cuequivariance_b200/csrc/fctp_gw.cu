@@ -256,7 +256,10 @@ __global__ void __launch_bounds__(kThreads, 1) fctp_gw_kernel(const __grid_const
           float v[8];
 #pragma unroll
           for (int q = 0; q < 8; ++q) v[q] = __uint_as_float(h[q]) + __uint_as_float(l[q]);
-          if (p.parts) {
+          if (p.parts && t.st == 1) {
+#pragma unroll
+            for (int q = 0; q < 8; q += 4) *reinterpret_cast<float4*>(dst + c + q) = make_float4(v[q], v[q + 1], v[q + 2], v[q + 3]);
+          } else if (p.parts) {
 #pragma unroll
             for (int q = 0; q < 8; ++q) dst[(int64_t)(c + q) * t.st] = v[q];
           } else if (t.st == 1) {
