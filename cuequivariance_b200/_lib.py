@@ -315,6 +315,7 @@ def lib() -> C.CDLL:
     L.cueq_b200_gemm_f32x3.argtypes = [C.POINTER(GemmF32x3Args), C.c_void_p]
     L.cueq_b200_gemm_f32x3_tn.argtypes = [C.POINTER(GemmF32x3TnArgs), C.c_void_p]
     L.cueq_b200_fctp_tri.argtypes = [C.POINTER(FctpTriArgs), C.c_void_p]
+    L.cueq_b200_fctp_tri_sum.argtypes = [C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_int, C.c_void_p, C.c_void_p]
     L.cueq_b200_fctp_tri_ready.argtypes = [C.c_int, C.c_int]
     L.cueq_b200_fctp_tri_weights.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int, C.POINTER(C.c_int32), C.POINTER(C.c_int32),
                                              C.c_void_p, C.c_void_p, C.c_void_p]

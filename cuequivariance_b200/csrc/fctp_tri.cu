@@ -332,20 +332,18 @@ __global__ void __launch_bounds__(kThreads, 1) fctp_tri_kernel(const __grid_cons
 }
 
 // The divisions of a sum, added in their order: the result does not depend on which thread block was faster.  Bound by memory
-// (a read of every partial result); added by red.global.add into the result instead, the last bits changed from call to call.
-// A block holds 256 / cols whole rows.
-__global__ void __launch_bounds__(256) fctp_tri_sum_kernel(const float4* __restrict__ parts, float* __restrict__ out, int64_t rows, int cols, int splits,
-                                                           int64_t ldo, const int* status) {
-  const int per = blockDim.x / cols, r = threadIdx.x / cols, c = threadIdx.x - r * cols;
-  if (r >= per || !status_clean(status)) return;                      // after a wait that ran out the parts are incomplete
-  for (int64_t z = (int64_t)blockIdx.x * per + r; z < rows; z += (int64_t)gridDim.x * per) {
-    const float4* src = parts + z * cols + c;
-    float4 v = __ldcs(src);
+// (a read of every partial result).  Added by red.global.add into the result instead, the last bits changed from call to call.
+__global__ void __launch_bounds__(256) fctp_tri_sum_kernel(const float4* __restrict__ parts, float4* __restrict__ out, int64_t n, int splits,
+                                                           const int* status) {
+  if (!status_clean(status)) return;                                  // after a wait that ran out the parts are incomplete
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    float4 v = __ldcs(parts + i);
+#pragma unroll 4
     for (int s = 1; s < splits; ++s) {
-      const float4 a = __ldcs(src + s * rows * cols);
+      const float4 a = __ldcs(parts + s * n + i);
       v.x += a.x; v.y += a.y; v.z += a.z; v.w += a.w;
     }
-    *reinterpret_cast<float4*>(out + z * ldo + 4 * c) = v;
+    out[i] = v;
   }
 }
 
@@ -466,27 +464,17 @@ int launch(const cueq_fctp_tri_args* a, TriParams& p, cudaStream_t st) {
   CUtensorMap hi, lo;
   if (int rc = make_map(&hi, BF16, a->b_hi, a->b_rows, C, K::NT)) return rc;
   if (int rc = make_map(&lo, BF16, BF16 ? a->b_hi : a->b_lo, a->b_rows, C, K::NT)) return rc;
-  float* const out = p.out + p.out_off;
-  const int64_t ldo = p.ldo;
   if (p.splits > 1) {
     if (!a->parts) return cueq::fail("fctp tri: a divided sum needs room for its partial results");
     p.out = (float*)a->parts;
-    p.out_off = 0;
-    p.ldo = (int64_t)a->nc * C;
     p.part = p.ldo * p.batch;
   }
-  int rc;
   switch (a->nc) {
-    case 1: rc = launch_c<BF16, C, 1>(hi, lo, p, st); break;
-    case 3: rc = launch_c<BF16, C, 3>(hi, lo, p, st); break;
-    case 5: rc = launch_c<BF16, C, 5>(hi, lo, p, st); break;
+    case 1: return launch_c<BF16, C, 1>(hi, lo, p, st);
+    case 3: return launch_c<BF16, C, 3>(hi, lo, p, st);
+    case 5: return launch_c<BF16, C, 5>(hi, lo, p, st);
     default: return cueq::fail("fctp tri: irreps of dimension 1, 3 or 5 only");
   }
-  if (rc || p.splits == 1) return rc;
-  const int cols = (int)(p.ldo / 4), per = 256 / cols, blocks = (p.batch + per - 1) / per;
-  fctp_tri_sum_kernel<<<blocks < 148 * 16 ? blocks : 148 * 16, 256, 0, st>>>((const float4*)a->parts, out, p.batch, cols, p.splits, ldo, p.status);
-  CUEQ_CUDA_OK(cudaGetLastError());
-  return 0;
 }
 
 }  // namespace
@@ -542,6 +530,17 @@ extern "C" int cueq_b200_fctp_tri(const cueq_fctp_tri_args* a, void* stream) {
     if (C == 64) return launch<false, 64>(a, p, st);
   }
   return cueq::fail("fctp tri: %d channels are not covered", C);
+}
+
+extern "C" int cueq_b200_fctp_tri_sum(const void* parts, void* out, int64_t batch, int64_t ldo, int splits, const void* status, void* stream) {
+  if (!parts || !out) return cueq::fail("fctp tri: null operand");
+  if (batch < 0 || ldo < 4 || ldo % 4 || splits < 1 || ((uintptr_t)parts | (uintptr_t)out) & 15) return cueq::fail("fctp tri: rows must be 16-byte aligned");
+  if (batch == 0) return 0;
+  const int64_t n = batch * ldo / 4, blocks = (n + 255) / 256;
+  fctp_tri_sum_kernel<<<(unsigned)(blocks < 148 * 16 ? blocks : 148 * 16), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+      (const float4*)parts, (float4*)out, n, splits, (const int*)status);
+  CUEQ_CUDA_OK(cudaGetLastError());
+  return 0;
 }
 
 extern "C" int cueq_b200_fctp_tri_weights(const void* w, int w_dtype, int dtype, int channels, int num_paths, const int32_t* w_off, const int32_t* order,

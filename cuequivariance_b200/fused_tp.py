@@ -403,7 +403,8 @@ class DenseUVW:
             tiles = -(-step // 128) * (c // rt)
             splits = self._tri_splits(tiles, c)
             out = (torch.empty if full else torch.zeros)((B, size), dtype=torch.float32, device=dev)
-            parts = torch.empty(splits * step * c * max(t[1] for t in launches), dtype=torch.float32, device=dev) if splits > 1 else None
+            # partial results of a divided sum; columns of an irrep without a path are never written
+            parts = (torch.empty if full else torch.zeros)(splits * step * size, dtype=torch.float32, device=dev) if splits > 1 else None
             for b0 in range(0, B, step):
                 nb = min(step, B - b0)
                 zp = -(-nb // 128) * 128
@@ -429,6 +430,9 @@ class DenseUVW:
                     a.paths = C.cast(paths, C.POINTER(_lib.FctpTriPath))
                     with profiling.kernel(name):
                         _lib.check(L.cueq_b200_fctp_tri(C.byref(a), stream))
+                if splits > 1:
+                    with profiling.kernel("fctp_tri_sum"):
+                        _lib.check(L.cueq_b200_fctp_tri_sum(a.parts, a.out, nb, size, splits, a.status, stream))
         return out
 
     def _tri_gw_paths(self):

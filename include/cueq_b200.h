@@ -351,8 +351,9 @@ int cueq_b200_gemm_f32x3_tn(const cueq_gemm_f32x3_tn_args* args, void* stream);
  *   R[z, c, r] (+)= sum over paths, p, q, a, b of coef[a][b][c] W[p, q, r] P[z, a, p] Q[z, b, q]
  * All multiplicities are `channels` (32, 64 in float32; 128 in bf16), irreps have dimension 1, 3 or 5.  P rows come
  * as they are (ir_mul), Q transposed ([column][sample], cueq_b200_fctp_tri_transpose), the weights as rows ((q, r), p)
- * (cueq_b200_fctp_tri_weights; row block k * channels^2 belongs to path k).  With splits > 1 the sum over q is divided among that
- * many thread blocks, whose partial results are added in a fixed order.  The columns of the irrep are overwritten. */
+ * (cueq_b200_fctp_tri_weights; row block k * channels^2 belongs to path k).  The columns of the irrep are overwritten.
+ * With splits > 1 the sum over q is divided among that many thread blocks and their results go to `parts`; when all irreps are
+ * done, cueq_b200_fctp_tri_sum adds them in a fixed order. */
 #define CUEQ_FCTP_TRI_MAX_PATHS 24
 typedef struct {
   int32_t a_src, a_off, na;   /* P: operand 0 or 1, its first column, its components                */
@@ -366,7 +367,7 @@ typedef struct {
   const void* b_hi;     /* device [b_rows, channels]: TF32 halves (float32) or bf16                */
   const void* b_lo;
   void* out;            /* device float32 [batch, ldo]                                             */
-  void* parts;          /* splits > 1: device float32 [splits, batch, nc * channels], 16-byte aligned, overwritten */
+  void* parts;          /* splits > 1: device float32 [splits, batch, ldo], 16-byte aligned, instead of `out` */
   const cueq_fctp_tri_path* paths;   /* host                                                       */
   void* status;         /* nullable device int32: 2 if a bounded wait ran out                      */
   int64_t lda[2], zp, b_rows, ldo, batch;
@@ -378,6 +379,8 @@ int cueq_b200_fctp_tri(const cueq_fctp_tri_args* args, void* stream);
 /* 1: the kernels for this type and multiplicity are there and were compiled to the registers that their division among the
  * warps counts on; 0: not (cueq_b200_fctp_tri refuses the call); -1: cannot be told without a device */
 int cueq_b200_fctp_tri_ready(int dtype, int channels);
+/* out [batch, ldo] = sum of parts [splits, batch, ldo] */
+int cueq_b200_fctp_tri_sum(const void* parts, void* out, int64_t batch, int64_t ldo, int splits, const void* status, void* stream);
 /* order[k] = 100 * (axis of p) + 10 * (axis of q) + (axis of r), axes of W[u][v][w]: 0, 1, 2; w_off in elements */
 int cueq_b200_fctp_tri_weights(const void* w, int w_dtype, int dtype, int channels, int num_paths, const int32_t* w_off,
                                const int32_t* order, void* hi, void* lo, void* stream);
