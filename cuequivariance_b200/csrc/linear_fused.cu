@@ -567,9 +567,9 @@ __global__ void __launch_bounds__(128) linear_gw_sum_kernel(const __grid_constan
   const int s = blockIdx.y, cls = s % p.num_classes;
   const LPath& q = p.path[s / p.num_classes];
   const int e = (blockIdx.x * 128 + threadIdx.x) * 4;
-  if (t.start[s] == t.start[s + 1] || e >= q.K * q.N || !status_clean(p.status)) return;
+  if (e >= q.K * q.N || !status_clean(p.status)) return;
   auto block_of = [&](int64_t item) { return (int)(((item + 1) * blocks + p.total - 1) / p.total) - 1; };
-  const int b0 = block_of(t.start[s]), n = block_of(t.start[s + 1] - 1) - b0 + 1;
+  const int b0 = block_of(t.start[s]), n = t.start[s] == t.start[s + 1] ? 0 : block_of(t.start[s + 1] - 1) - b0 + 1;   // 0: a class without rows
   const float* src = p.parts + (int64_t)(b0 + s) * p.slot + e;
   float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 8
@@ -577,10 +577,7 @@ __global__ void __launch_bounds__(128) linear_gw_sum_kernel(const __grid_constan
     const float4 a = __ldcs(reinterpret_cast<const float4*>(src + k * p.slot));
     v.x += a.x; v.y += a.y; v.z += a.z; v.w += a.w;
   }
-  float4* dst = reinterpret_cast<float4*>(p.out + cls * p.w_class_stride + q.w_off + e);
-  float4 o = *dst;
-  o.x += q.c * v.x; o.y += q.c * v.y; o.z += q.c * v.z; o.w += q.c * v.w;
-  *dst = o;
+  *reinterpret_cast<float4*>(p.out + cls * p.w_class_stride + q.w_off + e) = make_float4(q.c * v.x, q.c * v.y, q.c * v.z, q.c * v.w);
 }
 
 // Checks the arguments and fills the kernel parameters; `per_item` = nodes per tile or K block.  Returns the status.

@@ -224,7 +224,8 @@ class _FusedLinear(torch.autograd.Function):
             gx = (torch.empty_like if plan["full_in"] and ctx.all_rows else torch.zeros_like)(x)
             _FusedLinear._launch(plan, "map", bounds, gout, weight, gx, transposed=1)
         if ctx.needs_input_grad[2]:
-            gw = torch.zeros_like(weight)
+            # the weights are the blocks of the paths, all of them written; without any row nothing is
+            gw = (torch.empty_like if bounds[-1] > bounds[0] else torch.zeros_like)(weight)
             _FusedLinear._launch(plan, "gw", bounds, x, gout, gw)
         return None, None, gw, gx
 

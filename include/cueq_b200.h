@@ -424,7 +424,7 @@ int cueq_b200_fctp_gw(const cueq_fctp_gw_args* args, void* stream);
  * weights at w + k * w_class_stride.
  * linear_map: out[z, v, i] = c * sum_u W[u, v] x[z, u, i]; with `transposed` the input gradient: `x` holds the cotangent
  *   rows (addressed by out_off), `out` the gradient rows (addressed by x_off).
- * linear_gw:  out (the weight gradient, zeroed by the caller) [u, v] += c * sum_{z, i} x[z, u, i] g[z, v, i]; `w` = g.  The
+ * linear_gw:  out (the weight gradient) [u, v] = c * sum_{z, i} x[z, u, i] g[z, v, i], zeros for a class without rows; `w` = g.  The
  *   partial sums of its thread blocks go to `parts` (cueq_b200_linear_gw_floats(args) floats) and are added in a fixed order. */
 #define CUEQ_LINEAR_MAX_PATHS 8
 #define CUEQ_LINEAR_MAX_CLASSES 64
