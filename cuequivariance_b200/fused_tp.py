@@ -159,7 +159,7 @@ class _TensorCoreUVW(torch.autograd.Function):
             w16 = owner._weights_bf16(w, False)
             out = owner._fused_forward(w16, x1, x2, status)
             ctx.owner, ctx.status = owner, status
-            ctx.save_for_backward(w, x1, x2, w16)
+            ctx.save_for_backward(w, x1, x2, *(() if w.dtype == torch.bfloat16 else (w16,)))
             return out.to(x1.dtype)
         x1c, x2c = owner._as_kernel_input(x1), owner._as_kernel_input(x2)
         out = torch.zeros((B, owner.out_size), dtype=torch.float32, device=dev)
@@ -278,8 +278,8 @@ class DenseUVW:
         """The shared weights as bf16 rows of 64, in ``[u][v][w]`` order or (``transposed``) ``[v][u][w]``.  Made once per pass
         (the backward pass gets the forward's copy): neither an address nor a version counter tells that the values are
         still those of an earlier call."""
-        t = w.detach().to(torch.bfloat16).reshape(-1, 64, 64, 64)
-        return (t.transpose(1, 2) if transposed else t).reshape(-1, 64).contiguous()
+        t = w.detach().to(torch.bfloat16)
+        return (t.reshape(-1, 64, 64, 64).transpose(1, 2) if transposed else t).reshape(-1, 64)
 
     # -- tensor-core route ---------------------------------------------------------------------
     def _tc_applicable(self, w, x1, x2) -> bool:
