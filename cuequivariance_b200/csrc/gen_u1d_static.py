@@ -10,10 +10,10 @@ that most of its terms share is taken out, its cofactor and the remainder are tr
 way, down to sums of ``coefficient * segment`` or ``coefficient * shared product``, one multiply-add
 per term.  Factors are taken from the buffers that occur once in a term first (cotangent and weight,
 the one with fewer segments first) and from the repeated buffer last, which leaves its products as
-the innermost terms.  These bodies are bound by the FP32 issue rate, so the count of instructions is
-the time; for 0e+1o+2e+3o -> 0e+1o of degree 3, against one product and one multiply-add per term
-and a factored first operand only: forward 1089 -> 747, weight gradient 1155 -> 747, feature gradient
-2664 -> 1786 instructions.
+the innermost terms.  A body runs straight through once, so its time goes with its instructions and with the loads that
+nothing but other warps overlaps (47-64 % of the issue slots are used); for 0e+1o+2e+3o -> 0e+1o of degree 3, against one
+product and one multiply-add per term and a factored first operand only: forward 1089 -> 747, weight gradient 1155 -> 747,
+feature gradient 2664 -> 1786 instructions.
 
     python cuequivariance_b200/csrc/gen_u1d_static.py
 """

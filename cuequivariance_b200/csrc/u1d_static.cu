@@ -40,9 +40,11 @@ __host__ __device__ constexpr int block_of(int s) { return s < 1 ? 0 : s < 4 ? 1
 // reads cover whole lines (the lines stay in L1 between the block's components); a block of an output goes through
 // shared memory, so that every store of a warp is 128 contiguous bytes: stored component by component, each 32-byte
 // sector would be written 2l+1 times.  A separate transposition of the rows in and out cost as much as the smaller
-// kernels themselves: a read and a write of every feature, output and both their gradients.  Bound by the FP32 issue
-// rate: 16,384 atoms x 128 channels of 0e+1o+2e+3o -> 0e+1o, degree 3, forward 93 us, weight gradient 109 us, feature
-// gradient 267 us; the step 470 us, with transposed copies and without the factored sums (gen_u1d_static.py) 820 us.
+// kernels themselves: a read and a write of every feature, output and both their gradients.  No pipe
+// bounds the kernels: 8 to 20 warps per SM (registers) wait for loads that a body makes once and nothing else overlaps, and
+// use 47-64 % of the issue slots, 2.1-2.5 times the time of their instructions.  16,384 atoms x 128 channels of
+// 0e+1o+2e+3o -> 0e+1o, degree 3: forward 93 us, weight gradient 109 us, feature gradient 267 us; the step 470 us, with
+// transposed copies and without the factored sums (gen_u1d_static.py) 820 us.
 template <class K>
 __global__ void __launch_bounds__(128) u1d_static_kernel(const __grid_constant__ StaticParams P) {
   __shared__ float staging[4][32 * (2 * kMaxL + 1)];
