@@ -324,11 +324,11 @@ class StaticKernel:
 
 
 # One launch per gradient instead of one for all, where each gradient has a build-time kernel: for polynomials of more
-# than this many paths on more than this many (row, channel) pairs.  The two gradients of the largest symmetric
-# contraction (0e+1o+2e+3o -> 0e+1o, degree 3: 4,078 paths) take 209 registers together: 404 us against 269 + 110 us at
-# 16,384 x 128.  Smaller polynomials fit (the next one needs 80), and on few rows the launch itself is the time
-# (213 x 64: 288 us against 390 us per step).
-SPLIT_STATIC_PATHS, SPLIT_STATIC_ROWS = 1000, 1 << 18
+# than this many paths on at least this many (row, channel) pairs.  The two gradients of the largest symmetric
+# contraction (0e+1o+2e+3o -> 0e+1o, degree 3: 4,078 paths) take 209 registers together.  Forward and backward, together
+# against one by one: 16,384 atoms x 128 channels 502 / 473 us, 10,240 x 128 319 / 305, 16,384 x 64 256 / 265, 8,192 x 64 216 /
+# 262, 213 x 64 219 / 263 (there the launch itself is the time).  Smaller polynomials fit (the next one needs 80).
+SPLIT_STATIC_PATHS, SPLIT_STATIC_ROWS = 1000, 5 << 18
 
 
 def attach_static(program: "Uniform1dProgram") -> None:
