@@ -14,9 +14,13 @@ const GroupEntry* const kGroups[] = {&kGroupL0, &kGroupL1, &kGroupL2, &kGroupL3}
 const GroupEntry64* const kGroups64[] = {&kGroupL0F64, &kGroupL1F64, &kGroupL2F64, &kGroupL3F64};
 constexpr int kNumGroups = sizeof(kGroups) / sizeof(kGroups[0]);
 
-int pick_cpl(const cueq_cw_args* a) {
+// Channels per thread of the kernels with a warp per receiver.  Four hold up to 132 accumulators per thread and spill; with
+// two a warp has 64 channels, which is all there are where this matters.  Path subsets take two: 40,000 edges, 4 channels,
+// lmax 2, forward, 20 edges per receiver 152 -> 83 us (117 us on the table-driven kernel they came from), one edge 171 -> 84
+// us (258).  Whole groups of fewer than 64 channels keep four.
+int pick_cpl(const cueq_cw_args* a, bool masked) {
   if (a->channels_per_lane == 2 || a->channels_per_lane == 4) return a->channels_per_lane;
-  return a->extent >= 64 ? 2 : 4;
+  return masked || a->extent >= 64 ? 2 : 4;
 }
 
 // A polynomial with all paths of the group and 16-element x2 rows takes the kernels that know so at compile time and copy a
@@ -104,8 +108,8 @@ int run_forward(int g, const cueq_cw_args* a, const cueq_cw_options& o, int over
   p.status = reinterpret_cast<int*>(a->status);
   if (a->variant < 0 || a->variant > 2) return cueq::fail("channelwise: variant must be 0 (automatic), 1 or 2");
   const bool masked = is_masked(p, *kGroups[g]);
-  if (a->staging == 1 && !masked) return kGroups[g]->fwd_bulk(p, a->x1_mul_ir, pick_cpl(a), reinterpret_cast<cudaStream_t>(stream));
-  return kGroups[g]->fwd(p, a->x1_mul_ir, pick_cpl(a), masked, reinterpret_cast<cudaStream_t>(stream));
+  if (a->staging == 1 && !masked) return kGroups[g]->fwd_bulk(p, a->x1_mul_ir, pick_cpl(a, false), reinterpret_cast<cudaStream_t>(stream));
+  return kGroups[g]->fwd(p, a->x1_mul_ir, pick_cpl(a, masked), masked, reinterpret_cast<cudaStream_t>(stream));
 }
 
 int run_backward(int g, const cueq_cw_args* a, const cueq_cw_options& o, int overlap, void* stream) {
@@ -137,7 +141,10 @@ int run_backward(int g, const cueq_cw_args* a, const cueq_cw_options& o, int ove
   // and few edges per receiver the cotangent row is staged by a block for too little work; 100,000 edges, lmax 3, one warp
   // against one block per receiver: 64 channels, 20 edges 680 / 536 us, 5 edges 720 / 757 us; 32 channels, 5 edges
   // 1371 / 687 us; 2,000 edges on 100 receivers, 64 channels: 153 / 51 us.
-  const bool few = o.mean_degree > 0 && o.mean_degree < 8 && a->extent > 32 && a->extent % 128;
+  // Up to 32 channels the same holds for receivers of one edge (calls without a receiver index among them) only; 50,000 edges,
+  // lmax 2 x 3 -> 3, warp against block: 32 channels, one edge 804 / 972 us, two 645 / 644 us, four 568 / 479 us; 4 channels,
+  // one edge 675 / 853 us.
+  const bool few = o.mean_degree > 0 && o.mean_degree < (a->extent > 32 ? 8 : 2) && a->extent % 128;
   const bool masked = is_masked(p, *kGroups[g]);
   const bool block_per_receiver = a->variant >= 2 || (a->variant == 0 && a->channels_per_lane != 2 && !few);
   if (a->variant == 3 && a->extent % 128) return cueq::fail("channelwise backward: variant 3 needs a multiple of 128 channels");
@@ -146,7 +153,7 @@ int run_backward(int g, const cueq_cw_args* a, const cueq_cw_options& o, int ove
   const bool bulk = a->variant == 3 || (a->variant == 0 && kGroups[g]->d1 >= 3);
   if (block_per_receiver)
     return kGroups[g]->bwd_block(p, coef, a->x1_mul_ir, a->variant >= 2 || a->extent % 128 == 0 ? 4 : 2, bulk, masked, reinterpret_cast<cudaStream_t>(stream));
-  return kGroups[g]->bwd(p, coef, a->x1_mul_ir, pick_cpl(a), masked, reinterpret_cast<cudaStream_t>(stream));
+  return kGroups[g]->bwd(p, coef, a->x1_mul_ir, pick_cpl(a, masked), masked, reinterpret_cast<cudaStream_t>(stream));
 }
 
 }  // namespace
@@ -297,5 +304,5 @@ extern "C" int cueq_b200_cw_forward_noalloc(int g, const cueq_cw_noalloc_args* a
   cw_noalloc_prepare<<<blocks < 1 ? 1 : blocks, 256, 0, st>>>(a->receivers, (int)a->num_edges, (int)a->num_receivers, rowptr, t, ge.nval,
                                                               ge.nterm_fwd, tab_start, tab_j, tab_c);
   CUEQ_CUDA_OK(cudaGetLastError());
-  return ge.fwd(p, a->mul_ir, pick_cpl(&full), is_masked(p, ge), st);
+  return ge.fwd(p, a->mul_ir, pick_cpl(&full, is_masked(p, ge)), is_masked(p, ge), st);
 }
