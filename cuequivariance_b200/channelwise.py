@@ -204,6 +204,8 @@ class ChannelwisePlan:
         self.x1_blocks = x1_blocks          # ((mul, dim), ...) of x1
         self.out_blocks = out_blocks
         self.complete = all(g["mask"] == (1 << g["npath"]) - 1 for g in groups)   # whole groups of the library
+        # what a call's time depends on besides its edges: paths of the groups (scalars' are cheap), paths of the product, terms
+        self.work = (sum(g["npath"] * (1.0 if g["l1"] else 0.4) for g in groups), sum(len(g["out_segs"]) for g in groups), sum(c != 0 for g in groups for c in g["bwd_tab"][2]))
         self._dev: dict = {}
         self._templates: dict = {}          # constant launch arguments, see _ChannelwiseBase._run_groups
 
@@ -392,6 +394,37 @@ class _ChannelwiseBase:
                     _IDENTITY_ROWPTR[key] = rp
             return None, rp, batch
         return None
+
+    def _generic_is_faster(self, program, edges: int, receivers: int, backward: bool) -> bool:
+        """Few channels of float64, or four of float32 in a sparse subset of the groups' paths: these kernels spend their time
+        on what does not depend on the channels (the matrices of whole groups, staging, warps of which a few lanes work).
+
+        The lines are fitted to 385 forward and 745 backward pairs of times (products lmax 1 x 1 -> 1 to 3 x 3 -> 3, 2 to 32
+        channels, one to forty edges per receiver).  Of N paths in the groups (those of the scalars, which are cheap, count
+        0.4) the product has P, with T terms; d edges per receiver; ns per edge here against there:
+          float64 forward   (0.066 N + 0.056 P) (1 + 1.55 / d)   against  0.057 P (1 + 2.75 / d) + 0.0044 T channels
+          float64 backward  (0.193 N + 0.097 P) (1 + 4.8 / d)    against  0.121 P (1 + 3.27 / d) + 0.0172 T channels
+          float32 forward   (0.027 N + 0.0125 P) (1 + 3.7 / d),  backward  (0.139 N + 0.060 P) (1 + 1.26 / d)
+        200,000 edges, lmax 3 x 1 -> 1, eight edges per receiver, here against the generic kernel, us: float64, 4 channels,
+        forward 319 / 136, with all gradients 1035 / 457; 8 channels 326 / 229, 1084 / 772; 16 channels 1113 / 1389; float32, 4
+        channels 196 / 125, 584 / 401.  What takes no longer than the host does stays here, and whole groups of float32
+        always do."""
+        import torch
+
+        plan = self.plan
+        if not edges or not receivers or plan.extent > 32:
+            return False
+        n, p, t = plan.work
+        d = edges / receivers
+        if program.math_dtype == torch.float64:
+            if backward:
+                here, there, host = (0.193 * n + 0.097 * p) * (1 + 4.8 / d), 0.121 * p * (1 + 3.27 / d) + 0.0172 * t * plan.extent, 234e3
+            else:
+                here, there, host = (0.066 * n + 0.056 * p) * (1 + 1.55 / d), 0.057 * p * (1 + 2.75 / d) + 0.0044 * t * plan.extent, 80e3
+            return edges * here > host and here > 0.9 * there
+        if plan.complete or plan.extent > 4 or p >= 0.6 * n:
+            return False
+        return edges * (0.139 * n + 0.060 * p) * (1 + 1.26 / d) > 300e3 if backward else edges * (0.027 * n + 0.0125 * p) * (1 + 3.7 / d) > 70e3
 
     def _args(self, g, tabs, which, common, order, rowptr, nrecv, out_mul_ir, tensors, x1_is_block=False):
         """``x1_is_block``: tensors['x1'] (and 'gx1') hold only this group's irrep block,
@@ -598,7 +631,7 @@ class ChannelwiseForward(_ChannelwiseBase):
         if common is None:
             return None
         csr = self._csr(cfg.outputs[0], cfg.batch, xs[0].device)
-        if csr is None:
+        if csr is None or self._generic_is_faster(program, cfg.batch, csr[2], False):
             return None
         return [self._launch_forward(common, csr, common["x1_mul_ir"], *xs)]
 
@@ -621,7 +654,7 @@ class ChannelwiseBackward(_ChannelwiseBase):
         if common is None:
             return None
         csr = self._csr(cfg.inputs[3], cfg.batch, xs[0].device)
-        if csr is None:
+        if csr is None or self._generic_is_faster(program, cfg.batch, csr[2], True):
             return None
         for k, i in grad_specs:  # gradient layouts and addressing must mirror their inputs
             if cfg.layout(n_in + k) != cfg.layout(i) or cfg.outputs[k].mode != cfg.inputs[i].mode:
