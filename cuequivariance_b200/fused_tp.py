@@ -300,7 +300,8 @@ class DenseUVW:
         # bf16 with 64 channels has kernels of its own (fctp_fused.cu), which are faster: 5.4 against 6.2 ms for the output
         # and both input gradients of 32,768 samples of 64x(0e+1o+2e).  Other shapes used to write the coupled operand to
         # memory: the same sums in float32 took 23 ms, 10 ms here.  float32 with 96 channels stays there: chains of twelve
-        # additions in the tensor core, input gradients 3.8e-7 off where the memory route is 2.5e-7 off.
+        # additions in the tensor core, input gradients 3.8e-7 off where the memory route is 2.5e-7 off (the memory route's output
+        # is 6.3e-5 off with three irreps, in one chain per output component over all (u, v) of its paths).
         if c not in ((128,) if dtype == torch.bfloat16 else (32, 64)):
             return 0
         if dtype not in self._tri_ready:     # 0: a build whose kernels did not come out as they have to
