@@ -159,7 +159,7 @@ class _TensorCoreUVW(torch.autograd.Function):
             w16 = owner._weights_bf16(w, False)
             out = owner._fused_forward(w16, x1, x2, status)
             ctx.owner, ctx.status = owner, status
-            ctx.save_for_backward(w, x1, x2, *(() if w.dtype == torch.bfloat16 else (w16,)))
+            ctx.save_for_backward(w, x1, x2, *(() if w16 is w else (w16,)))
             return out.to(x1.dtype)
         x1c, x2c = owner._as_kernel_input(x1), owner._as_kernel_input(x2)
         out = torch.zeros((B, owner.out_size), dtype=torch.float32, device=dev)
@@ -275,11 +275,12 @@ class DenseUVW:
 
     @staticmethod
     def _weights_bf16(w: torch.Tensor, transposed: bool) -> torch.Tensor:
-        """The shared weights as bf16 rows of 64, in ``[u][v][w]`` order or (``transposed``) ``[v][u][w]``.  Made once per pass
+        """The shared weights in bf16, contiguous, in ``[u][v][w]`` order or (``transposed``) ``[v][u][w]``.  Made once per pass
         (the backward pass gets the forward's copy): neither an address nor a version counter tells that the values are
         still those of an earlier call."""
-        t = w.detach().to(torch.bfloat16)
-        return (t.reshape(-1, 64, 64, 64).transpose(1, 2) if transposed else t).reshape(-1, 64)
+        if w.dtype != torch.bfloat16 or not w.is_contiguous():
+            w = w.detach().to(torch.bfloat16).contiguous()
+        return w.view(-1, 64, 64, 64).transpose(1, 2).contiguous() if transposed else w
 
     # -- tensor-core route ---------------------------------------------------------------------
     def _tc_applicable(self, w, x1, x2) -> bool:
@@ -571,7 +572,7 @@ class DenseUVW:
         gxa = torch.zeros((B, xb.shape[1]), dtype=torch.float32, device=xb.device)
         a = _lib.FctpFusedGxArgs()
         a.xb, a.gout, a.w, a.gxa = xb.data_ptr(), gout16.data_ptr(), w16.data_ptr(), gxa.data_ptr()
-        a.ldb, a.ldg, a.lda, a.batch, a.w_rows = xb.shape[1], gout16.shape[1], gxa.shape[1], B, w16.shape[0]
+        a.ldb, a.ldg, a.lda, a.batch, a.w_rows = xb.shape[1], gout16.shape[1], gxa.shape[1], B, w16.numel() // 64
         a.num_units = len(units)
         a.units = C.cast(units, C.POINTER(_lib.FctpFusedUnit))
         a.status = status.data_ptr()
@@ -626,7 +627,7 @@ class DenseUVW:
         out = torch.empty((B, self.out_size), dtype=torch.float32, device=x1.device)
         a = _lib.FctpFusedArgs()
         a.x1, a.x2, a.w, a.out = x1c.data_ptr(), x2c.data_ptr(), w16.data_ptr(), out.data_ptr()
-        a.ld1, a.ld2, a.ldo, a.batch, a.w_rows = x1c.shape[1], x2c.shape[1], out.shape[1], B, w16.shape[0]
+        a.ld1, a.ld2, a.ldo, a.batch, a.w_rows = x1c.shape[1], x2c.shape[1], out.shape[1], B, w16.numel() // 64
         a.out_dtype, a.num_tasks = _lib.F32, len(tasks)
         a.tasks = C.cast(tasks, C.POINTER(_lib.FctpFusedTask))
         a.status = status.data_ptr()

@@ -21,10 +21,13 @@ def test_bf16_weights_follow_the_values():
         for transposed in (False, True):
             t = w.view(-1, 64, 64, 64)
             want = (t.transpose(1, 2) if transposed else t).reshape(-1, 64).to(torch.bfloat16)
-            assert torch.equal(prog._weights_bf16(w, transposed), want)
+            assert torch.equal(prog._weights_bf16(w, transposed).reshape(-1, 64), want)
         version = w._version
         w.data.mul_(-0.5)
         assert w._version == version
+    b = w.to(torch.bfloat16)
+    assert prog._weights_bf16(b, False) is b
+    assert torch.equal(prog._weights_bf16(b, True).reshape(-1, 64), b.view(-1, 64, 64, 64).transpose(1, 2).reshape(-1, 64))
 
 
 class _Owner:
