@@ -11,6 +11,10 @@ namespace cw {
 constexpr int kMaxPaths = 8;
 constexpr int kMaxTerms = 160;
 
+// A launch by itself; the first of a chain of groups that overlap, or one that waits for all before it; one that may start
+// while the group before it, in the chain too, still runs.
+enum { kAlone = 0, kStarts = 1, kFollows = 2 };
+
 template <class T>
 struct CwCoefT {
   T c[kMaxTerms];
@@ -44,7 +48,7 @@ struct CwParamsT {
   int recv_mod;             // backward: CSR rows are (pass, receiver) pairs; the cotangent row is row % recv_mod (0: off)
   unsigned path_mask;       // bit q: path q of the group belongs to the polynomial (MASKED kernels)
   int nx2;                  // components of an x2 row (MASKED kernels; 16 otherwise)
-  int overlap;              // launch: may start while the kernel before it in the stream, a group of the same call, still runs
+  int overlap;              // launch: kAlone, kStarts or kFollows
 };
 using CwParams = CwParamsT<float>;
 

@@ -342,9 +342,11 @@ struct StoreOut {
 
 template <class T> constexpr int kFwdMinBlocks = sizeof(T) == 8 ? 2 : CW_MINBLOCKS;
 
-template <class T, class G, int C, bool MUL_IR, bool MASKED>
+// OVERLAP: part of a chain of overlapping launches (launch_kernel).  The two instructions cost the l >= 1 kernels 5 % - two
+// registers at their limit of 128, a spill and 7 % more instructions - so a launch that gains nothing from it goes without.
+template <class T, class G, int C, bool MUL_IR, bool MASKED, bool OVERLAP>
 __global__ void __launch_bounds__(kWarps * 32, kFwdMinBlocks<T>) cw_fwd_kernel(const __grid_constant__ CwParamsT<T> p) {
-  let_next_start();
+  if constexpr (OVERLAP) let_next_start();
   extern __shared__ __align__(16) unsigned char smem_bytes[];
   T* smem = reinterpret_cast<T*>(smem_bytes);
   using S = Smem<G, C, T>;
@@ -391,7 +393,7 @@ __global__ void __launch_bounds__(kWarps * 32, kFwdMinBlocks<T>) cw_fwd_kernel(c
     }
     if (active) StoreOut<G, C, 0, MUL_IR, MASKED, T>::run(p.out + (int64_t)n * p.out_stride, p, ch, acc);
   }
-  wait_for_previous();
+  if constexpr (OVERLAP) wait_for_previous();
 }
 
 // ---- forward, staging by bulk copies ----------------------------------------------------------
@@ -795,7 +797,7 @@ int launch_kernel(void (*kernel)(Params...), dim3 grid, size_t smem, cudaStream_
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &attr;
-  cfg.numAttrs = overlap ? 1 : 0;
+  cfg.numAttrs = overlap == kFollows ? 1 : 0;
   CUEQ_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, args...));
   return 0;
 }
@@ -806,16 +808,20 @@ int grid_x(int num_receivers) {
   return want < 1 ? 1 : (want < cap ? want : cap);
 }
 
-template <class T, class G, int C, bool A, bool MASKED>
-int launch_fwd_t(const CwParamsT<T>& p, cudaStream_t st) {
+template <class T, class G, int C, bool A, bool MASKED, bool OVERLAP>
+int launch_fwd_o(const CwParamsT<T>& p, cudaStream_t st) {
   const size_t smem = Smem<G, C, T>::bytes_fwd();
   static cueq::PerDeviceFlag configured;
   if (!configured.get()) {
-    CUEQ_CUDA_OK(cudaFuncSetAttribute(cw_fwd_kernel<T, G, C, A, MASKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CUEQ_CUDA_OK(cudaFuncSetAttribute(cw_fwd_kernel<T, G, C, A, MASKED, OVERLAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     configured.set();
   }
   dim3 grid(grid_x(p.num_receivers), (p.extent + 32 * C - 1) / (32 * C));
-  return launch_kernel(cw_fwd_kernel<T, G, C, A, MASKED>, grid, smem, st, p.overlap, p);
+  return launch_kernel(cw_fwd_kernel<T, G, C, A, MASKED, OVERLAP>, grid, smem, st, p.overlap, p);
+}
+template <class T, class G, int C, bool A, bool MASKED>
+int launch_fwd_t(const CwParamsT<T>& p, cudaStream_t st) {
+  return p.overlap == kAlone ? launch_fwd_o<T, G, C, A, MASKED, false>(p, st) : launch_fwd_o<T, G, C, A, MASKED, true>(p, st);
 }
 
 template <class G, int C, bool A>
